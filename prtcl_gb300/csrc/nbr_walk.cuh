@@ -7,79 +7,98 @@
 
 namespace prtcl_gpu {
 
-// neighbour entries a sweep thread holds at a time (16 or 8; measured per
-// sweep on the 1M dam break)
+// neighbour entries a sweep thread holds at a time (16 or 8) where the sweep
+// does not choose
 constexpr uint32_t kNbrBatchDefault = 16;
 
 struct NbrList {
-  unsigned char const *chunks; // 96-byte chunks (16 offsets + 16 factors), chunk c of item i at (c * n + i)
+  unsigned char const *chunks; // units of 96-byte chunks (16 offsets + 16 factors), at chunk_unit(c, n, i, u)
   uint32_t const *idx32;       // [i * cap + k]: j (read for wide items only)
   uint2 const *cb;             // per item: (count | kWide, base)
   uint32_t cap;                // row length in entries, a multiple of 16
   uint32_t n;                  // rows
 };
 
-// Calls f(j, factor) for the neighbours of item i, in list order.  A chunk
-// of 16 entries is fetched with six 16-byte streaming loads (evict-first:
-// the lists are read once per sweep, the gathered particle records should
-// stay in L2), so that its 16 gathers can be in flight together.
-// (keep_l2: plain L2-cached loads instead, for a row that is walked again
-// right after)
-template <uint32_t kNbrBatch = kNbrBatchDefault, class F>
-__device__ __forceinline__ void for_each_nbr(NbrList const &L, uint32_t i, bool with_gf, F &&f, bool keep_l2 = false) {
+// One unit (32 bytes, 32-byte aligned) in one 256-bit load: streaming
+// (neither kept in L1 nor, for long, in L2: the lists are read once per
+// sweep, the gathered particle records should stay in both), or cached where
+// the row is walked again right after.
+template <bool KEEP> __device__ __forceinline__ void load_unit(unsigned char const *p, uint32_t (&w)[8]) {
+  if (KEEP)
+    asm("ld.global.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "l"(p));
+  else
+    asm("ld.global.L1::no_allocate.L2::evict_first.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+                 : "l"(p));
+}
+
+// Calls f(j, factor) for the neighbours of item i, in list order.  Entries
+// are taken kNbrBatch at a time (16: a whole chunk; 8: half a chunk, fewer
+// registers held per thread), so that as many gathers can be in flight
+// together.  Measured per sweep on the 1M dam break (see the shape lists in
+// schemes.cu).  KEEP: the row's units stay cached.
+template <uint32_t kNbrBatch = kNbrBatchDefault, bool KEEP = false, class F>
+__device__ __forceinline__ void for_each_nbr(NbrList const &L, uint32_t i, bool with_gf, F &&f) {
   uint2 cb = __ldg(L.cb + i);
   uint32_t c = min(cb.x & ~kWide, L.cap);
   bool wide = (cb.x & kWide) != 0;
-  unsigned char const *row = L.chunks + size_t(i) * kChunkBytes;
-  // entries are taken kNbrBatch at a time (16: a whole chunk; 8: half a
-  // chunk, fewer registers held per thread).  Measured per sweep on the 1M
-  // dam break: 8 is faster for the pressure acceleration, the WKBB18
-  // diagonal and system product; 16 for the density and pressure sweeps.
-  for (uint32_t kb = 0; kb < c; kb += kNbrBatch) {
-    uint32_t h = (kb % kChunk) / kNbrBatch; // batch within the chunk
-    uint4 const *ch = reinterpret_cast<uint4 const *>(row + size_t(kb / kChunk) * L.n * kChunkBytes);
-    uint32_t j[kNbrBatch];
-    if (wide) {
-      uint4 const *w32 = reinterpret_cast<uint4 const *>(L.idx32 + size_t(i) * L.cap + kb);
+  unsigned char const *ch = L.chunks + chunk_unit(0, L.n, i, 0);
+  size_t plane = chunk_plane(L.n);
+  constexpr int kHalves = int(kChunk / kNbrBatch), kUnits = int(kNbrBatch / 8);
+  for (uint32_t k0 = 0; k0 < c; k0 += kChunk, ch += plane) {
 #pragma unroll
-      for (int v = 0; v < int(kNbrBatch / 4); ++v) {
-        uint4 a = __ldcs(w32 + v);
-        j[4 * v] = a.x;
-        j[4 * v + 1] = a.y;
-        j[4 * v + 2] = a.z;
-        j[4 * v + 3] = a.w;
-      }
-    } else {
+    for (int h = 0; h < kHalves; ++h) {
+      uint32_t kb = k0 + uint32_t(h) * kNbrBatch;
+      if (h > 0 && kb >= c) break;
+      uint32_t j[kNbrBatch];
+      if (wide) {
+        uint4 const *w32 = reinterpret_cast<uint4 const *>(L.idx32 + size_t(i) * L.cap + kb);
 #pragma unroll
-      for (int v = 0; v < int(kNbrBatch / 8); ++v) {
-        uint4 a = keep_l2 ? __ldcg(ch + h * (kNbrBatch / 8) + v) : __ldcs(ch + h * (kNbrBatch / 8) + v);
-        uint32_t w[4] = {a.x, a.y, a.z, a.w};
+        for (int v = 0; v < int(kNbrBatch / 4); ++v) {
+          uint4 a = __ldcs(w32 + v);
+          j[4 * v] = a.x;
+          j[4 * v + 1] = a.y;
+          j[4 * v + 2] = a.z;
+          j[4 * v + 3] = a.w;
+        }
+      } else {
+        uint32_t w[8];
+        if (kHalves == 1) {
+          load_unit<KEEP>(ch, w);
+        } else {
+          // half a unit; its sector stays in L1 for the other half
+          uint4 a = __ldg(reinterpret_cast<uint4 const *>(ch) + h);
+          w[0] = a.x;
+          w[1] = a.y;
+          w[2] = a.z;
+          w[3] = a.w;
+        }
 #pragma unroll
-        for (int t = 0; t < 4; ++t) {
+        for (int t = 0; t < int(kNbrBatch / 2); ++t) {
           // signed 16-bit offsets from the row's base
-          j[8 * v + 2 * t] = cb.y + uint32_t(int32_t(int16_t(w[t] & 0xFFFFu)));
-          j[8 * v + 2 * t + 1] = cb.y + uint32_t(int32_t(w[t]) >> 16);
+          j[2 * t] = cb.y + uint32_t(int32_t(int16_t(w[t] & 0xFFFFu)));
+          j[2 * t + 1] = cb.y + uint32_t(int32_t(w[t]) >> 16);
         }
       }
-    }
-    float g[kNbrBatch];
-    if (with_gf) {
+      float g[kNbrBatch];
+      if (with_gf) {
 #pragma unroll
-      for (int v = 0; v < int(kNbrBatch / 4); ++v) {
-        uint4 const *gp = ch + 2 + h * (kNbrBatch / 4) + v;
-        uint4 a = keep_l2 ? __ldcg(gp) : __ldcs(gp);
-        g[4 * v] = __uint_as_float(a.x);
-        g[4 * v + 1] = __uint_as_float(a.y);
-        g[4 * v + 2] = __uint_as_float(a.z);
-        g[4 * v + 3] = __uint_as_float(a.w);
+        for (int u = 0; u < kUnits; ++u) {
+          uint32_t q[8];
+          load_unit<KEEP>(ch + (1 + h * kUnits + u) * int(kUnitSpan), q);
+#pragma unroll
+          for (int t = 0; t < 8; ++t) g[8 * u + t] = __uint_as_float(q[t]);
+        }
+      } else {
+#pragma unroll
+        for (int t = 0; t < int(kNbrBatch); ++t) g[t] = 0.0f;
       }
-    } else {
 #pragma unroll
-      for (int t = 0; t < int(kNbrBatch); ++t) g[t] = 0.0f;
+      for (int t = 0; t < int(kNbrBatch); ++t)
+        if (kb + t < c) f(j[t], g[t]);
     }
-#pragma unroll
-    for (int t = 0; t < int(kNbrBatch); ++t)
-      if (kb + t < c) f(j[t], g[t]);
   }
 }
 
@@ -94,9 +113,8 @@ __device__ __forceinline__ void for_each_staged(NbrList const &L, uint16_t const
   uint32_t c = min(cb.x & ~kWide, L.cap);
   for (uint32_t kb = 0; kb < c; kb += kNbrBatch) {
     uint32_t h = (kb % kChunk) / kNbrBatch;
-    size_t ci = size_t(kb / kChunk) * L.n + i;
-    uint4 const *ch = reinterpret_cast<uint4 const *>(L.chunks + ci * kChunkBytes);
-    uint4 const *sp = reinterpret_cast<uint4 const *>(slots + ci * kChunk);
+    unsigned char const *ch = L.chunks + chunk_unit(kb / kChunk, L.n, i, 1 + h * (kNbrBatch / 8));
+    uint4 const *sp = reinterpret_cast<uint4 const *>(slots + (size_t(kb / kChunk) * L.n + i) * kChunk);
     uint32_t sl[kNbrBatch];
 #pragma unroll
     for (int v = 0; v < int(kNbrBatch / 8); ++v) {
@@ -110,12 +128,11 @@ __device__ __forceinline__ void for_each_staged(NbrList const &L, uint16_t const
     }
     float g[kNbrBatch];
 #pragma unroll
-    for (int v = 0; v < int(kNbrBatch / 4); ++v) {
-      uint4 a = __ldcs(ch + 2 + h * (kNbrBatch / 4) + v);
-      g[4 * v] = __uint_as_float(a.x);
-      g[4 * v + 1] = __uint_as_float(a.y);
-      g[4 * v + 2] = __uint_as_float(a.z);
-      g[4 * v + 3] = __uint_as_float(a.w);
+    for (int u = 0; u < int(kNbrBatch / 8); ++u) {
+      uint32_t q[8];
+      load_unit<false>(ch + u * int(kUnitSpan), q);
+#pragma unroll
+      for (int t = 0; t < 8; ++t) g[8 * u + t] = __uint_as_float(q[t]);
     }
 #pragma unroll
     for (int t = 0; t < int(kNbrBatch); ++t)

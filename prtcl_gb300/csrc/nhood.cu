@@ -724,17 +724,19 @@ template <int BW> __device__ __forceinline__ uint32_t &bufw(uint32_t *buf, int g
 template <int BW>
 __device__ __forceinline__ void flush_chunk(ListOut const &lo, int g, uint32_t i, uint32_t chunk, bool wide,
                                             uint32_t *buf) {
-  size_t ci = size_t(chunk) * lo.n + i;
-  uint4 *dst = reinterpret_cast<uint4 *>(lo.chunks[g] + ci * kChunkBytes);
-  // offsets (2 vectors, not for a wide row), then the factors (4 vectors)
+  // offsets (unit 0, not for a wide row), then the factors (units 1 and 2)
   // when the lists carry them: sweeps read factors only from lists built
   // with a smoothing scale
-  int v0 = wide ? 2 : 0, nv = lo.with_gf ? 6 : 2;
-  for (int v = v0; v < nv; ++v)
-    dst[v] = make_uint4(bufw<BW>(buf, g, 4 * v), bufw<BW>(buf, g, 4 * v + 1), bufw<BW>(buf, g, 4 * v + 2),
-                        bufw<BW>(buf, g, 4 * v + 3));
+  unsigned char *ch = lo.chunks[g] + chunk_unit(chunk, lo.n, i, 0);
+  int u0 = wide ? 1 : 0, nu = lo.with_gf ? 3 : 1;
+  for (int u = u0; u < nu; ++u) {
+    uint4 *dst = reinterpret_cast<uint4 *>(ch + u * int(kUnitSpan));
+    for (int v = 0; v < 2; ++v)
+      dst[v] = make_uint4(bufw<BW>(buf, g, 8 * u + 4 * v), bufw<BW>(buf, g, 8 * u + 4 * v + 1),
+                          bufw<BW>(buf, g, 8 * u + 4 * v + 2), bufw<BW>(buf, g, 8 * u + 4 * v + 3));
+  }
   if (BW == 32) {
-    uint4 *sd = reinterpret_cast<uint4 *>(lo.slots[g] + ci * kChunk);
+    uint4 *sd = reinterpret_cast<uint4 *>(lo.slots[g] + (size_t(chunk) * lo.n + i) * kChunk);
     for (int v = 0; v < 2; ++v)
       sd[v] = make_uint4(bufw<BW>(buf, g, 24 + 4 * v), bufw<BW>(buf, g, 25 + 4 * v), bufw<BW>(buf, g, 26 + 4 * v),
                          bufw<BW>(buf, g, 27 + 4 * v));
@@ -765,7 +767,7 @@ __device__ __forceinline__ void row_add(ListOut const &lo, int g, uint32_t i, Ro
     for (uint32_t e = 0; e < k; ++e) {
       uint32_t w;
       if (e / kChunk == k / kChunk) w = bufw<BW>(buf, g, int((e % kChunk) / 2));
-      else w = reinterpret_cast<uint32_t const *>(lo.chunks[g] + (size_t(e / kChunk) * lo.n + i) * kChunkBytes)[(e % kChunk) / 2];
+      else w = reinterpret_cast<uint32_t const *>(lo.chunks[g] + chunk_unit(e / kChunk, lo.n, i, 0))[(e % kChunk) / 2];
       int32_t de = int32_t(int16_t((e & 1) ? (w >> 16) : (w & 0xFFFFu)));
       lo.idx32[g][size_t(i) * lo.cap[g] + e] = R.j0 + uint32_t(de);
     }
@@ -1187,6 +1189,11 @@ constexpr int kSplit = 4, kSplitNT = 128;
 constexpr size_t kSplitMaxQueries = 65536;
 __device__ __forceinline__ int split_first_visit(int sub) { return sub * 7; } // 0, 7, 14, 21; 27 at the end
 
+// the factor word of entry `slot` of the chunk whose unit 0 is at ch
+__device__ __forceinline__ uint32_t *factor_word(unsigned char *ch, uint32_t slot) {
+  return reinterpret_cast<uint32_t *>(ch + (1 + slot / 8) * kUnitSpan) + slot % 8;
+}
+
 template <class F>
 __device__ __forceinline__ void split_walk(GridView const &gv, float4 const *__restrict__ xs, int cell,
                                            float const *lo3, float const *hi3, int v0, int v1, f3 xi, F &&f) {
@@ -1316,10 +1323,10 @@ __global__ void __launch_bounds__(kSplitNT) k_build_lists_split(GridView gv, flo
       if (qq == int(g)) {
         uint32_t k = run[qq]++;
         if (k < lo.cap[qq]) {
-          unsigned char *ch = lo.chunks[qq] + (size_t(k / kChunk) * lo.n + i) * kChunkBytes;
+          unsigned char *ch = lo.chunks[qq] + chunk_unit(k / kChunk, lo.n, i, 0);
           if (wide[qq]) lo.idx32[qq][size_t(i) * lo.cap[qq] + k] = j;
           else reinterpret_cast<uint16_t *>(ch)[k % kChunk] = uint16_t(uint32_t(int32_t(j - j0[qq])) & 0xFFFFu);
-          if (lo.with_gf) reinterpret_cast<uint32_t *>(ch + 32)[k % kChunk] = __float_as_uint(f);
+          if (lo.with_gf) *factor_word(ch, k % kChunk) = __float_as_uint(f);
         }
       }
   });
@@ -1332,14 +1339,14 @@ __global__ void __launch_bounds__(kSplitNT) k_build_lists_split(GridView gv, flo
     atomicMax(&lo.maxcnt[g], n);
     if (n > lo.cap[g] || n % kChunk == 0) continue;
     // the partial last chunk (and half-chunk of a wide row), zero-filled
-    unsigned char *ch = lo.chunks[g] + (size_t(n / kChunk) * lo.n + i) * kChunkBytes;
+    unsigned char *ch = lo.chunks[g] + chunk_unit(n / kChunk, lo.n, i, 0);
     if (wide[g]) {
       for (uint32_t e = n; e % 8; ++e) lo.idx32[g][size_t(i) * lo.cap[g] + e] = 0u;
     } else {
       for (uint32_t slot = n % kChunk; slot < kChunk; ++slot) reinterpret_cast<uint16_t *>(ch)[slot] = 0u;
     }
     if (lo.with_gf)
-      for (uint32_t slot = n % kChunk; slot < kChunk; ++slot) reinterpret_cast<uint32_t *>(ch + 32)[slot] = 0u;
+      for (uint32_t slot = n % kChunk; slot < kChunk; ++slot) *factor_word(ch, slot) = 0u;
   }
 }
 
@@ -1811,7 +1818,7 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
     L.slots[g] = nullptr;
     if (n > 0) {
       PG_CUDA(cudaMalloc(&L.idx32[g], size_t(want) * n * 4));
-      PG_CUDA(cudaMalloc(&L.chunks[g], size_t(want / kChunk) * kChunkBytes * n));
+      PG_CUDA(cudaMalloc(&L.chunks[g], size_t(want / kChunk) * chunk_plane(n)));
       if (L.staged) PG_CUDA(cudaMalloc(&L.slots[g], size_t(want) * n * sizeof(uint16_t)));
     }
     L.cap[g] = want;
@@ -2066,7 +2073,7 @@ size_t Nhood::device_bytes() const {
     Lists const &L = kv.second;
     b += L.n * gg_.size() * sizeof(uint2);
     for (size_t g = 0; g < gg_.size() && g < size_t(kMaxGroups); ++g)
-      b += L.n * (size_t(L.cap[g]) * 4 + size_t(L.cap[g] / kChunk) * kChunkBytes);
+      b += L.n * size_t(L.cap[g]) * 4 + size_t(L.cap[g] / kChunk) * chunk_plane(L.n);
   }
   return b;
 }
@@ -2115,12 +2122,13 @@ size_t Nhood::copy_neighbors(int g, size_t i, int64_t *counts, int64_t *out, siz
     uint32_t cn = cb.x & ~kWide;
     counts[ng] = cn;
     if (!cn) continue;
-    // the item's chunks, one per chunk plane, packed on the host
+    // the offsets of the item's chunks, one unit per chunk plane, packed on
+    // the host as the chunks of a single item are
     size_t nch = v.cap[ng] / kChunk;
-    std::vector<unsigned char> row(nch * kChunkBytes);
+    std::vector<unsigned char> row(nch * chunk_plane(1));
     std::vector<uint32_t> e32(v.cap[ng]);
-    PG_CUDA(cudaMemcpy2DAsync(row.data(), kChunkBytes, v.chunks[ng] + i * kChunkBytes, size_t(v.n) * kChunkBytes,
-                              kChunkBytes, nch, cudaMemcpyDeviceToHost, s));
+    PG_CUDA(cudaMemcpy2DAsync(row.data(), chunk_plane(1), v.chunks[ng] + chunk_unit(0, v.n, i, 0), chunk_plane(v.n),
+                              kUnitBytes, nch, cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaMemcpyAsync(e32.data(), v.idx32[ng] + i * v.cap[ng], v.cap[ng] * 4, cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaStreamSynchronize(s));
     for (uint32_t slot = 0; slot < cn; ++slot) {
@@ -2150,7 +2158,7 @@ void Nhood::copy_lists(int q, int ng, int64_t *offsets, uint32_t *idx, size_t ca
   std::vector<unsigned char> ch;
   std::vector<uint32_t> e32;
   if (v.chunks[ng] && used) {
-    ch.resize(size_t(used / kChunk) * kChunkBytes * n);
+    ch.resize(size_t(used / kChunk) * chunk_plane(n));
     e32.resize(size_t(used) * n);
     PG_CUDA(cudaMemcpyAsync(ch.data(), v.chunks[ng], ch.size(), cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaMemcpy2DAsync(e32.data(), size_t(used) * 4, v.idx32[ng], size_t(v.cap[ng]) * 4, size_t(used) * 4, n,

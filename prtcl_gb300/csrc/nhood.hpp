@@ -43,15 +43,18 @@
 namespace prtcl_gpu {
 
 // Device view of the neighbour lists of one query group, one set per
-// neighbour group g.  In 96-byte chunks of 16 entries: chunk c of item i
-// holds its entries 16c..16c+15 as
-//   16 x uint16  j - base   (32 bytes)
-//   16 x float   the pair's kernel-gradient factor (64 bytes)
-// so a chunk is exactly three 32-byte sectors and every fetched sector is
-// used once (offsets are signed 16-bit: j = base + offset).  Chunk-major:
-// chunk c of item i sits at chunks[(c * n + i) * 96], so that the threads
-// of a warp, walking consecutive items, read their chunk c from one
-// contiguous 3 KB span.  Also per item:
+// neighbour group g.  In 96-byte chunks of 16 entries, each three units of
+// 32 bytes (one DRAM sector each): chunk c of item i holds its entries
+// 16c..16c+15 as
+//   unit 0      16 x uint16  j - base
+//   units 1, 2  16 x float   the pair's kernel-gradient factor
+// (offsets are signed 16-bit: j = base + offset).  Chunk-major, and within a
+// chunk's plane unit-major per 32 items: unit u of chunk c of item i sits at
+// chunk_unit(c, n, i, u).  A warp walking 32 consecutive items reads one unit
+// of its chunk c with one 32-byte load per thread from 1 KB of consecutive
+// bytes.  (With the three units of an item side by side, each 16-byte load of
+// a warp touched 24 cache lines instead of 4, and the L1 was the busiest unit
+// of the sweeps.)  Also per item:
 //   cb[g][i]    (count | kWide if "wide", base = the first neighbour's index)
 //   idx32[g]    j as 32-bit indices at [i * cap + k], written and read for
 //               "wide" items only (neighbours spanning >= 65536 indices)
@@ -60,6 +63,14 @@ namespace prtcl_gpu {
 // smoothing scale and evaluate the gradient in full otherwise.
 constexpr uint32_t kChunk = 16;
 constexpr uint32_t kChunkBytes = kChunk * 2 + kChunk * 4;
+constexpr uint32_t kUnitBytes = 32;
+// bytes of one chunk plane of n items, and of one unit of 32 items
+__host__ __device__ constexpr size_t chunk_plane(size_t n) { return ((n + 31) / 32) * (32 * kChunkBytes); }
+constexpr uint32_t kUnitSpan = 32 * kUnitBytes;
+// byte offset of unit u of chunk c of item i among n items
+__host__ __device__ constexpr size_t chunk_unit(size_t c, size_t n, size_t i, uint32_t u) {
+  return c * chunk_plane(n) + (i >> 5) * (32 * kChunkBytes) + u * kUnitSpan + (i & 31) * kUnitBytes;
+}
 // Staged lists (built on request for a query group in cell order): the
 // query items form tiles of kStageTile consecutive items (the list build's
 // blocks, and the staged sweeps' blocks).  The cells adjacent to a tile's
@@ -99,7 +110,7 @@ constexpr uint32_t kWide = 0x80000000u;
 inline uint32_t nbr_host_decode(uint2 cb, unsigned char const *chunks, size_t n, size_t i, uint32_t const *idx32row,
                                 uint32_t k) {
   if (cb.x & kWide) return idx32row[k];
-  unsigned char const *p = chunks + (size_t(k / kChunk) * n + i) * kChunkBytes + (k % kChunk) * 2;
+  unsigned char const *p = chunks + chunk_unit(k / kChunk, n, i, 0) + (k % kChunk) * 2;
   int16_t d = int16_t(uint16_t(p[0] | (p[1] << 8)));
   return cb.y + uint32_t(int32_t(d));
 }
