@@ -155,7 +155,7 @@ enum TuneKnob : int {
   kTuneJacobiUnroll,
   kTuneStaging,  // 1: staged lists and the staged Jacobi / PCG sweeps
   kTuneGridSort, // 1: grids of at most 128k items sorted in one launch of a thread-block cluster
-  kTuneListSplit, // 1: lists of query groups of at most 64k items built by four threads per query
+  kTuneListSplit, // 1: lists built by one warp per run of queries of a cell, 0: by one thread per query
   kTuneKnobs
 };
 struct Tuning {

@@ -1173,181 +1173,321 @@ __global__ void __launch_bounds__(kBuildNT, STAGE ? 5 : (NG <= 2 ? 9 : 1))
   }
 }
 
-// Lists of a small query group (the list_split knob): kSplit threads per
-// query, each walking a contiguous part of the query's visit sequence (own
-// cell, then adjacency slots 0..25: parts of 7, 7, 7 and 6 cells), so that
-// a query's dependent chain of cell walks is a quarter as long.  A first
-// walk counts each part's neighbours per group (with the first index and
-// the index range); the query's threads combine them by shuffles into each
-// row's count, base index and wide / narrow form, and a second walk writes
-// every entry straight to its place in the chunks (or idx32 for a wide
-// row), with its gradient factor.  The visited cells, the distance test and
-// the factor arithmetic are those of k_build_lists, so the rows are the
-// same entry for entry; the tail of a row's last chunk is zero-filled as
-// there.  For a query group of the grid (no fallback search).
-constexpr int kSplit = 4, kSplitNT = 128;
-constexpr size_t kSplitMaxQueries = 65536;
-__device__ __forceinline__ int split_first_visit(int sub) { return sub * 7; } // 0, 7, 14, 21; 27 at the end
-
 // the factor word of entry `slot` of the chunk whose unit 0 is at ch
 __device__ __forceinline__ uint32_t *factor_word(unsigned char *ch, uint32_t slot) {
   return reinterpret_cast<uint32_t *>(ch + (1 + slot / 8) * kUnitSpan) + slot % 8;
 }
 
-template <class F>
-__device__ __forceinline__ void split_walk(GridView const &gv, float4 const *__restrict__ xs, int cell,
-                                           float const *lo3, float const *hi3, int v0, int v1, f3 xi, F &&f) {
-  for (int v = v0; v < v1; ++v) {
-    int c = cell;
-    if (v > 0) {
-      int k = v - 1;
-      // slot k < 13: +offset[k]; slot 25 - k: -offset[k]
-      int kk = k < 13 ? k : 25 - k;
-      int sg = k < 13 ? 1 : -1;
-      float lb = 0.0f;
+// ---------------------------------------------------------------------------
+// Lists of a query group in the grid, one warp per run of queries (the
+// list_split knob, on by default)
+// ---------------------------------------------------------------------------
+//
+// The queries of a cell see the same 27 cells, so they share their candidates.
+// A unit is up to kUnit consecutive sorted items of one cell; a warp takes the
+// units that begin in its window of kWinItems sorted items (one that begins
+// there may run past its end, so a warp has at most kWinItems + kUnit - 1
+// items, however full the cells are).  Per unit:
+//   1. lanes 0..26 look up the 27 cells in visit order (own cell, adjacency
+//      slots 0..25); their ranges, one after the other, are the candidates,
+//      taken kCand at a time (a portion);
+//   2. 64 candidates at a time, two per lane, are tested against the unit's
+//      queries one by one (differences and squares packed); a ballot per 32
+//      candidates gives a query's hit mask;
+//   3. a row is one query's list towards one neighbour group.  The masks are
+//      divided over all lanes, which write the hits (row, candidate) to the
+//      warp's flat list, row after row, each in candidate order;
+//   4. the lanes take the flat list's hits 32 at a time, whatever row they
+//      belong to: the neighbour index and the gradient factor (square root
+//      and divisions) go straight to their places in the row's chunks.
+// So the tests and the factors run with full warps: with a thread per query
+// (k_build_lists) 12 to 18 of 32 lanes were active.  The visited cells, their
+// order, the test and the factor arithmetic are those of k_build_lists, hence
+// so are the rows' entries.  (A row is stored wide when its unit's candidates
+// span more than 16 bits, which may be before its own hits do; the words past
+// a row's end, which nothing reads, are not written.)  A row of several
+// portions that turns wide is converted where it does; a row longer than the
+// capacity is counted on, not written.
+//
+// What bounds it: instruction issue (70 % of the slots at 28 warps per SM on
+// the dam break) and the latency between a unit's phases, which the resident
+// warps hide: candidates kept in registers or staged with their positions in
+// shared memory left 16 to 24 warps and took 516 to 645 us on the 1M dam
+// break.  The register bounds below are the fastest of 8 to 20 blocks for each
+// form.  Measured in one call against a thread per query (and, up to 65,536
+// queries, against four threads per query, the form before this one): 4M
+// uniform points 2446 -> 1112 us, 1.5M clustered 1381 -> 719; with factors, 1M
+// dam break 659 -> 425 us, 27k 52 (four threads) -> 37, 5k 39 -> 28.
+constexpr int kWinItems = 16;
+constexpr int kCand = 320, kCandChunks = kCand / 32;
+constexpr int kUnit = 16;             // queries of a unit
+constexpr int kFlat = 640;            // hits of a portion written out together
+constexpr int kWarpNT = 64, kWarps = kWarpNT / 32;
+
+// a warp's shared memory
+struct ListWarp {
+  uint32_t sidx[kCand];              // sorted index of each candidate; its handle once tested, where no factor needs more
+  float4 qxy[kUnit];                 // query position, each coordinate twice
+  float2 qzz[kUnit];
+  uint32_t mask[kUnit][kCandChunks]; // hits of a query among 32 candidates
+  uint32_t second[kCandChunks];      // candidates of the second group
+  uint4 row[32];                     // per row: flat index -> entry, base index, wide
+  ulonglong2 to[32];                 // per row: its first chunk, its 32-bit indices
+  uint16_t flat[kFlat];              // row << 10 | candidate
+};
+static_assert(kCand <= 1024 && kCand <= kFlat, "a flat entry holds the candidate in 10 bits, a query's hits fit the list");
+static_assert(kUnit * 2 <= 32, "a lane per row");
+
+__device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane) {
 #pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        int o = sg * c_offsets[kk][a];
-        float b = o > 0 ? hi3[a] : (o < 0 ? lo3[a] : 0.0f);
-        lb += b * b;
+  for (int o = 1; o < 32; o <<= 1) {
+    uint32_t y = __shfl_up_sync(kFull, v, o);
+    if (lane >= o) v += y;
+  }
+  return v;
+}
+
+// the range of the items' indices that `in` holds for
+__device__ __forceinline__ void index_range(bool in, uint32_t handle, uint32_t &lo, uint32_t &hi) {
+  uint32_t j = handle & 0x0FFFFFFFu;
+  lo = min(lo, in ? j : 0xFFFFFFFFu);
+  hi = max(hi, in ? j : 0u);
+}
+
+template <int NG, bool GF>
+__global__ void __launch_bounds__(kWarpNT, GF ? 16 : 18) k_build_lists_warp(GridView gv, float4 const *__restrict__ xs, size_t N,
+                                                              int q, ListOut lo, float const *hp, float *hcache) {
+  static_assert(NG == 1 || NG == 2, "one or two neighbour groups");
+  __shared__ ListWarp s_warp[kWarps];
+  ListWarp &S = s_warp[threadIdx.x / 32];
+  int lane = threadIdx.x & 31;
+  KernelParams K = kparams(GF ? *hp : 1.0f);
+  if (blockIdx.x == 0 && threadIdx.x == 0) *hcache = GF ? K.h : __int_as_float(0x7fc00000);
+  size_t win = (size_t(blockIdx.x) * kWarps + threadIdx.x / 32) * kWinItems;
+  if (win >= N) return; // whole warps
+  // the units that begin in the window
+  int wcell = 0, wend = 0;
+  bool begins = false;
+  if (lane < kWinItems && win + lane < N) {
+    int s = int(win) + lane;
+    wcell = gv.s2c[s];
+    wend = gv.cell_start[wcell + 1];
+    begins = (s - gv.cell_start[wcell]) % kUnit == 0;
+  }
+  uint32_t units = __ballot_sync(kFull, begins);
+  size_t plane = chunk_plane(lo.n);
+  int rq = lane / NG, rg = lane % NG; // lane r's row: query, neighbour group
+  uint32_t longest = 0;
+  while (units) {
+    int b = __ffs(int(units)) - 1;
+    units &= units - 1u;
+    int u0 = int(win) + b, cell = __shfl_sync(kFull, wcell, b);
+    int ni = min(kUnit, __shfl_sync(kFull, wend, b) - u0);
+    // 1. the candidate ranges
+    int first = 0, len = 0;
+    if (lane < 27) {
+      int c = lane == 0 ? cell : gv.cell_adj[size_t(cell) * 26 + lane - 1];
+      if (c >= 0) {
+        first = gv.cell_start[c];
+        len = gv.cell_start[c + 1] - first;
       }
-      if (lb > 1.0001f) continue;
-      c = gv.cell_adj[size_t(cell) * 26 + k];
     }
-    if (c < 0) continue;
-    int s0 = gv.cell_start[c], s1 = gv.cell_start[c + 1];
-    for (int base = s0; base < s1; base += 32) {
-      int e = min(s1 - base, 32);
-      uint32_t mask = 0;
-      for (int t = 0; t < e; ++t) {
-        float d2 = nsq3(sub3(xi, mk3(xs[base + t])));
-        if (d2 < gv.r2lt) mask |= 1u << t;
+    // a cell's items are in (group, index) order: the unit's queries are consecutive
+    float4 X = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0xFFFFFFFFu));
+    if (lane < ni) X = xs[u0 + lane];
+    uint32_t qh = __float_as_uint(X.w);
+    uint32_t qm = __ballot_sync(kFull, lane < ni && int(qh >> 28) == q);
+    if (!qm) continue;
+    int q0 = __ffs(int(qm)) - 1, nq = __popc(qm);
+    if (lane >= q0 && lane < q0 + nq) {
+      S.qxy[lane - q0] = make_float4(X.x, X.x, X.y, X.y);
+      S.qzz[lane - q0] = make_float2(X.z, X.z);
+    }
+    uint32_t item = __shfl_sync(kFull, qh, min(q0 + rq, 31)) & 0x0FFFFFFFu; // lane r's row's query item
+    // (a group that shrank since the grid's update has no rows for its former items)
+    bool owner = rq < nq && item < lo.n;
+    if (owner)
+      S.to[lane] = make_ulonglong2(
+          reinterpret_cast<unsigned long long>(lo.chunks[rg] + chunk_unit(0, lo.n, item, 0)),
+          reinterpret_cast<unsigned long long>(lo.idx32[rg] + size_t(item) * lo.cap[rg]));
+    // the hit masks are read by 2^ps lanes per query, a range of words each
+    int ps = __clz(nq - 1) - 27, hq = lane >> ps, hp_ = lane & ((1 << ps) - 1);
+    int has_rows = __shfl_sync(kFull, owner ? 1 : 0, min(hq * NG, 31)); // (every lane takes part)
+    bool reader = hq < nq && has_rows != 0;
+    uint32_t cnt = 0, base = 0;
+    bool wide = false;
+    uint32_t jmin[NG], jmax[NG]; // of the candidates so far
+#pragma unroll
+    for (int g = 0; g < NG; ++g) {
+      jmin[g] = 0xFFFFFFFFu;
+      jmax[g] = 0u;
+    }
+    int end = int(warp_incl_scan(uint32_t(len), lane));
+    int total = __shfl_sync(kFull, end, 31), beg = end - len;
+    for (int p0 = 0; p0 < total; p0 += kCand) {
+      int np = min(kCand, total - p0), nk = (np + 31) / 32;
+      for (int t = max(0, p0 - beg), te = min(len, p0 + np - beg); t < te; ++t) S.sidx[beg + t - p0] = uint32_t(first + t);
+      __syncwarp();
+      // 2. the tests, 64 candidates at a time (two per lane), negated in
+      // registers (x - y == x + (-y)); past the portion's end at infinity,
+      // where no test holds.  The next 64 are loaded meanwhile.
+      float4 const far = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+      float4 A = lane < np ? xs[S.sidx[lane]] : far, B = lane + 32 < np ? xs[S.sidx[lane + 32]] : far;
+      for (int k = 0; k < nk; k += 2) {
+        int p = k * 32 + lane;
+        bool ia = p < np, ib = p + 32 < np;
+        float2 nx = make_float2(-A.x, -B.x), ny = make_float2(-A.y, -B.y), nz = make_float2(-A.z, -B.z);
+        uint32_t ha = __float_as_uint(A.w), hb = __float_as_uint(B.w);
+        if (!GF && ia) S.sidx[p] = ha;
+        if (!GF && ib) S.sidx[p + 32] = hb;
+        A = p + 64 < np ? xs[S.sidx[p + 64]] : far;
+        B = p + 96 < np ? xs[S.sidx[p + 96]] : far;
+        if constexpr (NG == 2) {
+          bool sa = ia && (ha >> 28) != 0u, sb = ib && (hb >> 28) != 0u;
+          uint2 m;
+          m.x = __ballot_sync(kFull, sa);
+          m.y = __ballot_sync(kFull, sb);
+          if (lane == 0) *reinterpret_cast<uint2 *>(&S.second[k]) = m;
+          index_range(sa, ha, jmin[1], jmax[1]);
+          index_range(sb, hb, jmin[1], jmax[1]);
+          ia = ia && !sa;
+          ib = ib && !sb;
+        }
+        index_range(ia, ha, jmin[0], jmax[0]);
+        index_range(ib, hb, jmin[0], jmax[0]);
+#pragma unroll 2
+        for (int t = 0; t < nq; ++t) {
+          float4 xy = S.qxy[t];
+          float2 dx = __fadd2_rn(make_float2(xy.x, xy.y), nx), dy = __fadd2_rn(make_float2(xy.z, xy.w), ny);
+          float2 dz = __fadd2_rn(S.qzz[t], nz);
+          // (packed sums of packed products come out fused, -fmad=false and the
+          // explicit rounding notwithstanding: three pairs of 160M changed)
+          float2 xx = __fmul2_rn(dx, dx), yy = __fmul2_rn(dy, dy), zz = __fmul2_rn(dz, dz);
+          float2 d2 = make_float2(xx.x + (yy.x + zz.x), xx.y + (yy.y + zz.y));
+          uint2 m;
+          m.x = __ballot_sync(kFull, d2.x < gv.r2lt); // == (double) d2 < r^2
+          m.y = __ballot_sync(kFull, d2.y < gv.r2lt);
+          if (lane == 0) *reinterpret_cast<uint2 *>(&S.mask[t][k]) = m;
+        }
       }
-      while (mask) {
-        int t = __ffs(int(mask)) - 1;
-        mask &= mask - 1u;
-        f(base + t);
+      // a row is wide once its group's candidates span more than 16 bits
+      bool spans = false;
+#pragma unroll
+      for (int g = 0; g < NG; ++g) {
+        uint32_t a = __reduce_min_sync(kFull, jmin[g]), z = __reduce_max_sync(kFull, jmax[g]);
+        if (rg == g) spans = a < z && z - a > 32767u;
+      }
+      __syncwarp();
+      // 3. the rows' hits: flat places by query, then group, then candidate
+      int k0 = (hp_ * nk) >> ps, k1 = ((hp_ + 1) * nk) >> ps;
+      uint32_t c0 = 0, c1 = 0;
+      if (reader)
+        for (int k = k0; k < k1; ++k) {
+          uint32_t m = S.mask[hq][k];
+          if constexpr (NG == 2) {
+            uint32_t w = m & S.second[k];
+            c1 += __popc(w);
+            m ^= w;
+          }
+          c0 += __popc(m);
+        }
+      uint32_t e0 = warp_incl_scan(c0, lane), e1 = NG == 2 ? warp_incl_scan(c1, lane) : 0u;
+      // of this lane's reader query and of its row's query: hits before it and up to its end
+      auto span = [&](int qq, uint32_t &b0, uint32_t &z0, uint32_t &b1, uint32_t &z1) {
+        int l0 = min(qq << ps, 31), l1 = min(((qq + 1) << ps) - 1, 31);
+        b0 = __shfl_sync(kFull, e0 - c0, l0);
+        z0 = __shfl_sync(kFull, e0, l1);
+        b1 = NG == 2 ? __shfl_sync(kFull, e1 - c1, l0) : 0u;
+        z1 = NG == 2 ? __shfl_sync(kFull, e1, l1) : 0u;
+      };
+      uint32_t b0, z0, b1, z1, rb0, rz0, rb1, rz1;
+      span(hq, b0, z0, b1, z1);
+      span(rq, rb0, rz0, rb1, rz1);
+      uint32_t f0 = (e0 - c0) + b1, f1 = z0 + (e1 - c1);              // this lane's places
+      uint32_t rbeg = rg == 0 ? rb0 + rb1 : rz0 + rb1;                // its row's places
+      uint32_t hits = owner ? (rg == 0 ? rz0 - rb0 : rz1 - rb1) : 0u;
+      uint32_t all = __shfl_sync(kFull, e0 + e1, 31);
+      for (uint32_t done = 0; done < all;) {
+        // as many whole queries as the flat list holds
+        bool qin = reader && b0 + b1 >= done && z0 + z1 <= done + uint32_t(kFlat);
+        uint32_t upto = __reduce_max_sync(kFull, qin ? z0 + z1 : 0u);
+        if (qin) {
+          uint32_t w0 = f0 - done, w1 = f1 - done, tag = uint32_t(hq * NG) << 10;
+          for (int k = k0; k < k1; ++k) {
+            uint32_t m = S.mask[hq][k], sec = NG == 2 ? S.second[k] : 0u;
+            while (m) {
+              int t = __ffs(int(m)) - 1;
+              m &= m - 1u;
+              uint32_t f = tag | uint32_t(k * 32 + t);
+              if (NG == 2 && ((sec >> t) & 1u)) S.flat[w1++] = uint16_t(f + 1024u);
+              else S.flat[w0++] = uint16_t(f);
+            }
+          }
+        }
+        __syncwarp();
+        bool in = hits > 0 && rbeg >= done && rbeg < upto;
+        // 4. entries; a row that turns wide: its entries of earlier portions
+        // to 32-bit indices
+        bool turned = in && spans && !wide;
+        for (uint32_t tm = __ballot_sync(kFull, turned && cnt > 0); tm; tm &= tm - 1u) {
+          int r = __ffs(int(tm)) - 1, g = r % NG;
+          uint32_t it = __shfl_sync(kFull, item, r), bs = __shfl_sync(kFull, base, r);
+          uint32_t ne = min(__shfl_sync(kFull, cnt, r), lo.cap[g]);
+          for (uint32_t e = lane; e < ne; e += 32) {
+            unsigned char const *ch = lo.chunks[g] + chunk_unit(e / kChunk, lo.n, it, 0);
+            int32_t d = reinterpret_cast<int16_t const *>(ch)[e % kChunk];
+            lo.idx32[g][size_t(it) * lo.cap[g] + e] = bs + uint32_t(d);
+          }
+        }
+        if (in) {
+          wide = wide || turned;
+          uint32_t p = S.flat[rbeg - done] & 1023u;
+          if (cnt == 0) base = (GF ? __float_as_uint(xs[S.sidx[p]].w) : S.sidx[p]) & 0x0FFFFFFFu;
+          S.row[lane] = make_uint4(cnt - (rbeg - done), base, wide ? 1u : 0u, 0u);
+        }
+        __syncwarp();
+        uint32_t nf = upto - done;
+        for (uint32_t e = lane; e < nf; e += 32) {
+          uint32_t f = S.flat[e], r = f >> 10, c = S.sidx[f & 1023u];
+          uint4 R = S.row[r];
+          ulonglong2 to = S.to[r];
+          float4 Y = GF ? xs[c] : make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(c));
+          uint32_t k = e + R.x, j = __float_as_uint(Y.w) & 0x0FFFFFFFu;
+          if (k < (NG == 2 && (r & 1u) ? lo.cap[NG - 1] : lo.cap[0])) {
+            unsigned char *ch = reinterpret_cast<unsigned char *>(to.x) + (k / kChunk) * plane;
+            if (R.z) reinterpret_cast<uint32_t *>(to.y)[k] = j;
+            else reinterpret_cast<uint16_t *>(ch)[k % kChunk] = uint16_t((j - R.y) & 0xFFFFu);
+            if constexpr (GF)
+              *factor_word(ch, k % kChunk) = __float_as_uint(
+                  kgrad_factor(K, nsq3(sub3({S.qxy[r / NG].x, S.qxy[r / NG].z, S.qzz[r / NG].x}, mk3(Y)))));
+          }
+        }
+        if (in) cnt += hits;
+        done = upto;
+        __syncwarp(); // the flat list and the row table are written again
       }
     }
+    if (owner) {
+      lo.cb[size_t(rg) * lo.n + item] = make_uint2(cnt | (wide ? kWide : 0u), base);
+      longest = max(longest, cnt);
+    }
+    __syncwarp(); // the queries are written again
+  }
+  // the longest row of each group: the host grows or shrinks the lists by it
+#pragma unroll
+  for (int g = 0; g < NG; ++g) {
+    uint32_t m = __reduce_max_sync(kFull, rg == g ? longest : 0u);
+    // (most warps find a longer row recorded already: no atomic)
+    if (lane == 0 && m > __ldcg(&lo.maxcnt[g])) atomicMax(&lo.maxcnt[g], m);
   }
 }
 
 template <int NG>
-__global__ void __launch_bounds__(kSplitNT) k_build_lists_split(GridView gv, float4 const *__restrict__ xs,
-                                                               float4 const *__restrict__ qpos, int q, ListOut lo,
-                                                               float const *hp, float *hcache,
-                                                               uint32_t const *__restrict__ order) {
-  uint32_t gt = blockIdx.x * kSplitNT + threadIdx.x;
-  uint32_t t = gt / kSplit;
-  int sub = int(gt % kSplit);
-  bool with_gf = hp != nullptr;
-  KernelParams K = kparams(with_gf ? *hp : 1.0f);
-  if (gt == 0) *hcache = with_gf ? K.h : __int_as_float(0x7fc00000);
-  bool active = t < lo.n; // the same for a query's kSplit threads (one warp holds whole queries)
-  uint32_t i = active ? (order ? order[t] : t) : 0u;
-  f3 xi = {0.0f, 0.0f, 0.0f};
-  int cell = -1;
-  float lo3[3] = {0.0f, 0.0f, 0.0f}, hi3[3] = {0.0f, 0.0f, 0.0f};
-  if (active) {
-    float4 x4 = qpos[i];
-    xi = mk3(x4);
-    cell = gv.s2c[gv.r2s[gv.goff[q] + i]];
-    int4 cg = gv.cell_gi[cell];
-    bool inside = face_bounds(x4.x, gv.rinv, cg.x, lo3[0], hi3[0]);
-    inside = face_bounds(x4.y, gv.rinv, cg.y, lo3[1], hi3[1]) && inside;
-    inside = face_bounds(x4.z, gv.rinv, cg.z, lo3[2], hi3[2]) && inside;
-    if (!inside)
-      for (int a = 0; a < 3; ++a) lo3[a] = hi3[a] = 0.0f;
-  }
-  int v0 = split_first_visit(sub), v1 = sub + 1 < kSplit ? split_first_visit(sub + 1) : 27;
-  // 1. per group: hits, the first hit's index, the index range
-  uint32_t cnt[NG], first[NG];
-  int32_t mn[NG], mx[NG];
-#pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    cnt[g] = 0u;
-    first[g] = 0u;
-    mn[g] = INT32_MAX;
-    mx[g] = INT32_MIN;
-  }
-  if (active)
-    split_walk(gv, xs, cell, lo3, hi3, v0, v1, xi, [&](int s) {
-      uint32_t h = __float_as_uint(xs[s].w);
-      uint32_t g = h >> 28, j = h & 0x0FFFFFFFu;
-#pragma unroll
-      for (int qq = 0; qq < NG; ++qq)
-        if (qq == int(g)) {
-          if (cnt[qq] == 0u) first[qq] = j;
-          mn[qq] = min(mn[qq], int32_t(j));
-          mx[qq] = max(mx[qq], int32_t(j));
-          ++cnt[qq];
-        }
-    });
-  // 2. the query's rows: each part's first entry, the count, base and form
-  uint32_t pre[NG], total[NG], j0[NG];
-  bool wide[NG];
-#pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    uint32_t x = cnt[g];
-#pragma unroll
-    for (int o = 1; o < kSplit; o <<= 1) {
-      uint32_t y = __shfl_up_sync(kFull, x, o, kSplit);
-      if (sub >= o) x += y;
-    }
-    pre[g] = x - cnt[g];
-    total[g] = __shfl_sync(kFull, x, kSplit - 1, kSplit);
-    int src = cnt[g] ? sub : kSplit;
-    int32_t lo_j = mn[g], hi_j = mx[g];
-#pragma unroll
-    for (int o = 1; o < kSplit; o <<= 1) {
-      src = min(src, __shfl_xor_sync(kFull, src, o, kSplit));
-      lo_j = min(lo_j, __shfl_xor_sync(kFull, lo_j, o, kSplit));
-      hi_j = max(hi_j, __shfl_xor_sync(kFull, hi_j, o, kSplit));
-    }
-    j0[g] = __shfl_sync(kFull, first[g], src < kSplit ? src : 0, kSplit);
-    if (src >= kSplit) j0[g] = 0u;
-    wide[g] = total[g] > 0u && (hi_j - int32_t(j0[g]) > 32767 || lo_j - int32_t(j0[g]) < -32768);
-  }
-  if (!active) return;
-  // 3. the entries at their places
-  uint32_t run[NG];
-#pragma unroll
-  for (int g = 0; g < NG; ++g) run[g] = pre[g];
-  split_walk(gv, xs, cell, lo3, hi3, v0, v1, xi, [&](int s) {
-    float4 xj = xs[s];
-    uint32_t h = __float_as_uint(xj.w);
-    uint32_t g = h >> 28, j = h & 0x0FFFFFFFu;
-    float f = with_gf ? kgrad_factor(K, nsq3(sub3(xi, mk3(xj)))) : 0.0f;
-#pragma unroll
-    for (int qq = 0; qq < NG; ++qq)
-      if (qq == int(g)) {
-        uint32_t k = run[qq]++;
-        if (k < lo.cap[qq]) {
-          unsigned char *ch = lo.chunks[qq] + chunk_unit(k / kChunk, lo.n, i, 0);
-          if (wide[qq]) lo.idx32[qq][size_t(i) * lo.cap[qq] + k] = j;
-          else reinterpret_cast<uint16_t *>(ch)[k % kChunk] = uint16_t(uint32_t(int32_t(j - j0[qq])) & 0xFFFFu);
-          if (lo.with_gf) *factor_word(ch, k % kChunk) = __float_as_uint(f);
-        }
-      }
-  });
-  if (sub != 0) return;
-#pragma unroll
-  for (int g = 0; g < NG; ++g) {
-    if (g >= lo.G) break;
-    uint32_t n = total[g];
-    lo.cb[size_t(g) * lo.n + i] = make_uint2(n | (wide[g] ? kWide : 0u), j0[g]);
-    atomicMax(&lo.maxcnt[g], n);
-    if (n > lo.cap[g] || n % kChunk == 0) continue;
-    // the partial last chunk (and half-chunk of a wide row), zero-filled
-    unsigned char *ch = lo.chunks[g] + chunk_unit(n / kChunk, lo.n, i, 0);
-    if (wide[g]) {
-      for (uint32_t e = n; e % 8; ++e) lo.idx32[g][size_t(i) * lo.cap[g] + e] = 0u;
-    } else {
-      for (uint32_t slot = n % kChunk; slot < kChunk; ++slot) reinterpret_cast<uint16_t *>(ch)[slot] = 0u;
-    }
-    if (lo.with_gf)
-      for (uint32_t slot = n % kChunk; slot < kChunk; ++slot) *factor_word(ch, slot) = 0u;
-  }
+void launch_build_lists_warp(size_t N, cudaStream_t s, GridView const &gv, float4 const *xs, int q, ListOut const &lo,
+                             float const *h, float *hcache) {
+  unsigned nb = div_up(div_up(N, kWinItems), kWarps);
+  if (h) k_build_lists_warp<NG, true><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache);
+  else k_build_lists_warp<NG, false><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache);
 }
 
 template <int NG, bool STAGE>
@@ -1765,10 +1905,18 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
     k_xsorted<<<div_up(N_, 256), 256, 0, s>>>(pt, sorted_vals_, N_, xsorted_); count_launch();
     PG_LAUNCH_CHECK();
   }
-  // a group that is not in cell order (never permuted, or resized since) is
-  // walked in grid order
+  // staged lists: with factors, for a group in cell order, at most two
+  // neighbour groups (the staged sweeps' layout)
+  bool ordered = !in_grid_[q] || n == 0 || permuted_count_[q] == n;
+  bool st = stage && h && in_grid_[q] && ordered && G <= 2;
+  // one warp per run of queries of the grid; a group outside it (each query
+  // looks up its own cells), more than two neighbour groups and staged lists
+  // take a thread per query
+  bool warp = !st && in_grid_[q] && G <= 2 && model_->tune.v[kTuneListSplit] != 0;
+  // with a thread per query, a group that is not in cell order (never
+  // permuted, or resized since) is walked in grid order
   uint32_t const *order = nullptr;
-  if (in_grid_[q] && n > 0 && permuted_count_[q] != n) {
+  if (!ordered && !warp) {
     if (n > order_cap_) {
       if (order_) PG_CUDA(cudaFree(order_));
       order_cap_ = n + n / 8;
@@ -1780,9 +1928,6 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
     PG_LAUNCH_CHECK();
     order = order_;
   }
-  // staged lists: with factors, for a group in cell order, at most two
-  // neighbour groups (the staged sweeps' layout)
-  bool st = stage && h && in_grid_[q] && !order && G <= 2;
   if (st != L.staged) {
     // a change of form reallocates every list of the group
     for (int g = 0; g < kMaxGroups; ++g) L.cap[g] = 0;
@@ -1862,11 +2007,11 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
     float4 const *qpos = static_cast<float4 const *>(gg_[q].pos->d);
     {
       ProfScope ps(model_->prof, "nhood_lists", s);
-      bool split = !st && model_->tune.v[kTuneListSplit] != 0 && n <= kSplitMaxQueries && in_grid_[q] && G <= 2;
-      if (split) {
-        unsigned nb2 = unsigned(div_up(n * kSplit, size_t(kSplitNT)));
-        if (G == 1) k_build_lists_split<1><<<nb2, kSplitNT, 0, s>>>(gv, xsorted_, qpos, q, lo, h, L.hcache, order);
-        else k_build_lists_split<2><<<nb2, kSplitNT, 0, s>>>(gv, xsorted_, qpos, q, lo, h, L.hcache, order);
+      if (warp) {
+        // a group that grew since the grid's update: no neighbours of items the grid does not hold
+        if (size_t(goff_[q + 1] - goff_[q]) != n) PG_CUDA(cudaMemsetAsync(L.cb, 0, size_t(G) * n * sizeof(uint2), s));
+        if (G == 1) launch_build_lists_warp<1>(N_, s, gv, xsorted_, q, lo, h, L.hcache);
+        else launch_build_lists_warp<2>(N_, s, gv, xsorted_, q, lo, h, L.hcache);
       } else if (st) {
         if (G == 1) launch_build_lists<1, true>(n, smem, s, gv, xsorted_, qpos, q, lo, h, L.hcache, order);
         else launch_build_lists<2, true>(n, smem, s, gv, xsorted_, qpos, q, lo, h, L.hcache, order);

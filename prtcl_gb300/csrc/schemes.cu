@@ -1848,7 +1848,7 @@ std::string tune_knob_table() {
   t += "jacobi_unroll 1 1=1 2=2 4=4\n";
   t += "staging 0 0=off 1=staged lists and sweeps (unbatched models)\n";
   t += "grid_sort 1 0=tiled launches 1=one cluster launch for grids of at most 128k items\n";
-  t += "list_split 1 0=one thread per query 1=four threads per query for query groups of at most 64k items\n";
+  t += "list_split 1 0=one thread per query 1=one warp per run of queries of a cell\n";
   return t;
 }
 

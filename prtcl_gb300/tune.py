@@ -15,8 +15,8 @@ the tuner is free to pick the fastest per workload:
 * grid_sort (single-scene models whose grid holds at most 128k items)
   sorts the grid in one launch of a thread-block cluster instead of the
   tiled radix-sort launches (0 or 1);
-* list_split (query groups of at most 64k items) builds each query's lists
-  with four threads, each walking a quarter of its cells (0 or 1).
+* list_split builds the lists with one warp per run of queries of a cell
+  instead of one thread per query (0 or 1).
 
 The cell size is not a knob: it equals the search radius, as in the
 reference's grid (util/grouped_uniform_grid.hpp:621-632), because the
@@ -177,7 +177,8 @@ class PlainTarget:
         self.d, self.loop, self.n = scene, loop, probe_steps
         self.viscosity = bool(loop.p.get("viscosity"))
         # items of the grid (fluid and boundary) and of the fluid group, where
-        # known: grid_sort and list_split are knobs only for the sizes they take
+        # known: grid_sort is a knob only for the sizes it takes, list_split
+        # only where its two forms are less than 2x apart
         self.grid_items = float("inf") if grid_items is None else grid_items
         self.fluid_items = float("inf") if fluid_items is None else fluid_items
 
