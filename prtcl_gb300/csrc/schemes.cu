@@ -46,6 +46,22 @@ constexpr int kSPcg = 0;     // scalars[0..7]: PCG
 constexpr int kSJacobi = 16; // scalars[16]: FP64 density error
 constexpr int kStPcgIter = 0, kStPcgActive = 1, kStPcgBody = 2;
 constexpr int kStJacIter = 4, kStJacDone = 5;
+// The relaxed-Jacobi loop starts from the pressure that setup has just set to
+// zero, so its first iteration needs no neighbours: with p = 0 every term of
+// the pressure acceleration is a zero, hence a = +0, hence every term of
+// iteration_pressure's sum is a zero, hence the sum is +0 (sums that start at
+// +0 and add or subtract zeros of either sign stay +0).  That holds while all
+// masses, volumes, densities and kernel gradients of the pairs are finite;
+// setup's helper sum c walks the same pairs with the same factors, and is not
+// finite where one of them is not (every item in the grid is its own
+// neighbour, so its own mass and density count too).  Setup notes what it
+// found (kStSetupBad, and in scalars[kSSetup..] the smoothing scale and rest
+// densities it used), the host checks that no field, list or pressure has
+// changed since, and k_jacobi_begin sets kStJacFirst where both agree.  Of
+// the 4 to 5 iterations a step takes, this takes out one pair of sweeps:
+// %MEASURED%
+constexpr int kStJacFirst = 6, kStSetupBad = 7; // kStSetupBad: 0 after a clean setup, until a solve takes it
+constexpr int kSSetup = 32; // scalars[32]: smoothing scale, then one rest density per fluid group
 
 // ---------------------------------------------------------------------------
 // argument structs
@@ -469,7 +485,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
                                                                  float const *__restrict__ rho, float *__restrict__ p,
                                                                  float *__restrict__ pr, float *__restrict__ s,
                                                                  float *__restrict__ AA, float const *rho0p, Globals G,
-                                                                 Nbrs<NF, NB> N) {
+                                                                 Nbrs<NF, NB> N, int *bad) {
   uint32_t i = grid_tid();
   if (i >= n) return;
   KernelParams K = kparams(*G.h);
@@ -495,6 +511,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
     });
   }
   cout[i] = make_float4(c.x, c.y, c.z, 0.0f);
+  if (!(isfinite(c.x) && isfinite(c.y) && isfinite(c.z))) *bad = 1;
   f3 vi = mk3(v[i]), ci = c;
   float mi = m[i];
   float sa = 0.0f, aa = 0.0f;
@@ -528,7 +545,26 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
   AA[i] = aa * ((dt * dt) * (rho0 / ri));
 }
 
-__global__ void k_set_i32(int *p, int v) { *p = v; }
+// before and after the set-up sweeps
+__global__ void k_setup_begin(int *status) { status[kStSetupBad] = 0; }
+struct RestDensities {
+  float const *p[kMaxNbrGroups];
+  int n;
+};
+__global__ void k_setup_end(int *nprde, int total, Globals G, RestDensities D, double *scalars) {
+  *nprde = total;
+  scalars[kSSetup] = double(*G.h);
+  for (int k = 0; k < D.n; ++k) scalars[kSSetup + 1 + k] = double(*D.p[k]);
+}
+// whether the loop's first iteration may take zero sums (see kStJacFirst):
+// `same` is the host's part
+__device__ __forceinline__ int jacobi_first(Globals const &G, RestDensities const &D, int *status,
+                                            double const *scalars, int same) {
+  bool ok = same && !status[kStSetupBad] && scalars[kSSetup] == double(*G.h);
+  for (int k = 0; k < D.n; ++k) ok = ok && scalars[kSSetup + 1 + k] == double(*D.p[k]) && isfinite(*D.p[k]);
+  status[kStSetupBad] = 1; // the solve changes the pressure
+  return ok ? 1 : 0;
+}
 
 // iisph.iteration_pressure_acceleration (schemes/iisph.hpp:358-423).
 // `done` (device-loop mode) skips the work once the loop has converged.
@@ -566,9 +602,15 @@ template <int NF, int NB, int NT = kNT, int MINB = kMinBlocks, int BT = 8>
 __global__ void __launch_bounds__(NT, MINB) k_iisph_accel(uint32_t n, float4 const *__restrict__ x, float const *__restrict__ p,
                                                      float const *__restrict__ rho, float4 *__restrict__ a,
                                                      float const *rho0p, Globals G, Nbrs<NF, NB> N, int const *done) {
-  if (done && *(volatile int const *)done) return;
+  // (the two words are loaded together)
+  int ended = done ? *(volatile int const *)done : 0, first = done ? *(volatile int const *)(done + 1) : 0;
+  if (ended) return;
   uint32_t i = grid_tid();
   if (i >= n) return;
+  if (first) {
+    a[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    return;
+  }
   KernelParams K = kparams(*G.h);
   iisph_accel_item<NF, NB, BT>(i, x, p, rho, a, K, use_cache(N, K), *rho0p, N);
 }
@@ -578,7 +620,9 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_accel(uint32_t n, float4 con
 template <int NF, int NB, int MINB = kMinBlocks, int BT = 8, bool DYN = false>
 __global__ void __launch_bounds__(kNT, MINB) k_iisph_accel_seg(float4 const *__restrict__ x, float const *__restrict__ p,
                                                          float const *__restrict__ rho, float4 *__restrict__ a,
-                                                         float const *rho0p, Globals G, Nbrs<NF, NB> N, SegArgs S) {
+                                                         float const *rho0p, Globals G, Nbrs<NF, NB> N, SegArgs S,
+                                                         int const *first) {
+  bool zero = *(volatile int const *)first != 0;
   KernelParams K = kparams(*G.h);
   bool uc = use_cache(N, K);
   float rho0 = *rho0p;
@@ -594,7 +638,10 @@ __global__ void __launch_bounds__(kNT, MINB) k_iisph_accel_seg(float4 const *__r
     if (t >= na) break;
     uint4 T = S.tiles[S.active[t]];
     uint32_t i = T.y + threadIdx.x;
-    if (i < T.z) iisph_accel_item<NF, NB, BT>(i, x, p, rho, a, K, uc, rho0, N);
+    if (i < T.z) {
+      if (zero) a[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      else iisph_accel_item<NF, NB, BT>(i, x, p, rho, a, K, uc, rho0, N);
+    }
     if (!DYN) t += gridDim.x;
   }
 }
@@ -656,13 +703,19 @@ __device__ __forceinline__ double iisph_pressure_item(uint32_t i, PressureArgs c
 template <int NF, int NB, int MINB = kMinBlocks, int BT = 16>
 __global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure(uint32_t n, PressureArgs A, Globals G, Nbrs<NF, NB> N, Red R,
                                                         int first, int last_group, int const *done) {
-  if (done && *(volatile int const *)done) return;
+  int ended = done ? *(volatile int const *)done : 0, zero = done ? *(volatile int const *)(done + 1) : 0;
+  if (ended) return;
   KernelParams K = kparams(*G.h);
   bool uc = use_cache(N, K);
   float rho0 = *A.rho0, dt = *G.dt, omega = *G.omega;
   double part = 0.0;
-  for (uint32_t i = grid_tid(); i < n; i += gridDim.x * blockDim.x)
-    part += iisph_pressure_item<NF, NB, BT>(i, A, K, uc, rho0, dt, omega, N);
+  if (zero) {
+    for (uint32_t i = grid_tid(); i < n; i += gridDim.x * blockDim.x)
+      part += pressure_finish(i, A, 0.0f, rho0, dt, omega);
+  } else {
+    for (uint32_t i = grid_tid(); i < n; i += gridDim.x * blockDim.x)
+      part += iisph_pressure_item<NF, NB, BT>(i, A, K, uc, rho0, dt, omega, N);
+  }
   double v[1] = {part}, out[1];
   if (reduce_commit<1>(v, R, out) && threadIdx.x == 0) {
     double start = first ? (done ? 0.0 : double(*G.aprde)) : R.scalars[kSJacobi];
@@ -677,7 +730,9 @@ __global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure(uint32_t n, Pressu
 // (DYN: a persistent grid whose blocks take tiles from a work counter; the
 // per-tile partial sums and their per-slot commit are unchanged)
 template <int NF, int NB, int MINB = kMinBlocks, int BT = 16, bool DYN = false>
-__global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure_seg(PressureArgs A, Globals G, Nbrs<NF, NB> N, SegArgs S) {
+__global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure_seg(PressureArgs A, Globals G, Nbrs<NF, NB> N, SegArgs S,
+                                                                  int const *first) {
+  bool zero = *(volatile int const *)first != 0;
   // one active tile per block (the hardware's block scheduling balances the
   // tiles' uneven costs); the blocks past the active tiles exit at once
   uint32_t na = S.nactive[0];
@@ -698,7 +753,10 @@ __global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure_seg(PressureArgs A
     uint4 T = S.tiles[t];
     uint32_t slot = T.x;
     uint32_t i = T.y + threadIdx.x;
-    double part = (i < T.z) ? iisph_pressure_item<NF, NB, BT>(i, A, K, uc, rho0, dt, omega, N) : 0.0;
+    double part = 0.0;
+    if (i < T.z)
+      part = zero ? pressure_finish(i, A, 0.0f, rho0, dt, omega)
+                  : iisph_pressure_item<NF, NB, BT>(i, A, K, uc, rho0, dt, omega, N);
     double v[1] = {part}, out[1];
     if (seg_commit<1>(v, S, slot, out, t) && threadIdx.x == 0) S.scal[slot * kSegScal + kSsAprde] = out[0];
     if (!DYN) break;
@@ -817,7 +875,11 @@ __global__ void __launch_bounds__(kNT, 4) k_iisph_pressure_staged(uint32_t n, Pr
 }
 
 // per-slot loop start: a slot without fluid items does not iterate
-__global__ void k_seg_jacobi_begin(SegArgs S) {
+__global__ void k_seg_jacobi_begin(SegArgs S, Globals G, Red R, RestDensities D, int same) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    R.status[kStJacDone] = 0;
+    R.status[kStJacFirst] = jacobi_first(G, D, R.status, R.scalars, same);
+  }
   for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < S.slots; k += gridDim.x * blockDim.x) {
     S.stat[k * kSegStat + kStJacIter] = 0;
     S.stat[k * kSegStat + kStJacDone] = (S.nprde[k] >= 1) ? 0 : 1;
@@ -829,7 +891,7 @@ __global__ void k_seg_jacobi_begin(SegArgs S) {
 // 0 solves, 1 iterations, 2 solves stopped at the cap, 3 largest final
 // aprde / nprde, 7 final aprde / nprde of the last solve
 __global__ void k_seg_jacobi_control(Globals G, SegArgs S, cudaGraphConditionalHandle h, int use_handle,
-                                     int kernels, int *all_done) {
+                                     int kernels, int *all_done, int *first) {
   int any = 0;
   int maxit = *G.jac_max > 0 ? *G.jac_max : 100;
   float eta = *G.jac_eta > 0.0f ? *G.jac_eta : 1e-3f;
@@ -864,6 +926,7 @@ __global__ void k_seg_jacobi_control(Globals G, SegArgs S, cudaGraphConditionalH
   }
   if (threadIdx.x == 0) {
     *all_done = any ? 0 : 1;
+    *first = 0;
     if (kernels) atomicAdd(&g_loop_kernels, (unsigned long long)kernels);
     if (use_handle) cudaGraphSetConditional(h, any ? 1u : 0u);
   }
@@ -871,7 +934,8 @@ __global__ void k_seg_jacobi_control(Globals G, SegArgs S, cudaGraphConditionalH
 
 // relaxed-Jacobi loop control (share/scripts/prtcl-lua.example.lua:409-420):
 // at least two iterations; stop when aprde / nprde < eta or at the cap
-__global__ void k_jacobi_begin(Globals G, Red R) {
+__global__ void k_jacobi_begin(Globals G, Red R, RestDensities D, int same) {
+  R.status[kStJacFirst] = jacobi_first(G, D, R.status, R.scalars, same);
   R.status[kStJacIter] = 0;
   R.status[kStJacDone] = (*G.nprde >= 1) ? 0 : 1;
   *G.jac_iters = 0;
@@ -887,6 +951,7 @@ __global__ void k_jacobi_control(Globals G, Red R, cudaGraphConditionalHandle h,
     bool converged = it >= 2 && rel < double(eta);
     if (converged || it >= maxit || it >= 100000) done = 1;
     R.status[kStJacDone] = done;
+    R.status[kStJacFirst] = 0;
     *G.jac_iters = it;
     if (done) {
       R.stats[0] += 1.0;
@@ -2278,7 +2343,8 @@ public:
         using Sh = decltype(sh);
         k_iisph_setup<NF, NB, Sh::nt, Sh::minb, Sh::bt><<<div_up(n, Sh::nt), Sh::nt, 0, s>>>(
             n, dptr<float4>(F.x), dptr<float4>(F.v), dptr<float4>(F.c), dptr<float>(F.m), dptr<float>(F.rho),
-            dptr<float>(F.p), pr, dptr<float>(F.s), dptr<float>(F.AA), S->u(F.rho0), G, N);
+            dptr<float>(F.p), pr, dptr<float>(F.s), dptr<float>(F.AA), S->u(F.rho0), G, N,
+            S->model_->status_d + kStSetupBad);
       });
       count_launch();
     }
@@ -2324,12 +2390,12 @@ public:
         if (SA->ntiles) {
           if (NF == 1 && NB == 1 && tv == 4)
             k_iisph_accel_seg<NF, NB, kMinBlocks, 8, true><<<std::min(SA->ntiles, kActiveBlocks), kNT, 0, s>>>(
-                x, p, rho, a, rho0, G, N, *SA);
+                x, p, rho, a, rho0, G, N, *SA, S->model_->status_d + kStJacFirst);
           else
             with_shape<AccelSegShapes, NF == 1 && NB == 1>(tv, [&](auto sh) {
               using Sh = decltype(sh);
               k_iisph_accel_seg<NF, NB, Sh::minb, Sh::bt><<<std::min(SA->ntiles, kActiveBlocks), kNT, 0, s>>>(
-                  x, p, rho, a, rho0, G, N, *SA);
+                  x, p, rho, a, rho0, G, N, *SA, S->model_->status_d + kStJacFirst);
             });
         }
       } else {
@@ -2377,12 +2443,14 @@ public:
       } else if (SA && NF == 1 && NB == 1 && tvp == 4) {
         if (SA->ntiles)
           k_iisph_pressure_seg<NF, NB, kMinBlocks, 16, true><<<std::min(SA->ntiles, kActiveBlocks), kNT, 0, s>>>(
-              PA, G, N, *SA);
+              PA, G, N, *SA, S->model_->status_d + kStJacFirst);
       } else
       with_shape<PressureShapes, NF == 1 && NB == 1>(tvp, [&](auto sh) {
         using Sh = decltype(sh);
         if (SA) {
-          if (SA->ntiles) k_iisph_pressure_seg<NF, NB, Sh::minb, Sh::bt><<<SA->ntiles, kNT, 0, s>>>(PA, G, N, *SA);
+          if (SA->ntiles)
+            k_iisph_pressure_seg<NF, NB, Sh::minb, Sh::bt><<<SA->ntiles, kNT, 0, s>>>(
+                PA, G, N, *SA, S->model_->status_d + kStJacFirst);
         } else {
           k_iisph_pressure<NF, NB, Sh::minb, Sh::bt><<<red_grid(n), kNT, 0, s>>>(n, PA, G, N, R, first, last, done);
         }
@@ -2414,6 +2482,7 @@ public:
     int nf = int(fluid_.size()), nb = int(bound_.size());
     // one fused sweep per group (pass 2 of a group reads only its own c)
     long long total = 0;
+    k_setup_begin<<<1, 1, 0, s>>>(model_->status_d); count_launch();
     for (auto *F : active()) {
       total += (long long)F->g->count;
       dispatch_fb<SETUP>(nf, nb, this, *F, lists(nh, F->g, G, s), G, s);
@@ -2424,8 +2493,38 @@ public:
       wrote_pressure(*F);
     }
     // nprde = number of fluid particles (the generated reduction adds 1 per particle)
-    k_set_i32<<<1, 1, 0, s>>>(G.nprde, int(total)); count_launch();
+    k_setup_end<<<1, 1, 0, s>>>(G.nprde, int(total), G, rest_densities(), model_->scalars_d); count_launch();
     PG_LAUNCH_CHECK();
+    if (capturing(s)) zero_key_.clear(); // queued for later, possibly more than once
+    else zero_key_ = zero_key(nh, s);
+  }
+  static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    PG_CUDA(cudaStreamIsCapturing(s, &c));
+    return c != cudaStreamCaptureStatusNone;
+  }
+  RestDensities rest_densities() {
+    RestDensities D{};
+    for (auto &F : fluid_)
+      if (D.n < kMaxNbrGroups) D.p[D.n++] = u(F.rho0);
+    return D;
+  }
+  // What the first iteration's zero sums rest on (kStJacFirst): the fields
+  // that setup read, the pressure it wrote, the grid of its lists and the
+  // stream it ran on.  A solve takes them only where the key is still the
+  // same; it is cleared by the solve, which changes the pressure.
+  std::vector<uint64_t> zero_key(Nhood &nh, cudaStream_t s) {
+    std::vector<uint64_t> k{reinterpret_cast<uint64_t>(&nh), nh.epoch(), reinterpret_cast<uint64_t>(s)};
+    auto add = [&](Group *g, std::initializer_list<VaryingField const *> fs) {
+      k.push_back(uint64_t(g->count));
+      for (auto *f : fs) {
+        k.push_back(reinterpret_cast<uint64_t>(f->d));
+        k.push_back(f->version);
+      }
+    };
+    for (auto &F : fluid_) add(F.g, {F.x, F.m, F.rho, F.p});
+    for (auto &B : bound_) add(B.g, {B.x, B.V});
+    return k;
   }
   void no_segments(char const *what) {
     for (auto &F : fluid_)
@@ -2494,12 +2593,15 @@ public:
     StageArgs st{};
     bool staged = !seg && act.size() == 1 && stage_args(nh, *views[0], *act[0], st);
     StageArgs const *stp = staged ? &st : nullptr;
+    // (the staged sweeps take every iteration in full)
+    int same = !staged && !zero_key_.empty() && !capturing(s) && zero_key_ == zero_key(nh, s) ? 1 : 0;
+    zero_key_.clear();
     if (seg) {
-      k_seg_jacobi_begin<<<div_up(std::max<uint32_t>(SA.slots, 1), 256), 256, 0, s>>>(SA); count_launch();
+      k_seg_jacobi_begin<<<div_up(std::max<uint32_t>(SA.slots, 1), 256), 256, 0, s>>>(SA, G, R, rest_densities(), same);
+      count_launch();
       k_seg_active<<<1, 1024, 0, s>>>(SA); count_launch();
-      k_set_i32<<<1, 1, 0, s>>>(R.status + kStJacDone, 0); count_launch();
     } else {
-      k_jacobi_begin<<<1, 1, 0, s>>>(G, R); count_launch();
+      k_jacobi_begin<<<1, 1, 0, s>>>(G, R, rest_densities(), same); count_launch();
     }
     PG_LAUNCH_CHECK();
     int kernels = 2 * int(act.size()) + 1;
@@ -2518,7 +2620,7 @@ public:
         if (sig) return;
         if (seg) {
           k_seg_jacobi_control<<<1, 1024, 0, cs>>>(G, SA, h, use_handle ? 1 : 0, use_handle ? kernels : 0,
-                                                   R.status + kStJacDone);
+                                                   R.status + kStJacDone, R.status + kStJacFirst);
         } else {
           k_jacobi_control<<<1, 1, 0, cs>>>(G, R, h, use_handle ? 1 : 0, use_handle ? kernels : 0);
         }
@@ -2553,6 +2655,7 @@ public:
 
 private:
   WhileLoop loop_;
+  std::vector<uint64_t> zero_key_;
 };
 
 // ---------------------------------------------------------------------------
