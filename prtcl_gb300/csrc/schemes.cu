@@ -58,8 +58,9 @@ constexpr int kStJacIter = 4, kStJacDone = 5;
 // found (kStSetupBad, and in scalars[kSSetup..] the smoothing scale and rest
 // densities it used), the host checks that no field, list or pressure has
 // changed since, and k_jacobi_begin sets kStJacFirst where both agree.  Of
-// the 4 to 5 iterations a step takes, this takes out one pair of sweeps:
-// %MEASURED%
+// the 4 to 5 iterations a step takes, this takes out one pair of sweeps (95 +
+// 138 us at 1M items; 11 us are left of them): set-up and solve of the 1M dam
+// break 1.54 -> 1.31 ms, of the 27k one 222 -> 204 us.
 constexpr int kStJacFirst = 6, kStSetupBad = 7; // kStSetupBad: 0 after a clean setup, until a solve takes it
 constexpr int kSSetup = 32; // scalars[32]: smoothing scale, then one rest density per fluid group
 
