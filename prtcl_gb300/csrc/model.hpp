@@ -154,7 +154,7 @@ enum TuneKnob : int {
   kTunePcgQ,
   kTuneJacobiUnroll,
   kTuneStaging,  // 1: staged lists and the staged Jacobi / PCG sweeps
-  kTuneGridSort, // 1: grids of at most 128k items sorted in one launch of a thread-block cluster
+  kTuneGridSort, // 1: grids built by counting, or sorted in one launch of a thread-block cluster (128k items); 0: radix sort
   kTuneListSplit, // 1: lists built by one warp per run of queries of a cell, 0: by one thread per query
   kTuneKnobs
 };

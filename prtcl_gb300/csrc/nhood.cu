@@ -15,6 +15,12 @@ namespace {
 constexpr uint32_t kFull = 0xffffffffu;
 
 // the 13 half-stencil offsets (util/grouped_uniform_grid.hpp:52-68)
+// (offset_of: the same for indices the compiler knows)
+__host__ __device__ constexpr int offset_of(int k, int a) {
+  constexpr int t[13][3] = {{1, 0, 0}, {0, 1, 0},  {0, 0, 1},  {1, 1, 0},   {1, 0, 1},  {0, 1, 1}, {1, 1, 1},
+                            {0, -1, 1}, {1, 0, -1}, {1, 1, -1}, {1, -1, -1}, {1, -1, 0}, {1, -1, 1}};
+  return t[k][a];
+}
 __constant__ int c_offsets[13][3] = {{1, 0, 0},  {0, 1, 0},   {0, 0, 1},  {1, 1, 0},  {1, 0, 1},
                                      {0, 1, 1},  {1, 1, 1},   {0, -1, 1}, {1, 0, -1}, {1, 1, -1},
                                      {1, -1, -1}, {1, -1, 0}, {1, -1, 1}};
@@ -60,6 +66,49 @@ __device__ __forceinline__ uint32_t key_pext(uint32_t u, KeyInfo const &k) {
   return r;
 }
 
+// the same for at most 10 bits, and back from every third bit of x
+__device__ __forceinline__ uint32_t spread3_10(uint32_t v) {
+  v = (v | v << 16) & 0x030000FFu;
+  v = (v | v << 8) & 0x0300F00Fu;
+  v = (v | v << 4) & 0x030C30C3u;
+  return (v | v << 2) & 0x09249249u;
+}
+__device__ __forceinline__ uint32_t compact3_10(uint32_t v) {
+  v &= 0x09249249u;
+  v = (v | v >> 2) & 0x030C30C3u;
+  v = (v | v >> 4) & 0x0300F00Fu;
+  v = (v | v >> 8) & 0x030000FFu;
+  return (v | v >> 16) & 0x3FFu;
+}
+// the table entry of a (short) cell key
+__device__ __forceinline__ uint32_t dir_index(uint32_t key, DirKey const &d) {
+  uint32_t r = 0;
+  for (int t = 0; t < d.nruns; ++t) r |= (key & d.mask[t]) >> d.shift[t];
+  return r;
+}
+// the biased grid index along axis a of table entry e (the inverse, for an
+// entry that an item maps to: its axis' deleted bits are bit 31, its opposite,
+// or bit 31 itself a constant), and whether an index can have an entry
+__device__ __forceinline__ uint32_t dir_axis(uint32_t e, int a, DirKey const &d, KeyInfo const &k) {
+  uint32_t key = 0;
+  for (int t = 0; t < d.nruns; ++t) key |= (e << d.shift[t]) & d.mask[t];
+  uint32_t r = compact3_10(key >> (2 - a)) & ((1u << k.bits) - 1u), u = 0;
+  if (k.nruns == 0) {
+    int b = 0;
+    for (uint32_t m = k.keep; m; m &= m - 1u, ++b)
+      if ((r >> b) & 1u) u |= m & (~m + 1u);
+  } else {
+    for (int t = 0; t < k.nruns; ++t) u |= (r << k.run_shift[t]) & k.run_mask[t];
+  }
+  DirAxis const &x = d.axis[a];
+  if (!(x.keep & 0x80000000u)) u |= x.b31_const;
+  return u | ((u >> 31) ? x.rel_eq : x.rel_ne);
+}
+__device__ __forceinline__ bool dir_valid(uint32_t u, DirAxis const &x) {
+  uint32_t t = u ^ ((u >> 31) ? 0xFFFFFFFFu : 0u);
+  return !(t & x.rel_eq) && !(~t & x.rel_ne) && ((x.keep & 0x80000000u) || (u & 0x80000000u) == x.b31_const);
+}
+
 __device__ __forceinline__ uint64_t make_key(uint32_t u0, uint32_t u1, uint32_t u2, KeyInfo const &k) {
   return (spread3(key_pext(u0, k)) << 2) | (spread3(key_pext(u1, k)) << 1) | spread3(key_pext(u2, k));
 }
@@ -85,6 +134,7 @@ __device__ __forceinline__ int32_t axis_gi(float x, float rinv, double radius) {
   float d = t - f;
   float near = fminf(d, 1.0f - d);
   if (near > fabsf(t) * 4.76837158203125e-07f + 1e-30f) return int32_t(f);
+  if (x == 0.0f) return 0; // (points clipped to a domain's edge come in numbers)
   return int32_t(floor(double(x) / radius));
 }
 __device__ __forceinline__ int3 x_to_gi(float4 x, GridView const &gv) {
@@ -402,55 +452,425 @@ __device__ __forceinline__ int group_of(uint32_t const *goff, int G, uint32_t n)
 // KEY: the key layout of the previous update is taken (it is confirmed
 // against these statistics before the grid is read), so the pass writes the
 // Z-order keys themselves (the work of k_cells_key) instead of the indices.
+// DIRECT: for a grid built by counting, also each item's place among its
+// cell's items (no handles).
 constexpr int kCellsUNT = 256;
-template <bool KEY>
-__global__ void __launch_bounds__(kCellsUNT) k_cells_u(const __grid_constant__ PosTable pt, GridView gv, int G, size_t N, uint32_t *ukeys,
-                                                       uint64_t *keys, uint32_t *vals, uint32_t *stats) {
-  __shared__ uint32_t sh[4][kCellsUNT / 32];
-  uint32_t ne = 0, eq = 0, a1 = 0, a0 = 0;
-  for (size_t n = blockIdx.x * size_t(blockDim.x) + threadIdx.x; n < N; n += size_t(gridDim.x) * blockDim.x) {
-    int g = group_of(gv.goff, G, uint32_t(n));
-    uint32_t i = uint32_t(n) - gv.goff[g];
-    int3 gi = x_to_gi(pt.pos[g][i], gv);
-    uint32_t u[3] = {unsign(gi.x), unsign(gi.y), unsign(gi.z)};
-    for (int a = 0; a < 3; ++a) {
-      uint32_t t = u[a] ^ ((u[a] >> 31) ? 0xFFFFFFFFu : 0u);
-      ne |= t;
-      eq |= ~t;
-      a1 |= u[a] & 0x80000000u;
-      a0 |= ~u[a] & 0x80000000u;
+// words of the update's statistics: per axis two OR-reductions of the biased
+// grid indices u (bit b < 31 of the first: some u has bit b unlike its bit 31;
+// of the second: some u has it like it; bit 31: some u has bit 31, some has it
+// not), the fullest cell and a ticket; the longest rows of the list build
+// follow
+constexpr int kStMaxCell = 6, kStDirTicket = 7, kStRows = 8, kStWords = 16;
+struct DirTable {
+  uint32_t *count;   // items of each entry, then its first sorted index (zero between updates)
+  uint32_t *touched; // runs of kDirRun entries with items, a word every kMark (zero between updates)
+  uint32_t *cell_of; // an occupied entry's cell
+  DirKey key;
+};
+// A tile is what one block counts and fills, a run of it what one warp does.
+// (Many items mark the same run.  Marks side by side, or one per tile, made
+// these stores the longest part of the first pass for points in random order:
+// 136 and 97 us for 4M.)
+constexpr uint32_t kDirTile = 4096, kDirRun = 512, kMark = 8;
+// an item's entry and its place among the items of its cell (the first of an
+// entry marks the tile)
+__device__ __forceinline__ uint2 dir_place(DirTable const &T, uint32_t key) {
+  uint32_t e = dir_index(key, T.key);
+  return make_uint2(e, atomicAdd(T.count + e, 1u));
+}
+template <bool KEY, bool DIRECT>
+__global__ void __launch_bounds__(kCellsUNT, 5) k_cells_u(const __grid_constant__ PosTable pt, GridView gv, int G, size_t N, uint32_t *ukeys,
+                                                       uint64_t *keys, uint32_t *vals, uint32_t *stats,
+                                                       const __grid_constant__ DirTable T) {
+  __shared__ uint32_t sh[6][kCellsUNT / 32];
+  uint32_t st[6] = {};
+  // two items at a time, so that their loads (and their counts) are in flight
+  // together
+  size_t step = size_t(gridDim.x) * blockDim.x;
+  for (size_t n0 = blockIdx.x * size_t(blockDim.x) + threadIdx.x; n0 < N; n0 += 2 * step) {
+    float4 x[2];
+    uint32_t idx[2];
+    int grp[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      size_t n = min(n0 + r * step, N - 1);
+      grp[r] = group_of(gv.goff, G, uint32_t(n));
+      idx[r] = uint32_t(n) - gv.goff[grp[r]];
+      x[r] = pt.pos[grp[r]][idx[r]];
     }
-    if constexpr (KEY)
-      keys[n] = make_key(u[0], u[1], u[2], gv.key) | seg_key(gv, item_seg(gv, g, i));
-    else
-      reinterpret_cast<uint4 *>(ukeys)[n] = make_uint4(u[0], u[1], u[2], 0u);
-    vals[n] = (uint32_t(g) << 28) | i;
+    uint2 place[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      size_t n = n0 + r * step;
+      if (n >= N) break;
+      int3 gi = x_to_gi(x[r], gv);
+      uint32_t u[3] = {unsign(gi.x), unsign(gi.y), unsign(gi.z)};
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        // t's bits below 31: unlike bit 31; its bit 31: bit 31
+        uint32_t t = u[a] ^ uint32_t(int32_t(u[a]) >> 31 & 0x7FFFFFFF);
+        st[2 * a] |= t;
+        st[2 * a + 1] |= ~t;
+      }
+      if constexpr (KEY) {
+        uint64_t key = make_key(u[0], u[1], u[2], gv.key) | seg_key(gv, item_seg(gv, grp[r], idx[r]));
+        if constexpr (DIRECT) place[r] = dir_place(T, uint32_t(key));
+        else keys[n] = key;
+      } else {
+        reinterpret_cast<uint4 *>(ukeys)[n] = make_uint4(u[0], u[1], u[2], 0u);
+      }
+      if constexpr (!DIRECT) vals[n] = (uint32_t(grp[r]) << 28) | idx[r];
+    }
+    if constexpr (DIRECT) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        size_t n = n0 + r * step;
+        if (n >= N) break;
+        reinterpret_cast<uint2 *>(keys)[n] = place[r];
+        if (place[r].y == 0) T.touched[place[r].x / kDirRun * kMark] = 1u;
+      }
+    }
   }
-  ne = __reduce_or_sync(kFull, ne);
-  eq = __reduce_or_sync(kFull, eq);
-  a1 = __reduce_or_sync(kFull, a1);
-  a0 = __reduce_or_sync(kFull, a0);
   int w = threadIdx.x >> 5;
-  if ((threadIdx.x & 31) == 0) {
-    sh[0][w] = ne;
-    sh[1][w] = eq;
-    sh[2][w] = a1;
-    sh[3][w] = a0;
+#pragma unroll
+  for (int k = 0; k < 6; ++k) {
+    uint32_t v = __reduce_or_sync(kFull, st[k]);
+    if ((threadIdx.x & 31) == 0) sh[k][w] = v;
   }
   __syncthreads();
-  if (threadIdx.x < 4) {
+  if (threadIdx.x < 6) {
     uint32_t v = 0;
     for (int k = 0; k < kCellsUNT / 32; ++k) v |= sh[threadIdx.x][k];
     if (v) atomicOr(&stats[threadIdx.x], v);
   }
 }
 
-__global__ void k_cells_key(uint32_t const *ukeys, uint32_t const *vals, size_t N, GridView gv, uint64_t *keys) {
+template <bool DIRECT>
+__global__ void k_cells_key(uint32_t const *ukeys, uint32_t const *vals, size_t N, GridView gv, uint64_t *keys,
+                            const __grid_constant__ DirTable T) {
   size_t n = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
   if (n < N) {
     uint4 u = reinterpret_cast<uint4 const *>(ukeys)[n];
     uint32_t h = vals[n];
-    keys[n] = make_key(u.x, u.y, u.z, gv.key) | seg_key(gv, item_seg(gv, int(h >> 28), h & 0x0FFFFFFFu));
+    uint64_t key = make_key(u.x, u.y, u.z, gv.key) | seg_key(gv, item_seg(gv, int(h >> 28), h & 0x0FFFFFFFu));
+    if constexpr (DIRECT) {
+      uint2 place = dir_place(T, uint32_t(key));
+      reinterpret_cast<uint2 *>(keys)[n] = place;
+      if (place.y == 0) T.touched[place.x / kDirRun * kMark] = 1u;
+    } else {
+      keys[n] = key;
+    }
+  }
+}
+
+// ---------------------------------------------------------------------------
+// the grid by counting (grid_sort 1, short cell keys)
+// ---------------------------------------------------------------------------
+//
+// Where the cell keys are few bits long, a table with an entry per possible
+// key takes the place of the radix sort, of the cell flags and of the hash
+// table of the cell keys.  An entry's number is the key without the bits that
+// tell nothing on their own axis (a flat scene's tall axis alone needs the
+// high bits): 19 bits for the 27k dam break, 25 for 1M particles.  It grows
+// with the key, so the entries are in cell order.
+//   1. the first pass counts the items of each entry; the count an item finds
+//      is its place among its cell's items (k_cells_u<true, true>);
+//   2. items and cells before each tile of kDirTile entries (k_dir_sums, which
+//      reads touched tiles only; its last block scans the blocks' totals),
+//      then every occupied entry's cell and first sorted index, in key order
+//      (k_dir_fill);
+//   3. the handles at their places, cell by cell (k_dir_scatter);
+//   4. per cell its grid index and key, decoded from the entry, the 26
+//      adjacent cells, looked up by entry, and its items' cell (k_dir_adj).
+//      The table keeps cells of earlier updates; one is taken only if it is a
+//      cell of this update with that entry;
+//   5. the places within a cell follow the order in which the counting threads
+//      came, so each cell's handles are ranked by value: (group, raw index),
+//      the order a stable sort gives (k_dir_order).
+// A cell of k items is ranked with k comparisons per item; one of more than
+// kDirMaxCell items is left as it is, and the update is repeated with the
+// radix sort before anything reads the grid (the count of the fullest cell
+// is confirmed with the key statistics).
+// What bounds it: the latency of six short launches for small scenes, random
+// 4- to 16-byte accesses in L2 for points in random order.  Whole updates by
+// the launches' events, against the sort (one cluster launch below 128k items)
+// with its tables, and with the sorted positions that the list build gathered
+// on its own before: 27k dam break 96 -> 49 us, 1M 242 -> 110, 4M uniform
+// points in random order 535 -> 238, 1.5M clustered 337 -> 175.
+constexpr int kDirectBits = 27;
+constexpr uint32_t kDirNT = 256, kDirMaxCell = 256;
+static_assert(kDirNT / 32 * kDirRun == kDirTile, "a warp per run");
+
+__device__ __forceinline__ uint64_t block_excl_scan64(uint64_t v, uint64_t *sh /* kDirNT / 32 */, uint64_t &total) {
+  int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  uint64_t x = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    uint64_t y = __shfl_up_sync(kFull, x, o);
+    if (lane >= o) x += y;
+  }
+  if (lane == 31) sh[w] = x;
+  __syncthreads();
+  uint64_t pre = x - v;
+  total = 0;
+  for (int k = 0; k < int(kDirNT / 32); ++k) {
+    if (k < w) pre += sh[k];
+    total += sh[k];
+  }
+  __syncthreads();
+  return pre;
+}
+
+// The marks of the calling warp's run in up to 32 tiles (tile first + k * step
+// for bit k), and in `any` those of the whole block's
+__device__ __forceinline__ uint32_t dir_marks(DirTable const &T, uint32_t first, uint32_t step, uint32_t n, uint32_t &any) {
+  __shared__ uint32_t all;
+  uint32_t lane = threadIdx.x & 31, w = threadIdx.x / 32;
+  if (threadIdx.x == 0) all = 0u;
+  __syncthreads();
+  bool here = lane < n && T.touched[((first + lane * step) * (kDirTile / kDirRun) + w) * kMark] != 0u;
+  uint32_t m = __ballot_sync(kFull, here);
+  if (lane == 0 && m) atomicOr(&all, m);
+  __syncthreads();
+  any = all;
+  return m;
+}
+
+// A block takes the tiles [b * per, (b + 1) * per), at most 32: sums[t] is
+// (occupied entries << 32 | items) before tile t in its block, base[b] the
+// same before block b (tiles without items have no sums).
+constexpr uint32_t kDirBlocks = 152 * 16;
+static_assert((1u << kDirectBits) / kDirTile <= 32 * kDirBlocks, "a block's tiles in one word");
+__global__ void __launch_bounds__(kDirNT) k_dir_sums(const __grid_constant__ DirTable T, uint32_t tiles, uint32_t per,
+                                                     uint64_t *sums, uint64_t *base, uint32_t *stats, int *ncells,
+                                                     int32_t *cell_start) {
+  __shared__ uint64_t sh[kDirNT / 32];
+  __shared__ int last;
+  uint32_t fullest = 0, t0 = blockIdx.x * per, any;
+  uint32_t marks = dir_marks(T, t0, 1, min(per, tiles - t0), any);
+  uint64_t run = 0;
+  for (; any; any &= any - 1u) {
+    uint32_t k = uint32_t(__ffs(int(any)) - 1), t = t0 + k;
+    if (threadIdx.x == 0) sums[t] = run;
+    uint32_t first = t * kDirTile + threadIdx.x / 32 * kDirRun; // the warp's run
+    uint32_t items = 0, cells = 0;
+    if ((marks >> k) & 1u) {
+      uint4 const *p = reinterpret_cast<uint4 const *>(T.count + first);
+      uint4 a[kDirRun / 128];
+#pragma unroll
+      for (int v = 0; v < int(kDirRun / 128); ++v) a[v] = p[v * 32 + (threadIdx.x & 31)];
+#pragma unroll
+      for (int v = 0; v < int(kDirRun / 128); ++v) {
+        items += a[v].x + a[v].y + a[v].z + a[v].w;
+        cells += (a[v].x ? 1u : 0u) + (a[v].y ? 1u : 0u) + (a[v].z ? 1u : 0u) + (a[v].w ? 1u : 0u);
+        fullest = max(max(fullest, max(a[v].x, a[v].y)), max(a[v].z, a[v].w));
+      }
+      items = __reduce_add_sync(kFull, items);
+      cells = __reduce_add_sync(kFull, cells);
+    }
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x / 32] = uint64_t(cells) << 32 | items;
+    __syncthreads();
+    for (int k = 0; k < int(kDirNT / 32); ++k) run += sh[k];
+    __syncthreads();
+  }
+  fullest = __reduce_max_sync(kFull, fullest);
+  if ((threadIdx.x & 31) == 0 && fullest > __ldcg(&stats[kStMaxCell])) atomicMax(&stats[kStMaxCell], fullest);
+  if (threadIdx.x == 0) base[blockIdx.x] = run;
+  __threadfence();
+  if (threadIdx.x == 0) last = atomicAdd(&stats[kStDirTicket], 1u) == gridDim.x - 1 ? 1 : 0;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  constexpr uint32_t kPer = (kDirBlocks + kDirNT - 1) / kDirNT;
+  uint64_t v[kPer], mine = 0, total;
+#pragma unroll
+  for (uint32_t k = 0; k < kPer; ++k) {
+    uint32_t b = threadIdx.x * kPer + k;
+    v[k] = b < gridDim.x ? __ldcg(base + b) : 0ull;
+    mine += v[k];
+  }
+  uint64_t pre = block_excl_scan64(mine, sh, total);
+#pragma unroll
+  for (uint32_t k = 0; k < kPer; ++k) {
+    uint32_t b = threadIdx.x * kPer + k;
+    if (b < gridDim.x) base[b] = pre;
+    pre += v[k];
+  }
+  if (threadIdx.x == 0) {
+    *ncells = int(total >> 32);
+    cell_start[total >> 32] = int32_t(total & 0xFFFFFFFFu);
+  }
+}
+
+__global__ void __launch_bounds__(kDirNT) k_dir_fill(const __grid_constant__ DirTable T, uint32_t tiles, uint32_t per,
+                                                     uint64_t const *__restrict__ sums,
+                                                     uint64_t const *__restrict__ base,
+                                                     int32_t *__restrict__ cell_start, uint32_t *__restrict__ entry) {
+  __shared__ uint64_t sh[kDirNT / 32];
+  // (tiles with items lie together: neighbouring ones go to different blocks)
+  uint32_t any, marks = dir_marks(T, blockIdx.x, gridDim.x, (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x, any);
+  for (; any; any &= any - 1u) {
+    uint32_t k = uint32_t(__ffs(int(any)) - 1), t = blockIdx.x + k * gridDim.x;
+    bool here = (marks >> k) & 1u;
+    if (here && (threadIdx.x & 31) == 0) T.touched[(t * (kDirTile / kDirRun) + threadIdx.x / 32) * kMark] = 0u;
+    constexpr uint32_t kPer = kDirTile / kDirNT;
+    uint32_t e0 = t * kDirTile + threadIdx.x * kPer;
+    uint4 *p = reinterpret_cast<uint4 *>(T.count + e0), *pc = reinterpret_cast<uint4 *>(T.cell_of + e0);
+    uint32_t c[kPer] = {};
+    uint64_t mine = 0;
+    if (here)
+#pragma unroll
+      for (int v = 0; v < int(kPer / 4); ++v) {
+        uint4 a = p[v];
+        c[4 * v] = a.x;
+        c[4 * v + 1] = a.y;
+        c[4 * v + 2] = a.z;
+        c[4 * v + 3] = a.w;
+      }
+#pragma unroll
+    for (int k = 0; k < int(kPer); ++k) mine += c[k] ? (1ull << 32 | c[k]) : 0ull;
+    uint64_t total, run = base[t / per] + sums[t] + block_excl_scan64(mine, sh, total);
+    if (!mine) continue;
+#pragma unroll
+    for (int v = 0; v < int(kPer / 4); ++v) {
+      uint32_t id[4], first[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint32_t n = c[4 * v + k];
+        id[k] = uint32_t(run >> 32);
+        first[k] = n ? uint32_t(run) : 0u; // an empty entry's count stays zero (its cell is never taken)
+        if (n) {
+          cell_start[id[k]] = int32_t(first[k]);
+          entry[id[k]] = e0 + 4 * v + k;
+          run += 1ull << 32 | n;
+        }
+      }
+      p[v] = make_uint4(first[0], first[1], first[2], first[3]);
+      pc[v] = make_uint4(id[0], id[1], id[2], id[3]);
+    }
+  }
+}
+
+__global__ void k_dir_scatter(GridView gv, int G, uint2 const *__restrict__ places, uint32_t const *__restrict__ first,
+                              size_t N, uint32_t *__restrict__ vals) {
+  size_t n = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (n >= N) return;
+  uint2 kp = places[n];
+  int g = group_of(gv.goff, G, uint32_t(n));
+  vals[first[kp.x] + kp.y] = (uint32_t(g) << 28) | (uint32_t(n) - gv.goff[g]);
+}
+
+// (and the positions in that order, which the list build reads)
+__global__ void k_dir_order(const __grid_constant__ PosTable pt, uint32_t const *__restrict__ vals,
+                            int32_t const *__restrict__ s2c, int32_t const *__restrict__ cell_start, size_t N,
+                            uint32_t *__restrict__ out, float4 *__restrict__ xs) {
+  size_t s = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (s >= N) return;
+  uint32_t h = vals[s];
+  int c = s2c[s], b = cell_start[c], e = cell_start[c + 1], r = int(s);
+  float4 x = pt.pos[h >> 28][h & 0x0FFFFFFFu];
+  if (e - b <= int(kDirMaxCell)) { // (a fuller cell: repeated with the radix sort)
+    r = b;
+    for (int t = b; t < e; ++t) r += vals[t] < h ? 1 : 0;
+  }
+  out[r] = h;
+  x.w = __uint_as_float(h);
+  xs[r] = x;
+}
+
+// one thread per cell; a block's adjacency rows go out through shared memory,
+// so that the stores are whole lines
+constexpr int kDirAdjNT = 128, kDirAdjItems = 4096;
+static_assert(kDirAdjNT <= 256, "a cell of the block in 8 bits");
+__global__ void __launch_bounds__(kDirAdjNT) k_dir_adj(GridView gv, const __grid_constant__ DirTable T,
+                                                       uint32_t const *__restrict__ entry, uint64_t *cell_key,
+                                                       int4 *cell_gi, int32_t *adj, int32_t *s2c) {
+  __shared__ int32_t sh[kDirAdjNT * 26];
+  __shared__ int32_t start[kDirAdjNT + 1];
+  __shared__ uint8_t owner[kDirAdjItems];
+  int C = *gv.ncells;
+  for (int c0 = int(blockIdx.x) * kDirAdjNT; c0 < C; c0 += int(gridDim.x) * kDirAdjNT) {
+    int c = c0 + int(threadIdx.x), nc = min(kDirAdjNT, C - c0);
+    start[threadIdx.x] = gv.cell_start[min(c, C)];
+    if (threadIdx.x == 0) start[nc] = gv.cell_start[c0 + nc];
+    if (c < C) {
+      uint32_t e = entry[c];
+      T.count[e] = 0u; // for the next update
+      // the segment's part of the entry, and per axis the parts of the index
+      // before, at and after the cell's (an entry is the OR of its parts)
+      // (all ones where the index has no entry)
+      uint32_t key = 0, own = e, part[3][3];
+      int gi[3];
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        uint32_t u = dir_axis(e, a, T.key, gv.key);
+        gi[a] = int32_t(u - 0x7FFFFFFFu);
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+          uint32_t v = unsign(gi[a] + (o - 1));
+          uint32_t k = spread3_10(key_pext(v, gv.key)) << (2 - a);
+          if (o == 1) key |= k;
+          part[a][o] = dir_valid(v, T.key.axis[a]) ? dir_index(k, T.key) : 0xFFFFFFFFu;
+        }
+        own &= ~part[a][1];
+      }
+      cell_gi[c] = make_int4(gi[0], gi[1], gi[2], 0);
+      if (gv.seg_shift < 32) {
+        uint32_t full = 0;
+        for (int t = 0; t < T.key.nruns; ++t) full |= (e << T.key.shift[t]) & T.key.mask[t];
+        key |= full >> gv.seg_shift << gv.seg_shift;
+      }
+      cell_key[c] = key;
+      // 13 at a time: every entry's cell, then those cells' entries
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t d[13];
+        uint32_t at[13];
+#pragma unroll
+        for (int q = 0; q < 13; ++q) {
+          int sg = half ? -1 : 1, x = 1 + sg * offset_of(q, 0), y = 1 + sg * offset_of(q, 1), z = 1 + sg * offset_of(q, 2);
+          at[q] = own | part[0][x] | part[1][y] | part[2][z];
+          d[q] = at[q] != 0xFFFFFFFFu ? T.cell_of[at[q]] : 0xFFFFFFFFu;
+        }
+#pragma unroll
+        for (int q = 0; q < 13; ++q) {
+          bool is = d[q] < uint32_t(C) && entry[d[q]] == at[q];
+          sh[threadIdx.x * 26 + (half ? 25 - q : q)] = is ? int32_t(d[q]) : -1;
+        }
+      }
+    }
+    __syncthreads();
+    int words = nc * 26;
+    for (int w = int(threadIdx.x); w < words; w += kDirAdjNT) adj[size_t(c0) * 26 + w] = sh[w];
+    // the block's items' cells: noted by the cells' threads where they fit,
+    // else found among the block's first indices
+    int s0 = start[0], ns = start[nc] - s0;
+    if (ns <= kDirAdjItems) {
+      if (c < C)
+        for (int s = start[threadIdx.x] - s0, e = start[threadIdx.x + 1] - s0; s < e; ++s) owner[s] = uint8_t(threadIdx.x);
+      __syncthreads();
+      for (int s = int(threadIdx.x); s < ns; s += kDirAdjNT) s2c[s0 + s] = c0 + owner[s];
+    } else {
+      for (int s = s0 + int(threadIdx.x); s < s0 + ns; s += kDirAdjNT) {
+        int lo = 0, hi = nc - 1;
+        while (lo < hi) {
+          int mid = (lo + hi + 1) >> 1;
+          if (start[mid] <= s) lo = mid;
+          else hi = mid - 1;
+        }
+        s2c[s] = c0 + lo;
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// raw -> sorted, for the readers that start from an item
+__global__ void k_r2s(uint32_t const *__restrict__ vals, GridView gv, size_t N, int32_t *__restrict__ r2s) {
+  size_t s = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
+  if (s < N) {
+    uint32_t h = vals[s];
+    r2s[gv.goff[h >> 28] + (h & 0x0FFFFFFFu)] = int32_t(s);
   }
 }
 
@@ -482,7 +902,7 @@ __global__ void __launch_bounds__(kScanNT) k_cf_count(uint64_t const *__restrict
 // number of cell starts at or before s, minus one
 __global__ void __launch_bounds__(kScanNT) k_cf_fill(const __grid_constant__ PosTable pt, GridView gv, uint64_t const *__restrict__ keys,
                                                      uint32_t const *__restrict__ vals, uint32_t const *excl_tiles,
-                                                     size_t N, int32_t *s2c, int32_t *r2s, int32_t *cell_start,
+                                                     size_t N, int32_t *s2c, int32_t *cell_start,
                                                      uint64_t *cell_key, int4 *cell_gi, int *ncells,
                                                      int32_t *cell_adj) {
   __shared__ uint32_t sh[32];
@@ -516,7 +936,6 @@ __global__ void __launch_bounds__(kScanNT) k_cf_fill(const __grid_constant__ Pos
     s2c[si] = c;
     uint32_t h = vals[si];
     uint32_t g = h >> 28, i = h & 0x0FFFFFFFu;
-    r2s[gv.goff[g] + i] = int32_t(si);
     if (fl[k]) {
       cell_start[c] = int32_t(si);
       cell_key[c] = key[k];
@@ -1498,11 +1917,21 @@ void launch_build_lists(size_t n, size_t smem, cudaStream_t s, GridView const &g
   k_build_lists<NG, STAGE><<<div_up(n, kBuildNT), kBuildNT, smem, s>>>(gv, xs, qpos, q, lo, h, hcache, order);
 }
 
-__global__ void k_pair_count(uint2 const *cb, size_t n, unsigned long long *total) {
-  size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
-  unsigned long long c = (i < n) ? (cb[i].x & ~kWide) : 0u;
+// (one atomic per block of a resident grid: an atomic per warp on the one
+// word took 88 us for 4M rows, this 9)
+constexpr int kPairNT = 256;
+__global__ void __launch_bounds__(kPairNT) k_pair_count(uint2 const *cb, size_t n, unsigned long long *total) {
+  __shared__ unsigned long long sh[kPairNT / 32];
+  unsigned long long c = 0;
+  for (size_t i = blockIdx.x * size_t(kPairNT) + threadIdx.x; i < n; i += size_t(gridDim.x) * kPairNT)
+    c += cb[i].x & ~kWide;
   for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(kFull, c, o);
-  if ((threadIdx.x & 31) == 0 && c) atomicAdd(total, c);
+  if ((threadIdx.x & 31) == 0) sh[threadIdx.x / 32] = c;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int k = 1; k < kPairNT / 32; ++k) c += sh[k];
+    if (c) atomicAdd(total, c);
+  }
 }
 
 __global__ void k_group_flags(uint32_t const *vals, size_t N, uint32_t g, uint32_t *flags) {
@@ -1588,10 +2017,10 @@ static void exclusive_scan(uint32_t const *in, uint32_t *out, size_t n, uint32_t
 }
 
 Nhood::Nhood() {
-  PG_CUDA(cudaMalloc(&stats_d_, 16 * sizeof(uint32_t)));
+  PG_CUDA(cudaMalloc(&stats_d_, kStWords * sizeof(uint32_t)));
   PG_CUDA(cudaMalloc(&ncells_d_, sizeof(int)));
   PG_CUDA(cudaMemset(ncells_d_, 0, sizeof(int)));
-  PG_CUDA(cudaMallocHost(&stats_h_, 16 * sizeof(uint32_t)));
+  PG_CUDA(cudaMallocHost(&stats_h_, kStWords * sizeof(uint32_t)));
 }
 
 static void free_all(std::initializer_list<void *> ps) {
@@ -1602,7 +2031,8 @@ static void free_all(std::initializer_list<void *> ps) {
 Nhood::~Nhood() {
   for (auto &kv : lists_) free_lists(kv.second);
   free_all({keys_a_, keys_b_, vals_a_, vals_b_, ukeys_, flags_, scan_, r2s_, s2c_, cell_start_, cell_adj_, cell_key_,
-            cell_gi_, xsorted_, hist_, block_sums_, stats_d_, ncells_d_, order_, hkeys_, hvals_});
+            cell_gi_, xsorted_, hist_, block_sums_, stats_d_, ncells_d_, order_, hkeys_, hvals_, dir_count_, dir_cell_,
+            dir_sums_, dir_touched_});
   cudaFreeHost(stats_h_);
 }
 
@@ -1650,6 +2080,7 @@ void Nhood::load(Model &m) {
   gg_ = ng;
   if (!same) {
     has_grid_ = false;
+    dense_ = false;
     for (auto &c : permuted_count_) c = 0;
     for (auto &kv : lists_) free_lists(kv.second);
     lists_.clear();
@@ -1703,9 +2134,11 @@ GridView Nhood::view() const {
   return v;
 }
 
-// the cell-key layout of the bit statistics ne, eq, a1, a0 of k_cells_u
+// the cell-key layout of the bit statistics of k_cells_u: the bits that are
+// informative on any axis
 static KeyInfo key_from_stats(uint32_t const *st) {
-  uint32_t ne = st[0], eq = st[1], a1 = st[2], a0 = st[3];
+  uint32_t ne = st[0] | st[2] | st[4], eq = st[1] | st[3] | st[5];
+  bool a1 = ne >> 31, a0 = eq >> 31;
   KeyInfo k{};
   k.keep = ne & eq & 0x7FFFFFFFu;
   k.rel_eq = eq & ~ne & 0x7FFFFFFFu;
@@ -1719,16 +2152,142 @@ static KeyInfo key_from_stats(uint32_t const *st) {
 static bool same_key(KeyInfo const &a, KeyInfo const &b) {
   return a.keep == b.keep && a.rel_eq == b.rel_eq && a.rel_ne == b.rel_ne && a.b31_const == b.b31_const;
 }
+// the table layout for it: the key bits that are informative on their own
+// axis, and the segment's (no runs: keys too long, or scattered too far)
+static DirKey dir_from_stats(uint32_t const *st, KeyInfo const &k, int seg_bits) {
+  DirKey d{};
+  int total = 3 * k.bits + seg_bits;
+  if (total > 32 || total == 0) return d;
+  uint64_t keep = ((uint64_t(1) << seg_bits) - 1) << (3 * k.bits);
+  for (int a = 0; a < 3; ++a) {
+    uint32_t ne = st[2 * a], eq = st[2 * a + 1], own = ne & eq & 0x7FFFFFFFu;
+    DirAxis &x = d.axis[a];
+    x.rel_eq = eq & ~ne & 0x7FFFFFFFu;
+    x.rel_ne = ne & ~eq & 0x7FFFFFFFu;
+    if ((ne >> 31) && (eq >> 31)) own |= 0x80000000u;
+    else x.b31_const = (ne >> 31) ? 0x80000000u : 0u;
+    x.keep = own;
+    int b = 0; // position among the kept bits
+    for (uint32_t m = k.keep; m; m &= m - 1, ++b)
+      if (own & m & (~m + 1u)) keep |= uint64_t(1) << (3 * b + 2 - a);
+  }
+  int out = 0, n = 0;
+  for (uint64_t m = keep; m;) {
+    if (n == kDirRuns) return DirKey{};
+    int lo = __builtin_ctzll(m), len = 0;
+    while (lo + len < 64 && ((m >> (lo + len)) & 1u)) ++len;
+    uint64_t run = ((uint64_t(1) << len) - 1) << lo;
+    d.mask[n] = uint32_t(run);
+    d.shift[n] = uint32_t(lo - out);
+    ++n;
+    out += len;
+    m &= ~run;
+  }
+  d.nruns = n;
+  d.bits = out;
+  return d;
+}
+static bool same_dir(DirKey const &a, DirKey const &b) {
+  if (a.nruns != b.nruns || a.bits != b.bits) return false;
+  for (int t = 0; t < a.nruns; ++t)
+    if (a.mask[t] != b.mask[t] || a.shift[t] != b.shift[t]) return false;
+  for (int x = 0; x < 3; ++x)
+    if (a.axis[x].keep != b.axis[x].keep || a.axis[x].rel_eq != b.axis[x].rel_eq ||
+        a.axis[x].rel_ne != b.axis[x].rel_ne || a.axis[x].b31_const != b.axis[x].b31_const)
+      return false;
+  return true;
+}
 
 void Nhood::settle(cudaStream_t s) {
   if (!key_check_) return;
-  PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+  PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, kStRows * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
   PG_CUDA(cudaStreamSynchronize(s));
-  key_check_ = false;
-  if (!same_key(key_from_stats(stats_h_), key_)) {
-    key_known_ = false;
-    update(s);
+  if (!confirmed()) update(s);
+}
+
+// Whether a grid of N items is built by counting, with the tables allocated:
+// the knob is on, the entries are at most 2^27 and 128 an item (8 bytes each,
+// about what the lists take; an entry that no item maps to is never read) or
+// 2^18, and the last counted grid at this radius had no overfull cell.
+bool Nhood::direct_ready(size_t N, cudaStream_t s) {
+  if (!model_->tune.v[kTuneGridSort] || dense_ || !dir_key_.nruns || dir_key_.bits > kDirectBits) return false;
+  size_t entries = std::max<size_t>(size_t(1) << dir_key_.bits, kDirTile);
+  if (entries > std::max<size_t>(128 * N, size_t(1) << 18)) return false;
+  if (entries > dir_cap_) {
+    free_all({dir_count_, dir_cell_, dir_sums_, dir_touched_});
+    dir_count_ = dir_cell_ = nullptr;
+    dir_sums_ = nullptr;
+    dir_touched_ = nullptr;
+    dir_cap_ = 0;
+    size_t tiles = entries / kDirTile, runs = entries / kDirRun;
+    PG_CUDA(cudaMalloc(&dir_count_, entries * sizeof(uint32_t)));
+    PG_CUDA(cudaMalloc(&dir_cell_, entries * sizeof(uint32_t)));
+    PG_CUDA(cudaMalloc(&dir_sums_, (tiles + kDirBlocks) * sizeof(uint64_t)));
+    PG_CUDA(cudaMalloc(&dir_touched_, runs * kMark * sizeof(uint32_t)));
+    PG_CUDA(cudaMemsetAsync(dir_count_, 0, entries * sizeof(uint32_t), s));
+    PG_CUDA(cudaMemsetAsync(dir_touched_, 0, runs * kMark * sizeof(uint32_t), s));
+    dir_cap_ = entries;
   }
+  return true;
+}
+
+void Nhood::build_direct(GridView const &gv, int G, size_t N, cudaStream_t s) {
+  PosTable pt{};
+  for (int g = 0; g < G; ++g)
+    if (gg_[g].pos) pt.pos[g] = static_cast<float4 const *>(gg_[g].pos->d);
+  uint32_t tiles = uint32_t(std::max<size_t>(size_t(1) << dir_key_.bits, kDirTile) / kDirTile);
+  unsigned nb = div_up(N, 256);
+  DirTable T{dir_count_, dir_touched_, dir_cell_, dir_key_};
+  uint32_t per = (tiles + kDirBlocks - 1) / kDirBlocks;
+  unsigned tb = div_up(tiles, per);
+  uint64_t *base = dir_sums_ + tiles;
+  {
+    ProfScope ps(model_->prof, "grid_sort", s);
+    k_dir_sums<<<tb, kDirNT, 0, s>>>(T, tiles, per, dir_sums_, base, stats_d_, ncells_d_, cell_start_); count_launch();
+    k_dir_fill<<<std::min(tiles, kDirBlocks), kDirNT, 0, s>>>(T, tiles, per, dir_sums_, base, cell_start_, scan_);
+    count_launch();
+    k_dir_scatter<<<nb, 256, 0, s>>>(gv, G, reinterpret_cast<uint2 const *>(keys_a_), dir_count_, N, vals_b_);
+    count_launch();
+    PG_LAUNCH_CHECK();
+  }
+  {
+    ProfScope ps(model_->prof, "grid_cells", s);
+    k_dir_adj<<<std::min(div_up(N, kDirAdjNT), kDirBlocks), kDirAdjNT, 0, s>>>(gv, T, scan_, cell_key_, cell_gi_,
+                                                                             cell_adj_, s2c_);
+    count_launch();
+    k_dir_order<<<nb, 256, 0, s>>>(pt, vals_b_, s2c_, cell_start_, N, vals_a_, xsorted_); count_launch();
+    xsorted_of_ = pos_versions();
+    xsorted_epoch_ = epoch_;
+    PG_LAUNCH_CHECK();
+  }
+  sorted_keys_ = nullptr;
+  sorted_vals_ = vals_a_;
+  counted_ = true;
+  key_check_ = true; // the fullest cell is confirmed with the key statistics
+}
+
+// the statistics read back (stats_h_) fit the grid as built; where they do
+// not, the next update takes the layout, or the sort, that they ask for
+bool Nhood::confirmed() {
+  key_check_ = false;
+  bool ok = true;
+  KeyInfo k = key_from_stats(stats_h_);
+  if (!same_key(k, key_) ||
+      (counted_ && !same_dir(dir_from_stats(stats_h_, k, seg_count_ ? seg_bits_ : 0), dir_key_)))
+    ok = key_known_ = false;
+  if (counted_ && stats_h_[kStMaxCell] > kDirMaxCell) {
+    dense_ = true;
+    ok = false;
+  }
+  return ok;
+}
+
+// raw -> sorted of the present grid
+void Nhood::need_r2s(cudaStream_t s) {
+  if (r2s_epoch_ == epoch_ || !N_) return;
+  k_r2s<<<div_up(N_, 256), 256, 0, s>>>(sorted_vals_, view(), N_, r2s_); count_launch();
+  PG_LAUNCH_CHECK();
+  r2s_epoch_ = epoch_;
 }
 
 // grouped_uniform_grid::update (util/grouped_uniform_grid.hpp:126-337)
@@ -1754,6 +2313,7 @@ void Nhood::update(cudaStream_t s) {
   ensure_grid_capacity(N);
   epoch_++;
   has_grid_ = true;
+  counted_ = false;
   if (N == 0) {
     key_check_ = false; // no statistics to confirm
     PG_CUDA(cudaMemsetAsync(ncells_d_, 0, sizeof(int), s));
@@ -1762,14 +2322,21 @@ void Nhood::update(cudaStream_t s) {
     return;
   }
   GridView gv = view();
+  r2s_epoch_ = 0;
   // 1. grid indices, handles, bit statistics
-  PG_CUDA(cudaMemsetAsync(stats_d_, 0, 16 * sizeof(uint32_t), s));
+  PG_CUDA(cudaMemsetAsync(stats_d_, 0, kStWords * sizeof(uint32_t), s));
   unsigned nb = div_up(N, 256);
+  bool direct = key_known_ && direct_ready(N, s);
+  DirTable T{dir_count_, dir_touched_, dir_cell_, dir_key_};
   {
     ProfScope ps(model_->prof, "grid_keys", s);
-    unsigned ub = std::min<unsigned>(div_up(N, kCellsUNT), 152u * 8u);
-    if (key_known_) k_cells_u<true><<<ub, kCellsUNT, 0, s>>>(pt, gv, G, N, nullptr, keys_a_, vals_a_, stats_d_);
-    else k_cells_u<false><<<ub, kCellsUNT, 0, s>>>(pt, gv, G, N, ukeys_, nullptr, vals_a_, stats_d_);
+    unsigned ub = std::min<unsigned>(div_up(N, kCellsUNT), 152u * 5u); // one resident wave
+    if (direct)
+      k_cells_u<true, true><<<ub, kCellsUNT, 0, s>>>(pt, gv, G, N, nullptr, keys_a_, nullptr, stats_d_, T);
+    else if (key_known_)
+      k_cells_u<true, false><<<ub, kCellsUNT, 0, s>>>(pt, gv, G, N, nullptr, keys_a_, vals_a_, stats_d_, T);
+    else
+      k_cells_u<false, false><<<ub, kCellsUNT, 0, s>>>(pt, gv, G, N, ukeys_, nullptr, vals_a_, stats_d_, T);
     count_launch();
   }
   PG_LAUNCH_CHECK();
@@ -1780,9 +2347,10 @@ void Nhood::update(cudaStream_t s) {
     k = key_;
     key_check_ = true;
   } else {
-    PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, 4 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, kStRows * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaStreamSynchronize(s));
     k = key_from_stats(stats_h_);
+    dir_key_ = dir_from_stats(stats_h_, k, seg_count_ ? seg_bits_ : 0);
     key_known_ = true;
     key_check_ = false;
   }
@@ -1794,10 +2362,20 @@ void Nhood::update(cudaStream_t s) {
                 std::to_string(k.bits) + " informative bits per axis");
   key_ = k;
   gv = view();
+  if (!keyed && direct_ready(N, s)) {
+    direct = true;
+    T = DirTable{dir_count_, dir_touched_, dir_cell_, dir_key_};
+    k_cells_key<true><<<nb, 256, 0, s>>>(ukeys_, vals_a_, N, gv, keys_a_, T); count_launch();
+    PG_LAUNCH_CHECK();
+  }
+  if (direct) {
+    build_direct(gv, G, N, s);
+    return;
+  }
   // 2. compressed Z-order keys (segment above them)
   model_->prof.begin("grid_sort", s);
   if (!keyed) {
-    k_cells_key<<<nb, 256, 0, s>>>(ukeys_, vals_a_, N, gv, keys_a_); count_launch();
+    k_cells_key<false><<<nb, 256, 0, s>>>(ukeys_, vals_a_, N, gv, keys_a_, T); count_launch();
     PG_LAUNCH_CHECK();
   }
   // 3. stable LSD radix sort over the informative bits
@@ -1852,7 +2430,7 @@ void Nhood::update(cudaStream_t s) {
     ensure_sums(tiles_c, block_sums_, block_sums_cap_);
     k_cf_count<<<unsigned(tiles_c), kScanNT, 0, s>>>(kin, N, block_sums_); count_launch();
     k_scan_single<<<1, 1024, 0, s>>>(block_sums_, tiles_c); count_launch();
-    k_cf_fill<<<unsigned(tiles_c), kScanNT, 0, s>>>(pt, gv, kin, vin, block_sums_, N, s2c_, r2s_, cell_start_,
+    k_cf_fill<<<unsigned(tiles_c), kScanNT, 0, s>>>(pt, gv, kin, vin, block_sums_, N, s2c_, cell_start_,
                                                    cell_key_, cell_gi_, ncells_d_, cell_adj_);
     count_launch();
     PG_LAUNCH_CHECK();
@@ -1901,7 +2479,7 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
   PosTable pt{};
   for (int g = 0; g < G; ++g)
     if (gg_[g].pos) pt.pos[g] = static_cast<float4 const *>(gg_[g].pos->d);
-  if (N_ > 0) {
+  if (N_ > 0 && !(xsorted_epoch_ == epoch_ && xsorted_of_ == pos_versions())) {
     k_xsorted<<<div_up(N_, 256), 256, 0, s>>>(pt, sorted_vals_, N_, xsorted_); count_launch();
     PG_LAUNCH_CHECK();
   }
@@ -1998,11 +2576,12 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
     }
     size_t smem = size_t(G) * (st ? 32 : 24) * kBuildNT * 4;
     lo.cb = L.cb;
-    lo.maxcnt = stats_d_ + 8;
+    lo.maxcnt = stats_d_ + kStRows;
     lo.n = uint32_t(n);
     lo.G = G;
     lo.with_gf = h != nullptr ? 1 : 0;
-    PG_CUDA(cudaMemsetAsync(stats_d_ + 8, 0, 8 * sizeof(uint32_t), s));
+    PG_CUDA(cudaMemsetAsync(stats_d_ + kStRows, 0, kMaxListGroups * sizeof(uint32_t), s));
+    if (!warp && in_grid_[q]) need_r2s(s);
     GridView gv = view();
     float4 const *qpos = static_cast<float4 const *>(gg_[q].pos->d);
     {
@@ -2031,24 +2610,21 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
     // one read-back: the rows' lengths, and the grid's key statistics when
     // its layout is still to be confirmed
     if (key_check_)
-      PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, 16 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, kStWords * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     else
-      PG_CUDA(cudaMemcpyAsync(stats_h_ + 8, stats_d_ + 8, 8 * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+      PG_CUDA(cudaMemcpyAsync(stats_h_ + kStRows, stats_d_ + kStRows, kMaxListGroups * sizeof(uint32_t),
+                              cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaStreamSynchronize(s));
-    if (key_check_) {
-      key_check_ = false;
-      if (!same_key(key_from_stats(stats_h_), key_)) {
-        // the layout changed: a new grid (read-back layout), then these lists
-        key_known_ = false;
-        update(s);
-        build_lists(q, L, s, h, stage);
-        return;
-      }
+    if (key_check_ && !confirmed()) {
+      // a new grid (read-back layout, or sorted), then these lists
+      update(s);
+      build_lists(q, L, s, h, stage);
+      return;
     }
     bool grow = false;
     for (int g = 0; g < G; ++g)
-      if (stats_h_[8 + g] > L.cap[g]) {
-        alloc_slots(g, (stats_h_[8 + g] + kChunk - 1) / kChunk * kChunk + kChunk);
+      if (stats_h_[kStRows + g] > L.cap[g]) {
+        alloc_slots(g, (stats_h_[kStRows + g] + kChunk - 1) / kChunk * kChunk + kChunk);
         grow = true;
       }
     if (!grow) {
@@ -2057,7 +2633,7 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
       // the lists do not hold the largest capacity ever needed
       bool shrink = false;
       for (int g = 0; g < G && attempt < 7; ++g) {
-        uint32_t want = std::max<uint32_t>((stats_h_[8 + g] + kChunk - 1) / kChunk * kChunk + kChunk, 48u);
+        uint32_t want = std::max<uint32_t>((stats_h_[kStRows + g] + kChunk - 1) / kChunk * kChunk + kChunk, 48u);
         if (L.cap[g] > 2 * want && L.cap[g] > 128u) {
           alloc_slots(g, want);
           shrink = true;
@@ -2171,8 +2747,10 @@ void Nhood::set_segments(std::vector<uint16_t const *> const &seg, uint32_t coun
   if (count > 65536) throw Error("set_segments: at most 65536 segments");
   seg_ = seg;
   seg_count_ = count;
+  int before = seg_bits_;
   seg_bits_ = 0;
   while (count > 1 && (uint32_t(1) << seg_bits_) < count) ++seg_bits_;
+  if (seg_bits_ != before) key_known_ = false; // the table's layout holds the segment's bits
   has_grid_ = false;
 }
 
@@ -2183,7 +2761,7 @@ uint64_t Nhood::pair_count(int q, cudaStream_t s) {
   PG_CUDA(cudaMemsetAsync(d, 0, sizeof *d, s));
   for (size_t g = 0; g < gg_.size(); ++g)
     if (v.n && v.cb[g]) {
-      k_pair_count<<<div_up(v.n, 256), 256, 0, s>>>(v.cb[g], v.n, d);
+      k_pair_count<<<std::min(div_up(v.n, kPairNT), 152u * 8u), kPairNT, 0, s>>>(v.cb[g], v.n, d);
       count_launch();
     }
   PG_LAUNCH_CHECK();
@@ -2213,7 +2791,7 @@ size_t Nhood::device_bytes() const {
   // keys 2x8, values 2x4, ukeys 16, flags 4, scan 4, r2s 4, s2c 4, cell
   // start 4, adjacency 104, cell key 8, cell index 16, sorted positions 16
   size_t b = cap_ * (16 + 8 + 16 + 4 + 4 + 4 + 4 + 4 + 104 + 8 + 16 + 16);
-  b += hist_cap_ * 4 + block_sums_cap_ * 4;
+  b += hist_cap_ * 4 + block_sums_cap_ * 4 + dir_cap_ * 8 + hash_cap_ * 12;
   for (auto const &kv : lists_) {
     Lists const &L = kv.second;
     b += L.n * gg_.size() * sizeof(uint2);

@@ -17,16 +17,16 @@
 //      the order of most-significant differing bits across axes, so the
 //      compressed key orders cells exactly like the reference.  At most 21
 //      informative bits per axis are supported (63-bit keys).
-//   3. a stable LSD radix sort of (key, handle) pairs, 8-bit digits, starting
-//      from group-major identity order: cells in the reference's Morton
-//      order; within a cell (group, raw index) order.  The reference's
-//      parallel sort is unstable, so its within-cell order is unspecified;
-//      cell membership and cell order are exact.
-//   4. cell boundaries, cell ids by prefix scan, cell ranges, cell keys and
-//      grid indices, and raw -> sorted.
+//   3. the items in cell order: cells in the reference's Morton order; within
+//      a cell (group, raw index) order.  The reference's parallel sort is
+//      unstable, so its within-cell order is unspecified; cell membership and
+//      cell order are exact.  Short keys: by counting in a table with an
+//      entry per key (nhood.cu, "the grid by counting"); long ones: a stable
+//      LSD radix sort of (key, handle) pairs from group-major identity order.
+//   4. cell ids, cell ranges, cell keys and grid indices.
 //   5. the 26-cell adjacency: slot k < 13 holds the cell at +offset[k],
-//      slot 25-k the cell at -offset[k] (:52-68, :312-337); found by binary
-//      search over the sorted cell keys.
+//      slot 25-k the cell at -offset[k] (:52-68, :312-337); looked up in the
+//      same table, or in a hash table of the cell keys.
 // Neighbour lists (built lazily per query group, reused by every procedure
 // until positions change or the grid is updated): for each query item the
 // own cell and adjacency slots 0..25 in order, each cell's items in sorted
@@ -133,6 +133,19 @@ struct KeyInfo {
   uint32_t run_shift[kKeyRuns] = {};
 };
 
+// The entry of a cell key of at most 32 bits in the table of a grid built by
+// counting: the key's kept bits, as runs (nruns 0: no table)
+constexpr int kDirRuns = 8;
+struct DirAxis { // the bits of the biased grid index along one axis, as in KeyInfo
+  uint32_t keep = 0, rel_eq = 0, rel_ne = 0, b31_const = 0;
+};
+struct DirKey {
+  int nruns = 0, bits = 0;
+  DirAxis axis[3];
+  uint32_t mask[kDirRuns] = {};
+  uint32_t shift[kDirRuns] = {};
+};
+
 // split `keep` into runs of consecutive set bits (at most kKeyRuns)
 inline void key_runs(KeyInfo &k) {
   k.nruns = 0;
@@ -184,7 +197,10 @@ public:
   Nhood(Nhood const &) = delete;
   Nhood &operator=(Nhood const &) = delete;
 
-  void set_radius(double r) { radius_ = r; }
+  void set_radius(double r) {
+    if (r != radius_) dense_ = false;
+    radius_ = r;
+  }
   double radius() const { return radius_; }
   void load(Model &m);
   void update(cudaStream_t s);
@@ -223,6 +239,8 @@ public:
   size_t staged_tiles(int q, size_t &tiles, cudaStream_t s);
 
   GridView view() const;
+  // raw -> sorted (GridView::r2s) is made where a reader asks for it
+  void need_r2s(cudaStream_t s);
   // sorted positions with their handles in w (current after the lists of a
   // group have been built for the present positions)
   float4 const *sorted_positions() const { return xsorted_; }
@@ -261,6 +279,9 @@ private:
   // first.  Called before the grid is read on the host or permutes fields;
   // the list build confirms it at its own synchronisation instead.
   void settle(cudaStream_t s);
+  bool direct_ready(size_t N, cudaStream_t s);
+  void build_direct(GridView const &gv, int G, size_t N, cudaStream_t s);
+  bool confirmed();
   bool lists_fresh(Lists const &L) const;
   std::vector<uint64_t> pos_versions() const;
   void free_lists(Lists &L);
@@ -272,7 +293,7 @@ private:
   uint32_t goff_[kMaxGroups + 1] = {};
   int in_grid_[kMaxGroups] = {};
   KeyInfo key_{};
-  // The cell-key layout is a function of four bit statistics of all items'
+  // The cell-key layout is a function of the bit statistics of all items'
   // grid indices (k_cells_u).  An update reuses the last layout without
   // reading the statistics back (key_known_), and flags it for the check
   // (key_check_) at the next synchronisation; in a simulation the layout
@@ -282,6 +303,16 @@ private:
   // list build walks a group that was not in grid order instead)
   size_t permuted_count_[kMaxGroups] = {};
   uint32_t *order_ = nullptr; // group items in grid order (list build)
+  // grid by counting: per cell key the item count (zero between updates), the
+  // cell, and the tile sums; counted_: the present grid was built that way;
+  // dense_: a cell was too full for it, at this radius
+  uint32_t *dir_count_ = nullptr, *dir_cell_ = nullptr;
+  uint64_t *dir_sums_ = nullptr;
+  uint32_t *dir_touched_ = nullptr;
+  DirKey dir_key_{};
+  size_t dir_cap_ = 0;
+  bool counted_ = false, dense_ = false;
+  uint64_t r2s_epoch_ = 0;
   uint64_t *hkeys_ = nullptr;  // cell-key hash table (adjacency lookups)
   int32_t *hvals_ = nullptr;
   size_t hash_cap_ = 0;
@@ -301,11 +332,14 @@ private:
   uint64_t *cell_key_ = nullptr;
   int4 *cell_gi_ = nullptr;
   float4 *xsorted_ = nullptr;
+  // the grid and the positions that a counted grid's update left in xsorted_
+  uint64_t xsorted_epoch_ = 0;
+  std::vector<uint64_t> xsorted_of_;
   uint32_t *hist_ = nullptr;
   size_t hist_cap_ = 0;
   uint32_t *block_sums_ = nullptr;
   size_t block_sums_cap_ = 0;
-  uint32_t *stats_d_ = nullptr; // bit statistics / counters (16 words)
+  uint32_t *stats_d_ = nullptr; // bit statistics / counters
   int *ncells_d_ = nullptr;
   uint32_t *stats_h_ = nullptr; // pinned
   uint64_t const *sorted_keys_ = nullptr;

@@ -1913,7 +1913,7 @@ std::string tune_knob_table() {
   t += "pcg_q 0 " + shapes_text<PcgShapes>() + " 4=cell-tiles (no lists; plain models)\n";
   t += "jacobi_unroll 1 1=1 2=2 4=4\n";
   t += "staging 0 0=off 1=staged lists and sweeps (unbatched models)\n";
-  t += "grid_sort 1 0=tiled launches 1=one cluster launch for grids of at most 128k items\n";
+  t += "grid_sort 1 0=tiled radix sort 1=counting where the keys are short, else one cluster launch up to 128k items\n";
   t += "list_split 1 0=one thread per query 1=one warp per run of queries of a cell\n";
   return t;
 }
@@ -2816,6 +2816,7 @@ public:
     float4 const *xs = nullptr;
     int fg = F.g->index, bg = bound_.empty() ? -1 : bound_[0].g->index;
     if constexpr (kTuned) {
+      if (!seg && tv_q == 4) nh.need_r2s(s);
       gv = nh.view();
       // the tiles walk the grid's cells: the fluid group must be in the grid
       if (!seg && tv_q == 4 && gv.in_grid[fg]) {

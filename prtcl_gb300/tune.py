@@ -12,9 +12,10 @@ the tuner is free to pick the fastest per workload:
 * staging (single-scene models) builds staged neighbour lists and runs the
   staged relaxed-Jacobi and PCG sweeps, which read their neighbours'
   records from shared memory (0 or 1);
-* grid_sort (single-scene models whose grid holds at most 128k items)
-  sorts the grid in one launch of a thread-block cluster instead of the
-  tiled radix-sort launches (0 or 1);
+* grid_sort builds the grid by counting (short cell keys), or sorts a grid
+  of at most 128k items in one launch of a thread-block cluster, instead of
+  the tiled radix-sort launches (0 or 1; searched for single-scene models
+  whose grid holds at most 128k items);
 * list_split builds the lists with one warp per run of queries of a cell
   instead of one thread per query (0 or 1).
 
