@@ -1604,7 +1604,7 @@ __device__ __forceinline__ uint32_t *factor_word(unsigned char *ch, uint32_t slo
 //
 // The queries of a cell see the same 27 cells, so they share their candidates.
 // A unit is up to kUnit consecutive sorted items of one cell; a warp takes the
-// units that begin in its window of kWinItems sorted items (one that begins
+// units that begin in its window of up to kWinItems sorted items (one that begins
 // there may run past its end, so a warp has at most kWinItems + kUnit - 1
 // items, however full the cells are).  Per unit:
 //   1. lanes 0..26 look up the 27 cells in visit order (own cell, adjacency
@@ -1636,8 +1636,17 @@ __device__ __forceinline__ uint32_t *factor_word(unsigned char *ch, uint32_t slo
 // form.  Measured in one call against a thread per query (and, up to 65,536
 // queries, against four threads per query, the form before this one): 4M
 // uniform points 2446 -> 1112 us, 1.5M clustered 1381 -> 719; with factors, 1M
-// dam break 659 -> 425 us, 27k 52 (four threads) -> 37, 5k 39 -> 28.
-constexpr int kWinItems = 16;
+// dam break 659 -> 425 us, 27k 52 (four threads) -> 37, 5k 39 -> 28.  Writing
+// two hits of a mask per round (put_hits) took the 4M points to 1081 us, 150k
+// clustered ones 108 -> 96 and the 1M dam break to 392.
+//
+// A grid of few items gets smaller windows, so that its warps, of two or three
+// units at 16 items, become more and shorter ones; each costs its own look at
+// the window.  Items of the grid, us at windows of 16 / 8 / 4: 17k 26 / 20 /
+// 16, 36k 29 / 25 / 24, 62k 35 / 28 / 31, 84k 39 / 33 / 37, 149k 54 / 51 / 63,
+// 255k 79 / 78 / 104, 465k 140 / 140 / 200.
+constexpr uint32_t kWinItems = 16;
+constexpr size_t kWinSmall = 40'000, kWinMedium = 200'000; // windows of a quarter, a half up to these
 constexpr int kCand = 320, kCandChunks = kCand / 32;
 constexpr int kUnit = 16;             // queries of a unit
 constexpr int kFlat = 640;            // hits of a portion written out together
@@ -1666,6 +1675,19 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, int lane) {
   return v;
 }
 
+// the set bits of m, tagged, to the places from `at` on (moved past them): the
+// lowest and the highest in each round
+__device__ __forceinline__ void put_hits(uint16_t *flat, uint32_t &at, uint32_t m, uint32_t tag) {
+  uint32_t end = at + __popc(m);
+  for (uint32_t a = at, z = end; m;) {
+    uint32_t t = uint32_t(__ffs(int(m)) - 1), u = uint32_t(31 - __clz(int(m)));
+    flat[a++] = uint16_t(tag + t);
+    flat[--z] = uint16_t(tag + u);
+    m &= (m - 1u) & ((1u << u) - 1u);
+  }
+  at = end;
+}
+
 // the range of the items' indices that `in` holds for
 __device__ __forceinline__ void index_range(bool in, uint32_t handle, uint32_t &lo, uint32_t &hi) {
   uint32_t j = handle & 0x0FFFFFFFu;
@@ -1675,19 +1697,20 @@ __device__ __forceinline__ void index_range(bool in, uint32_t handle, uint32_t &
 
 template <int NG, bool GF>
 __global__ void __launch_bounds__(kWarpNT, GF ? 16 : 18) k_build_lists_warp(GridView gv, float4 const *__restrict__ xs, size_t N,
-                                                              int q, ListOut lo, float const *hp, float *hcache) {
+                                                              int q, ListOut lo, float const *hp, float *hcache,
+                                                              uint32_t window) {
   static_assert(NG == 1 || NG == 2, "one or two neighbour groups");
   __shared__ ListWarp s_warp[kWarps];
   ListWarp &S = s_warp[threadIdx.x / 32];
   int lane = threadIdx.x & 31;
   KernelParams K = kparams(GF ? *hp : 1.0f);
   if (blockIdx.x == 0 && threadIdx.x == 0) *hcache = GF ? K.h : __int_as_float(0x7fc00000);
-  size_t win = (size_t(blockIdx.x) * kWarps + threadIdx.x / 32) * kWinItems;
+  size_t win = (size_t(blockIdx.x) * kWarps + threadIdx.x / 32) * window;
   if (win >= N) return; // whole warps
   // the units that begin in the window
   int wcell = 0, wend = 0;
   bool begins = false;
-  if (lane < kWinItems && win + lane < N) {
+  if (lane < int(window) && win + lane < N) {
     int s = int(win) + lane;
     wcell = gv.s2c[s];
     wend = gv.cell_start[wcell + 1];
@@ -1833,14 +1856,13 @@ __global__ void __launch_bounds__(kWarpNT, GF ? 16 : 18) k_build_lists_warp(Grid
         if (qin) {
           uint32_t w0 = f0 - done, w1 = f1 - done, tag = uint32_t(hq * NG) << 10;
           for (int k = k0; k < k1; ++k) {
-            uint32_t m = S.mask[hq][k], sec = NG == 2 ? S.second[k] : 0u;
-            while (m) {
-              int t = __ffs(int(m)) - 1;
-              m &= m - 1u;
-              uint32_t f = tag | uint32_t(k * 32 + t);
-              if (NG == 2 && ((sec >> t) & 1u)) S.flat[w1++] = uint16_t(f + 1024u);
-              else S.flat[w0++] = uint16_t(f);
+            uint32_t m = S.mask[hq][k], f = tag | uint32_t(k * 32);
+            if constexpr (NG == 2) {
+              uint32_t sec = m & S.second[k];
+              m ^= sec;
+              put_hits(S.flat, w1, sec, f + 1024u);
             }
+            put_hits(S.flat, w0, m, f);
           }
         }
         __syncwarp();
@@ -1904,9 +1926,10 @@ __global__ void __launch_bounds__(kWarpNT, GF ? 16 : 18) k_build_lists_warp(Grid
 template <int NG>
 void launch_build_lists_warp(size_t N, cudaStream_t s, GridView const &gv, float4 const *xs, int q, ListOut const &lo,
                              float const *h, float *hcache) {
-  unsigned nb = div_up(div_up(N, kWinItems), kWarps);
-  if (h) k_build_lists_warp<NG, true><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache);
-  else k_build_lists_warp<NG, false><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache);
+  uint32_t window = N <= kWinSmall ? kWinItems / 4 : N <= kWinMedium ? kWinItems / 2 : kWinItems;
+  unsigned nb = div_up(div_up(N, window), kWarps);
+  if (h) k_build_lists_warp<NG, true><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache, window);
+  else k_build_lists_warp<NG, false><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache, window);
 }
 
 template <int NG, bool STAGE>
