@@ -74,12 +74,43 @@ __device__ __forceinline__ f3 pgrad(bool cached, float factor, KernelParams cons
   return cached ? kgrad_from(factor, xij) : kgradW(K, xij);
 }
 
+// the sum with the pair's term where the pair counts
+__device__ __forceinline__ float add_if(bool in, float a, float t) { return in ? a + t : a; }
+__device__ __forceinline__ f3 add_if(bool in, f3 a, f3 t) {
+  f3 s = add3(a, t);
+  return {in ? s.x : a.x, in ? s.y : a.y, in ? s.z : a.z};
+}
+__device__ __forceinline__ f3 sub_if(bool in, f3 a, f3 t) {
+  f3 s = sub3(a, t);
+  return {in ? s.x : a.x, in ? s.y : a.y, in ? s.z : a.z};
+}
+
 struct FluidN {
   NbrList L;
   float4 const *xm; // (x, y, z, m)
   float4 const *v;  // velocity
   float4 const *a;  // acceleration
   float const *pr;  // p / (rho rho)
+};
+
+// a / b in a walk: without a branch where FLAT, noting in `off` operands that
+// this does not divide exactly (the row is then walked again, dividing)
+template <bool FLAT> __device__ __forceinline__ float divide_noting(float a, float b, bool &off) {
+  if (!FLAT) return a / b;
+  float q = divide_flat(a, b);
+  off = off || !divides_flat(a, b, q);
+  return q;
+}
+template <bool FLAT> __device__ __forceinline__ float divide_noting(float a, Divisor const &b, bool &off) {
+  if (!FLAT) return a / b.d;
+  off = off || !quotient_exact(a, b);
+  return quotient(a, b);
+}
+
+// a neighbour's record and a second value of it
+template <class T> struct WithRec {
+  float4 x;
+  T v;
 };
 
 struct BoundN {
@@ -156,10 +187,12 @@ unsigned red_grid(size_t n) { return unsigned(std::min<size_t>(div_up(n, kNT), k
 // per-item arithmetic does not depend on the shape, and the sweeps with an
 // FP64 reduction keep 128 threads per block and their grid, so the shape of
 // the reduction tree does not change.
-// Walking 8 entries at a time is the default of every sweep.  Measured per
-// launch on the 1M dam break (8 / 16 entries): density 99 / 111 us, pressure
-// 138 / 157, acceleration 95 / 105, set-up 236 / 249, diagonal 117 / 126,
-// PCG product 154 / 172; at 27k items the two are within 2 us of each other.
+// The defaults are the fastest forms of the walk (nbr_walk.cuh, which has the
+// times) at 1M items; where the second one is the other number of records,
+// density 87 (4) / 88 us (8), set-up 193 (8) / 199 (4), diagonal 113 (4) / 118
+// (8).  The tiled sweeps of a batch have rows of other lengths side by side and
+// fewer warps once scenes have converged: 48 scenes, 8 steps, second form /
+// default, acceleration 7.8 / 6.7 ms, pressure 10.0 / 9.7, PCG product 3.0 / 2.8.
 template <int NT_, int MINB_, int BT_> struct Shape {
   static constexpr int nt = NT_, minb = MINB_, bt = BT_;
 };
@@ -171,6 +204,14 @@ using FreeShapes = std::tuple<Shape<kNT, kMinBlocks, B0>, Shape<kNT, kMinBlocks,
 template <int B0, int B1>
 using RedShapes = std::tuple<Shape<kNT, kMinBlocks, B0>, Shape<kNT, kMinBlocks, B1>, Shape<kNT, 6, B0>,
                              Shape<kNT, 12, B0>>;
+// Up to kSmallItems every block of a sweep is resident at once at four blocks
+// per SM, so warps are few anyway and a thread may have the registers to load
+// its entries ahead: where the knob has its default, the set-up, Jacobi and PCG
+// sweeps take this shape.  At 27k items set-up 17.6 -> 14.6 us, acceleration
+// 16.4 -> 10.7, pressure 19.4 -> 14.4, PCG product 23.3 -> 17.0; at 150k items
+// pressure 29.4 -> 32.6.
+constexpr uint32_t kSmallItems = 152 * 4 * kNT;
+using SmallShape = Shape<kNT, 4, 8 | kAhead>;
 // f(shape) with the knob's shape where the layout is tuned, else the default
 template <class Shapes, bool Tuned, class F> void with_shape(int v, F &&f) {
   if constexpr (Tuned) {
@@ -183,20 +224,31 @@ template <class Shapes, bool Tuned, class F> void with_shape(int v, F &&f) {
   }
   f(std::tuple_element_t<0, Shapes>{});
 }
+// the same for a plain launch over n items of a sweep that takes SmallShape
+template <class Shapes, bool Tuned, bool Small, class F> void with_shape_for(uint32_t n, int v, F &&f) {
+  if constexpr (Small) {
+    if (v == 0 && n <= kSmallItems) {
+      f(SmallShape{});
+      return;
+    }
+  }
+  with_shape<Shapes, Tuned>(v, f);
+}
 template <class Sh> std::string shape_text() {
-  return std::to_string(Sh::nt) + "x" + std::to_string(Sh::minb) + "/" + std::to_string(Sh::bt);
+  return std::to_string(Sh::nt) + "x" + std::to_string(Sh::minb) + "/" + std::to_string(Sh::bt & 0xFF);
 }
 template <class Shapes> std::string shapes_text() {
   return "0=" + shape_text<std::tuple_element_t<0, Shapes>>() + " 1=" + shape_text<std::tuple_element_t<1, Shapes>>() +
          " 2=" + shape_text<std::tuple_element_t<2, Shapes>>() + " 3=" + shape_text<std::tuple_element_t<3, Shapes>>();
 }
-using DensityShapes = FreeShapes<8, 16>;
-using SetupShapes = FreeShapes<8, 16>;
-using AccelShapes = FreeShapes<8, 16>;
-using AccelSegShapes = RedShapes<8, 16>;
-using PressureShapes = RedShapes<8, 16>;
-using DiagShapes = FreeShapes<8, 16>;
-using PcgShapes = RedShapes<8, 16>;
+using DensityShapes = FreeShapes<4 | kFill, 8 | kFill>;
+using SetupShapes = FreeShapes<8, 4>;
+using AccelShapes = FreeShapes<8 | kAlone, 8 | kFill>;
+using AccelSegShapes = RedShapes<8 | kFill, 8 | kAlone>;
+using PressureShapes = RedShapes<8 | kAlone, 8 | kFill>;
+using DiagShapes = FreeShapes<4 | kFill, 8 | kFill>;
+using PcgShapes = RedShapes<8 | kAlone, 8>;
+using PcgSegShapes = RedShapes<8, 8 | kAlone>;
 
 // Staged sweeps (the `staging` knob; lists built staged, nhood.hpp): a
 // block's items are the tiles of kStageTile consecutive items the list build
@@ -371,29 +423,35 @@ __global__ void k_seg_active(SegArgs S) { seg_list_active(S); }
 //   rho_i = sum_f m_j W(x_ij) + sum_b (V_j rho0) W(x_ij)
 // ---------------------------------------------------------------------------
 
-template <int NF, int NB, int NT = kNT, int MINB = kMinBlocks, int BT = 16>
+// use(record, in, kernel parameters): the walk of the sweeps that evaluate the
+// kernel per pair
+template <uint32_t FORM, class Load, class Use>
+__device__ __forceinline__ void walk_kernel(NbrList const &L, uint32_t i, QuickKernel const &K, Load &&load, Use &&use) {
+  if (K.quick) walk_nbrs<FORM, false>(L, i, load, [&](float4 x, float, bool in) { use(x, in, K); });
+  else walk_nbrs_singly(L, i, load, [&](float4 x, float, bool in) { use(x, in, K.k); });
+}
+
+template <int NF, int NB, int NT = kNT, int MINB = kMinBlocks, int BT = 4 | kFill>
 __global__ void __launch_bounds__(NT, MINB) k_density(uint32_t n, float4 const *__restrict__ x, float *__restrict__ rho,
                                                  float const *rho0p, Globals G, Nbrs<NF, NB> N) {
   uint32_t i = grid_tid();
   if (i >= n) return;
-  KernelParams K = kparams(*G.h);
+  QuickKernel K = quick_kernel(kparams(*G.h));
   float rho0 = *rho0p;
   f3 xi = mk3(x[i]);
   float acc = 0.0f;
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    for_each_nbr<BT>(F.L, i, false, [&](uint32_t j_, float) {
-      float4 xm = __ldg(F.xm + j_);
-      acc += xm.w * kW(K, sub3(xi, mk3(xm)));
+    walk_kernel<BT>(F.L, i, K, [&](uint32_t j) { return __ldg(F.xm + j); }, [&](float4 xm, bool in, auto const &k) {
+      acc = add_if(in, acc, xm.w * kW(k, sub3(xi, mk3(xm))));
     });
   }
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    for_each_nbr<BT>(B.L, i, false, [&](uint32_t j_, float) {
-      float4 xv = __ldg(B.xV + j_);
-      acc += (xv.w * rho0) * kW(K, sub3(xi, mk3(xv)));
+    walk_kernel<BT>(B.L, i, K, [&](uint32_t j) { return __ldg(B.xV + j); }, [&](float4 xv, bool in, auto const &k) {
+      acc = add_if(in, acc, (xv.w * rho0) * kW(k, sub3(xi, mk3(xv))));
     });
   }
   rho[i] = acc;
@@ -405,13 +463,14 @@ __global__ void __launch_bounds__(kNT, kMinBlocks) k_volume(uint32_t n, float4 c
                                                 Globals G, Nbrs<0, NB> N) {
   uint32_t i = grid_tid();
   if (i >= n) return;
-  KernelParams K = kparams(*G.h);
+  QuickKernel K = quick_kernel(kparams(*G.h));
   f3 xi = mk3(x[i]);
   float acc = 0.0f;
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    for_each_nbr(B.L, i, false, [&](uint32_t j_, float) { acc += kW(K, sub3(xi, mk3(__ldg(B.xV + j_))));
+    walk_kernel<4 | kFill>(B.L, i, K, [&](uint32_t j) { return __ldg(B.xV + j); }, [&](float4 xv, bool in, auto const &k) {
+      acc = add_if(in, acc, kW(k, sub3(xi, mk3(xv))));
     });
   }
   V[i] = 1.0f / acc;
@@ -494,23 +553,34 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
   float rho0 = *rho0p, dt = *G.dt;
   f3 xi = mk3(x[i]);
   float ri = rho[i];
-  f3 c = {0.0f, 0.0f, 0.0f};
+  Divisor rr = divisor(ri * ri);
+  f3 c;
+  bool flat = uc, off;
+  do {
+    c = {0.0f, 0.0f, 0.0f};
+    off = false;
 #pragma unroll
-  for (int q = 0; q < NF; ++q) {
-    FluidN const &F = N.f[q];
-    for_each_nbr<BT, true>(F.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xm = __ldg(F.xm + j_);
-      c = sub3(c, scl3(xm.w / (ri * ri), pgrad(uc, gf_, K, sub3(xi, mk3(xm)))));
-    });
-  }
+    for (int q = 0; q < NF; ++q) {
+      FluidN const &F = N.f[q];
+      walk_nbrs_cached<BT, true>(F.L, i, flat, [&](uint32_t j) { return __ldg(F.xm + j); },
+                                 [&](float4 xm, float gf, bool in, auto cached) {
+        constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
+        c = sub_if(in, c, scl3(divide_noting<kFlat>(xm.w, rr, off), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xm)))));
+      });
+    }
 #pragma unroll
-  for (int q = 0; q < NB; ++q) {
-    BoundN const &B = N.b[q];
-    for_each_nbr<BT, true>(B.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xv = __ldg(B.xV + j_);
-      c = sub3(c, scl3(((0.7f * 2.0f) * rho0) * (xv.w / (ri * ri)), pgrad(uc, gf_, K, sub3(xi, mk3(xv)))));
-    });
-  }
+    for (int q = 0; q < NB; ++q) {
+      BoundN const &B = N.b[q];
+      walk_nbrs_cached<BT, true>(B.L, i, flat, [&](uint32_t j) { return __ldg(B.xV + j); },
+                                 [&](float4 xv, float gf, bool in, auto cached) {
+        constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
+        c = sub_if(in, c, scl3(((0.7f * 2.0f) * rho0) * divide_noting<kFlat>(xv.w, rr, off),
+                               pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
+      });
+    }
+    if (!off) break;
+    flat = false;
+  } while (true);
   cout[i] = make_float4(c.x, c.y, c.z, 0.0f);
   if (!(isfinite(c.x) && isfinite(c.y) && isfinite(c.z))) *bad = 1;
   f3 vi = mk3(v[i]), ci = c;
@@ -519,25 +589,24 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    for_each_nbr<BT>(F.L, i, uc, [&](uint32_t j_, float gf_) {
-      uint32_t j = j_;
-      float4 xm = __ldg(F.xm + j);
-      f3 g = pgrad(uc, gf_, K, sub3(xi, mk3(xm)));
-      float mj = xm.w;
-      sa += mj * dot3(sub3(vi, mk3(__ldg(F.v + j))), g);
-      aa += mj * dot3(ci, g);
-      aa -= (mj * (mi / (ri * ri))) * nsq3(g);
+    walk_nbrs_cached<BT>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.v + j))}; },
+                         [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
+      f3 g = pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)));
+      float mj = r.x.w;
+      sa = add_if(in, sa, mj * dot3(sub3(vi, r.v), g));
+      aa = add_if(in, aa, mj * dot3(ci, g));
+      aa = add_if(in, aa, -((mj * (mi / (ri * ri))) * nsq3(g)));
     });
   }
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    for_each_nbr<BT>(B.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xv = __ldg(B.xV + j_);
-      f3 g = pgrad(uc, gf_, K, sub3(xi, mk3(xv)));
+    walk_nbrs_cached<BT>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+                         [&](float4 xv, float gf, bool in, auto cached) {
+      f3 g = pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)));
       float w = rho0 * xv.w;
-      sa += w * dot3(sub3(vi, f3{0.0f, 0.0f, 0.0f}), g);
-      aa += w * dot3(ci, g);
+      sa = add_if(in, sa, w * dot3(sub3(vi, f3{0.0f, 0.0f, 0.0f}), g));
+      aa = add_if(in, aa, w * dot3(ci, g));
     });
   }
   p[i] = 0.0f;
@@ -569,7 +638,7 @@ __device__ __forceinline__ int jacobi_first(Globals const &G, RestDensities cons
 
 // iisph.iteration_pressure_acceleration (schemes/iisph.hpp:358-423).
 // `done` (device-loop mode) skips the work once the loop has converged.
-template <int NF, int NB, int BT = 8>
+template <int NF, int NB, int BT = 8 | kAlone>
 __device__ __forceinline__ void iisph_accel_item(uint32_t i, float4 const *__restrict__ x, float const *__restrict__ p,
                                                  float const *__restrict__ rho, float4 *__restrict__ a,
                                                  KernelParams const &K, bool uc, float rho0, Nbrs<NF, NB> const &N) {
@@ -580,26 +649,25 @@ __device__ __forceinline__ void iisph_accel_item(uint32_t i, float4 const *__res
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    for_each_nbr<BT>(F.L, i, uc, [&](uint32_t j_, float gf_) {
-      uint32_t j = j_;
-      float4 xm = __ldg(F.xm + j);
-      float coef = xm.w * (pri + __ldg(F.pr + j));
-      acc = sub3(acc, scl3(coef, pgrad(uc, gf_, K, sub3(xi, mk3(xm)))));
+    walk_nbrs_cached<BT>(F.L, i, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), __ldg(F.pr + j)}; },
+                         [&](WithRec<float> const &r, float gf, bool in, auto cached) {
+      float coef = r.x.w * (pri + r.v);
+      acc = sub_if(in, acc, scl3(coef, pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
     });
   }
   float bterm = (2.0f * pi) / (ri * ri);
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    for_each_nbr<BT>(B.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xv = __ldg(B.xV + j_);
+    walk_nbrs_cached<BT>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+                         [&](float4 xv, float gf, bool in, auto cached) {
       float coef = ((0.7f * rho0) * xv.w) * bterm;
-      acc = sub3(acc, scl3(coef, pgrad(uc, gf_, K, sub3(xi, mk3(xv)))));
+      acc = sub_if(in, acc, scl3(coef, pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
     });
   }
   a[i] = make_float4(acc.x, acc.y, acc.z, 0.0f);
 }
-template <int NF, int NB, int NT = kNT, int MINB = kMinBlocks, int BT = 8>
+template <int NF, int NB, int NT = kNT, int MINB = kMinBlocks, int BT = 8 | kAlone>
 __global__ void __launch_bounds__(NT, MINB) k_iisph_accel(uint32_t n, float4 const *__restrict__ x, float const *__restrict__ p,
                                                      float const *__restrict__ rho, float4 *__restrict__ a,
                                                      float const *rho0p, Globals G, Nbrs<NF, NB> N, int const *done) {
@@ -618,7 +686,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_accel(uint32_t n, float4 con
 // batched models: the tiles of the slots still iterating
 // (DYN: each block takes the next tile from a work counter instead of a
 // static share of the tiles; the tiles' items and arithmetic are the same)
-template <int NF, int NB, int MINB = kMinBlocks, int BT = 8, bool DYN = false>
+template <int NF, int NB, int MINB = kMinBlocks, int BT = 8 | kAlone, bool DYN = false>
 __global__ void __launch_bounds__(kNT, MINB) k_iisph_accel_seg(float4 const *__restrict__ x, float const *__restrict__ p,
                                                          float const *__restrict__ rho, float4 *__restrict__ a,
                                                          float const *rho0p, Globals G, Nbrs<NF, NB> N, SegArgs S,
@@ -676,7 +744,7 @@ __device__ __forceinline__ double pressure_finish(uint32_t i, PressureArgs const
 }
 
 // one item of iteration_pressure; returns its density-error term
-template <int NF, int NB, int BT = 16>
+template <int NF, int NB, int BT = 8 | kAlone>
 __device__ __forceinline__ double iisph_pressure_item(uint32_t i, PressureArgs const &A, KernelParams const &K, bool uc,
                                                       float rho0, float dt, float omega, Nbrs<NF, NB> const &N) {
   f3 xi = mk3(A.x[i]), ai = mk3(A.a[i]);
@@ -684,24 +752,23 @@ __device__ __forceinline__ double iisph_pressure_item(uint32_t i, PressureArgs c
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    for_each_nbr<BT>(F.L, i, uc, [&](uint32_t j_, float gf_) {
-      uint32_t j = j_;
-      float4 xm = __ldg(F.xm + j);
-      ap += xm.w * dot3(sub3(ai, mk3(__ldg(F.a + j))), pgrad(uc, gf_, K, sub3(xi, mk3(xm))));
+    walk_nbrs_cached<BT>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.a + j))}; },
+                         [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
+      ap = add_if(in, ap, r.x.w * dot3(sub3(ai, r.v), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
     });
   }
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    for_each_nbr<BT>(B.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xv = __ldg(B.xV + j_);
-      ap += (rho0 * xv.w) * dot3(sub3(ai, f3{0.0f, 0.0f, 0.0f}), pgrad(uc, gf_, K, sub3(xi, mk3(xv))));
+    walk_nbrs_cached<BT>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+                         [&](float4 xv, float gf, bool in, auto cached) {
+      ap = add_if(in, ap, (rho0 * xv.w) * dot3(sub3(ai, f3{0.0f, 0.0f, 0.0f}), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
     });
   }
   return pressure_finish(i, A, ap, rho0, dt, omega);
 }
 
-template <int NF, int NB, int MINB = kMinBlocks, int BT = 16>
+template <int NF, int NB, int MINB = kMinBlocks, int BT = 8 | kAlone>
 __global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure(uint32_t n, PressureArgs A, Globals G, Nbrs<NF, NB> N, Red R,
                                                         int first, int last_group, int const *done) {
   int ended = done ? *(volatile int const *)done : 0, zero = done ? *(volatile int const *)(done + 1) : 0;
@@ -730,7 +797,7 @@ __global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure(uint32_t n, Pressu
 // each slot's iteration goes to scal[slot][kSsAprde]
 // (DYN: a persistent grid whose blocks take tiles from a work counter; the
 // per-tile partial sums and their per-slot commit are unchanged)
-template <int NF, int NB, int MINB = kMinBlocks, int BT = 16, bool DYN = false>
+template <int NF, int NB, int MINB = kMinBlocks, int BT = 8 | kAlone, bool DYN = false>
 __global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure_seg(PressureArgs A, Globals G, Nbrs<NF, NB> N, SegArgs S,
                                                                   int const *first) {
   bool zero = *(volatile int const *)first != 0;
@@ -813,7 +880,7 @@ __global__ void __launch_bounds__(kNT, 4) k_iisph_accel_staged(uint32_t n, float
         });
         a[i] = make_float4(acc.x, acc.y, acc.z, 0.0f);
       } else {
-        iisph_accel_item<1, 1, BT>(i, x, p, rho, a, K, uc, rho0, N);
+        iisph_accel_item<1, 1, 8 | kAlone>(i, x, p, rho, a, K, uc, rho0, N);
       }
     }
     __syncthreads(); // the next tile reuses the shared memory
@@ -861,7 +928,7 @@ __global__ void __launch_bounds__(kNT, 4) k_iisph_pressure_staged(uint32_t n, Pr
         });
         part += pressure_finish(i, A, ap, rho0, dt, omega);
       } else {
-        part += iisph_pressure_item<1, 1, BT>(i, A, K, uc, rho0, dt, omega, N);
+        part += iisph_pressure_item<1, 1, 8 | kAlone>(i, A, K, uc, rho0, dt, omega, N);
       }
     }
     __syncthreads();
@@ -990,29 +1057,40 @@ __global__ void __launch_bounds__(kNT, kMinBlocks) k_viscosity(uint32_t n, float
   float hh = (0.01f * h) * h;
   f3 xi = mk3(x[i]), vi = mk3(v[i]);
   float ri = rho[i];
-  f3 ai = mk3(a[i]);
+  f3 ai, a0 = mk3(a[i]);
+  Divisor rdiv = divisor(ri);
+  bool flat = uc, off;
+  do {
+    ai = a0;
+    off = false;
 #pragma unroll
-  for (int q = 0; q < NF; ++q) {
-    FluidN const &F = N.f[q];
-    for_each_nbr(F.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xr = __ldg(F.xm + j_);
-      f3 xij = sub3(xi, mk3(xr));
-      float coef = (((10.0f * (mu / ri)) * xr.w) * dot3(sub3(vi, mk3(__ldg(F.v + j_))), xij)) / (nsq3(xij) + hh);
-      ai = add3(ai, scl3(coef, pgrad(uc, gf_, K, xij)));
-    });
-  }
+    for (int q = 0; q < NF; ++q) {
+      FluidN const &F = N.f[q];
+      walk_nbrs_cached<8>(F.L, i, flat, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.v + j))}; },
+                          [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
+        constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
+        f3 xij = sub3(xi, mk3(r.x));
+        float coef = divide_noting<kFlat>(((10.0f * (mu / ri)) * r.x.w) * dot3(sub3(vi, r.v), xij), nsq3(xij) + hh, off);
+        ai = add_if(in, ai, scl3(coef, pgrad(is_cached(cached), gf, K, xij)));
+      });
+    }
 #pragma unroll
-  for (int q = 0; q < NB; ++q) {
-    BoundN const &B = N.b[q];
-    float bmu = *B.mu;
-    for_each_nbr(B.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xv = __ldg(B.xV + j_);
-      f3 xij = sub3(xi, mk3(xv));
-      float coef = (((10.0f * (bmu / ri)) * ((rho0 * xv.w) / ri)) * dot3(sub3(vi, f3{0.0f, 0.0f, 0.0f}), xij)) /
-                   (nsq3(xij) + hh);
-      ai = add3(ai, scl3(coef, pgrad(uc, gf_, K, xij)));
-    });
-  }
+    for (int q = 0; q < NB; ++q) {
+      BoundN const &B = N.b[q];
+      float bmu = *B.mu;
+      walk_nbrs_cached<8>(B.L, i, flat, [&](uint32_t j) { return __ldg(B.xV + j); },
+                          [&](float4 xv, float gf, bool in, auto cached) {
+        constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
+        f3 xij = sub3(xi, mk3(xv));
+        float vr = divide_noting<kFlat>(rho0 * xv.w, rdiv, off);
+        float coef = divide_noting<kFlat>(((10.0f * (bmu / ri)) * vr) * dot3(sub3(vi, f3{0.0f, 0.0f, 0.0f}), xij),
+                                          nsq3(xij) + hh, off);
+        ai = add_if(in, ai, scl3(coef, pgrad(is_cached(cached), gf, K, xij)));
+      });
+    }
+    if (!off) break;
+    flat = false;
+  } while (true);
   a[i] = make_float4(ai.x, ai.y, ai.z, 0.0f);
 }
 
@@ -1034,24 +1112,32 @@ __global__ void __launch_bounds__(kNT, kMinBlocks) k_correction(uint32_t n, uint
   f3 xi = mk3(x[i]);
   float ri = rho[i];
   M3 A;
+  Divisor rdiv = divisor(ri);
+  bool flat = uc, off;
+  do {
 #pragma unroll
-  for (int e = 0; e < 9; ++e) A.m[e] = 0.0f;
+    for (int e = 0; e < 9; ++e) A.m[e] = 0.0f;
+    off = false;
 #pragma unroll
-  for (int q = 0; q < NF; ++q) {
-    FluidN const &F = N.f[q];
-    for_each_nbr(F.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xm = __ldg(F.xm + j_);
-      f3 xj = mk3(xm);
-      f3 g = pgrad(uc, gf_, K, sub3(xi, xj));
-      f3 d = sub3(xj, xi);
-      float sc = xm.w / ri;
-      float gv[3] = {g.x, g.y, g.z}, dv[3] = {d.x, d.y, d.z};
+    for (int q = 0; q < NF; ++q) {
+      FluidN const &F = N.f[q];
+      walk_nbrs_cached<8>(F.L, i, flat, [&](uint32_t j) { return __ldg(F.xm + j); },
+                          [&](float4 xm, float gf, bool in, auto cached) {
+        constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
+        f3 xj = mk3(xm);
+        f3 g = pgrad(is_cached(cached), gf, K, sub3(xi, xj));
+        f3 d = sub3(xj, xi);
+        float sc = divide_noting<kFlat>(xm.w, rdiv, off);
+        float gv[3] = {g.x, g.y, g.z}, dv[3] = {d.x, d.y, d.z};
 #pragma unroll
-      for (int c = 0; c < 3; ++c)
+        for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int r = 0; r < 3; ++r) A.m[3 * c + r] = A.m[3 * c + r] + sc * (gv[r] * dv[c]);
-    });
-  }
+          for (int r = 0; r < 3; ++r) A.m[3 * c + r] = add_if(in, A.m[3 * c + r], sc * (gv[r] * dv[c]));
+      });
+    }
+    if (!off) break;
+    flat = false;
+  } while (true);
   M3 R = pinv3(A);
 #pragma unroll
   for (int e = 0; e < 9; ++e) L[size_t(e) * cap + i] = R.m[e];
@@ -1070,7 +1156,7 @@ __global__ void k_identity9(uint32_t n, uint32_t cap, float *L) {
 // (x, m / rho).
 // GC (wkbb18_gc, share/schemes/wkbb18_gc.prtcl): every kernel gradient
 // premultiplied by the item's gradient correction L_i (planar, capacity lcap)
-template <int NB, bool GC = false, int NT = kNT, int MINB = kMinBlocks, int BT = 8>
+template <int NB, bool GC = false, int NT = kNT, int MINB = kMinBlocks, int BT = 4 | kFill>
 __global__ void __launch_bounds__(NT, MINB) k_wkbb18_diag(uint32_t n, uint32_t cap, float4 const *__restrict__ xmr,
                                                      float const *__restrict__ rho, float *__restrict__ sp,
                                                      float const *rho0p, float const *mup, Globals G, NbrList self,
@@ -1091,34 +1177,34 @@ __global__ void __launch_bounds__(NT, MINB) k_wkbb18_diag(uint32_t n, uint32_t c
   for (int k = 0; k < 9; ++k) S[k] = 0.0f;
   float hh = (0.01f * h) * h;
   float cmu = 10.0f * (mu / ri);
-  for_each_nbr<BT>(self, i, uc, [&](uint32_t j_, float gf_) {
-    float4 xj = __ldg(xmr + j_);
+  // (bound by its arithmetic: 113 us with divisions, 119 without their branches)
+  walk_nbrs_cached<BT>(self, i, uc, [&](uint32_t j) { return __ldg(xmr + j); },
+                       [&](float4 xj, float gf, bool in, auto cached) {
     f3 xij = sub3(xi, mk3(xj));
     float coef = (cmu * xj.w) / (nsq3(xij) + hh);
-    f3 g = pgrad(uc, gf_, K, xij);
+    f3 g = pgrad(is_cached(cached), gf, K, xij);
     if (GC) g = mv3(Li, g);
     float gv[3] = {g.x, g.y, g.z}, xv[3] = {xij.x, xij.y, xij.z};
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-      for (int r = 0; r < 3; ++r) S[3 * c + r] += coef * (gv[r] * xv[c]);
-    });
-
+      for (int r = 0; r < 3; ++r) S[3 * c + r] = add_if(in, S[3 * c + r], coef * (gv[r] * xv[c]));
+  });
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
     float bmu = *B.mu;
-    for_each_nbr<BT>(B.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xv = __ldg(B.xV + j_);
+    walk_nbrs_cached<BT>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+                         [&](float4 xv, float gf, bool in, auto cached) {
       f3 xij = sub3(xi, mk3(xv));
       float coef = ((10.0f * (bmu / ri)) * ((rho0 * xv.w) / ri)) / (nsq3(xij) + hh);
-      f3 g = pgrad(uc, gf_, K, xij);
+      f3 g = pgrad(is_cached(cached), gf, K, xij);
       if (GC) g = mv3(Li, g);
       float gv[3] = {g.x, g.y, g.z}, xw[3] = {xij.x, xij.y, xij.z};
 #pragma unroll
       for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int r = 0; r < 3; ++r) S[3 * c + r] += coef * (gv[r] * xw[c]);
+        for (int r = 0; r < 3; ++r) S[3 * c + r] = add_if(in, S[3 * c + r], coef * (gv[r] * xw[c]));
     });
   }
   M3 A;
@@ -1160,7 +1246,7 @@ struct PcgArgs {
 
 // system product of wkbb18.accumulate_acceleration (schemes/wkbb18.hpp:
 // 339-396): (A w)_i = w_i - dt * a_f(w)_i
-template <int NB, bool GC, int BT = 8>
+template <int NB, bool GC, int BT = 8 | kAlone>
 __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const &K, bool uc, float dt, float rho0,
                                             float mu, Nbrs<0, NB> const &N, float4 const *__restrict__ w, uint32_t i) {
   float Li[9];
@@ -1172,31 +1258,40 @@ __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const
   f3 xi = mk3(P.xmr[i]), wi = mk3(w[i]);
   float ri = P.rho[i];
   float cmu = 10.0f * (mu / ri);
-  f3 af = {0.0f, 0.0f, 0.0f};
-  for_each_nbr<BT>(P.self, i, uc, [&](uint32_t j_, float gf_) {
-    uint32_t j = j_;
-    float4 xj = __ldg(P.xmr + j);
-    f3 xij = sub3(xi, mk3(xj));
-    float coef = ((cmu * xj.w) * dot3(sub3(wi, mk3(__ldg(w + j))), xij)) / (nsq3(xij) + hh);
-    f3 g = pgrad(uc, gf_, K, xij);
-    if (GC) g = mv3(Li, g);
-    af = add3(af, scl3(coef, g));
-    });
-
-#pragma unroll
-  for (int q = 0; q < NB; ++q) {
-    BoundN const &B = N.b[q];
-    float bmu = *B.mu;
-    float cb_mu = 10.0f * (bmu / ri);
-    for_each_nbr<BT>(B.L, i, uc, [&](uint32_t j_, float gf_) {
-      float4 xv = __ldg(B.xV + j_);
-      f3 xij = sub3(xi, mk3(xv));
-      float coef = ((cb_mu * ((rho0 * xv.w) / ri)) * dot3(wi, xij)) / (nsq3(xij) + hh);
-      f3 g = pgrad(uc, gf_, K, xij);
+  Divisor rdiv = divisor(ri);
+  f3 af;
+  bool flat = uc, off;
+  do {
+    af = {0.0f, 0.0f, 0.0f};
+    off = false;
+    walk_nbrs_cached<BT>(P.self, i, flat, [&](uint32_t j) { return WithRec<f3>{__ldg(P.xmr + j), mk3(__ldg(w + j))}; },
+                         [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
+      constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
+      f3 xij = sub3(xi, mk3(r.x));
+      float coef = divide_noting<kFlat>((cmu * r.x.w) * dot3(sub3(wi, r.v), xij), nsq3(xij) + hh, off);
+      f3 g = pgrad(is_cached(cached), gf, K, xij);
       if (GC) g = mv3(Li, g);
-      af = add3(af, scl3(coef, g));
+      af = add_if(in, af, scl3(coef, g));
     });
-  }
+#pragma unroll
+    for (int q = 0; q < NB; ++q) {
+      BoundN const &B = N.b[q];
+      float bmu = *B.mu;
+      float cb_mu = 10.0f * (bmu / ri);
+      walk_nbrs_cached<BT>(B.L, i, flat, [&](uint32_t j) { return __ldg(B.xV + j); },
+                           [&](float4 xv, float gf, bool in, auto cached) {
+        constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
+        f3 xij = sub3(xi, mk3(xv));
+        float vr = divide_noting<kFlat>(rho0 * xv.w, rdiv, off);
+        float coef = divide_noting<kFlat>((cb_mu * vr) * dot3(wi, xij), nsq3(xij) + hh, off);
+        f3 g = pgrad(is_cached(cached), gf, K, xij);
+        if (GC) g = mv3(Li, g);
+        af = add_if(in, af, scl3(coef, g));
+      });
+    }
+    if (!off) break;
+    flat = false;
+  } while (true);
   return sub3(wi, scl3(dt, af));
 }
 
@@ -1219,7 +1314,7 @@ __device__ __forceinline__ double pcg_q_finish(PcgArgs const &P, uint32_t i, f3 
 // y = M r, p = -y; dots b.b, r.r, r.y (solver/cg_openmp.hpp:48-96)
 // per-item parts of the PCG kernels (shared by the plain and the tiled
 // launches, so both compute the same values)
-template <int NB, bool GC, int BT = 8>
+template <int NB, bool GC, int BT = 8 | kAlone>
 __device__ __forceinline__ void pcg_init_item(PcgArgs const &P, KernelParams const &K, bool uc, float dt, float rho0,
                                               float mu, Nbrs<0, NB> const &N, uint32_t i, double &bb, double &rr,
                                               double &ry) {
@@ -1238,7 +1333,7 @@ __device__ __forceinline__ void pcg_init_finish(PcgArgs const &P, uint32_t i, f3
   rr += f2d(dot3(r, r));
   ry += f2d(dot3(r, y));
 }
-template <int NB, bool GC, int BT = 8>
+template <int NB, bool GC, int BT = 8 | kAlone>
 __device__ __forceinline__ double pcg_q_item(PcgArgs const &P, KernelParams const &K, bool uc, float dt, float rho0,
                                              float mu, Nbrs<0, NB> const &N, uint32_t i) {
   return pcg_q_finish(P, i, wkbb18_system<NB, GC, BT>(P, K, uc, dt, rho0, mu, N, P.P, i));
@@ -1297,7 +1392,7 @@ __device__ __forceinline__ void pcg_update_scalars(double *sc, int *st, double r
   }
 }
 
-template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8>
+template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8 | kAlone>
 __global__ void __launch_bounds__(kNT, MINB) k_pcg_init(PcgArgs P, Globals G, Nbrs<0, NB> N, Red R) {
   KernelParams K = kparams(*G.h);
   bool uc = use_cache(N, K);
@@ -1310,7 +1405,7 @@ __global__ void __launch_bounds__(kNT, MINB) k_pcg_init(PcgArgs P, Globals G, Nb
 }
 
 // q = A p; p.q; alpha or break (solver/cg_openmp.hpp:121-151)
-template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8>
+template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8 | kAlone>
 __global__ void __launch_bounds__(kNT, MINB) k_pcg_q(PcgArgs P, Globals G, Nbrs<0, NB> N, Red R) {
   if (!*(volatile int *)&R.status[kStPcgActive]) return;
   KernelParams K = kparams(*G.h);
@@ -1388,7 +1483,7 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_init_staged(PcgArgs P, Globals G
         pcg_init_finish(P, i, wkbb18_system_staged<BT>(P, K, uc, dt, rho0, mu, bmu, SA, B, sx, sy, P.X, i), bb, rr,
                         ry);
       else
-        pcg_init_item<1, false, BT>(P, K, uc, dt, rho0, mu, N, i, bb, rr, ry);
+        pcg_init_item<1, false, 8 | kAlone>(P, K, uc, dt, rho0, mu, N, i, bb, rr, ry);
     }
     __syncthreads();
   }
@@ -1412,7 +1507,7 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_q_staged(PcgArgs P, Globals G, N
     bool st = stage_system(SA, tile, sx, sy, P, B, P.P);
     if (i < P.n)
       pq += st ? pcg_q_finish(P, i, wkbb18_system_staged<BT>(P, K, uc, dt, rho0, mu, bmu, SA, B, sx, sy, P.P, i))
-               : pcg_q_item<1, false, BT>(P, K, uc, dt, rho0, mu, N, i);
+               : pcg_q_item<1, false, 8 | kAlone>(P, K, uc, dt, rho0, mu, N, i);
     __syncthreads();
   }
   double v[1] = {pq}, out[1];
@@ -1584,7 +1679,7 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_q_tiles(PcgArgs P, Globals G, Nb
     if (has) {
       f3 q;
       if (over) {
-        q = wkbb18_system<NB, false, 8>(P, K, uc, dt, rho0, mu, N, P.P, i);
+        q = wkbb18_system<NB, false, 8 | kAlone>(P, K, uc, dt, rho0, mu, N, P.P, i);
       } else {
         f3 xi = mk3(P.xmr[i]), wi = mk3(P.P[i]);
         float ri = P.rho[i];
@@ -1664,7 +1759,7 @@ __global__ void k_pcg_control(PcgArgs P, Red R, cudaGraphConditionalHandle h, in
 
 // --- the PCG loop over the tiles of a batched model, per slot -------------
 
-template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8>
+template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8 | kAlone>
 __global__ void __launch_bounds__(kNT, MINB) k_pcg_init_seg(PcgArgs P, Globals G, Nbrs<0, NB> N, SegArgs S) {
   uint4 T = S.tiles[blockIdx.x];
   uint32_t slot = T.x;
@@ -1682,7 +1777,7 @@ __global__ void __launch_bounds__(kNT, MINB) k_pcg_init_seg(PcgArgs P, Globals G
   }
 }
 
-template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8>
+template <int NB, bool GC = false, int MINB = kMinBlocks, int BT = 8 | kAlone>
 __global__ void __launch_bounds__(kNT, MINB) k_pcg_q_seg(PcgArgs P, Globals G, Nbrs<0, NB> N, SegArgs S) {
   uint4 T = S.tiles[blockIdx.x];
   uint32_t slot = T.x;
@@ -2340,7 +2435,7 @@ public:
       auto N = S->nbrs<NF, NB>(v, s);
       float *pr = S->model_->pr_buffer(F.g, s);
       ProfScope ps(S->model_->prof, "iisph_setup", s);
-      with_shape<SetupShapes, NF == 1 && NB == 1>(S->model_->tune.v[kTuneSetup], [&](auto sh) {
+      with_shape_for<SetupShapes, NF == 1 && NB == 1, NF == 1 && NB == 1>(n, S->model_->tune.v[kTuneSetup], [&](auto sh) {
         using Sh = decltype(sh);
         k_iisph_setup<NF, NB, Sh::nt, Sh::minb, Sh::bt><<<div_up(n, Sh::nt), Sh::nt, 0, s>>>(
             n, dptr<float4>(F.x), dptr<float4>(F.v), dptr<float4>(F.c), dptr<float>(F.m), dptr<float>(F.rho),
@@ -2390,7 +2485,7 @@ public:
       } else if (SA) {
         if (SA->ntiles) {
           if (NF == 1 && NB == 1 && tv == 4)
-            k_iisph_accel_seg<NF, NB, kMinBlocks, 8, true><<<std::min(SA->ntiles, kActiveBlocks), kNT, 0, s>>>(
+            k_iisph_accel_seg<NF, NB, kMinBlocks, 8 | kAlone, true><<<std::min(SA->ntiles, kActiveBlocks), kNT, 0, s>>>(
                 x, p, rho, a, rho0, G, N, *SA, S->model_->status_d + kStJacFirst);
           else
             with_shape<AccelSegShapes, NF == 1 && NB == 1>(tv, [&](auto sh) {
@@ -2400,7 +2495,7 @@ public:
             });
         }
       } else {
-        with_shape<AccelShapes, NF == 1 && NB == 1>(tv, [&](auto sh) {
+        with_shape_for<AccelShapes, NF == 1 && NB == 1, NF == 1 && NB == 1>(n, tv, [&](auto sh) {
           using Sh = decltype(sh);
           k_iisph_accel<NF, NB, Sh::nt, Sh::minb, Sh::bt><<<div_up(n, Sh::nt), Sh::nt, 0, s>>>(n, x, p, rho, a, rho0,
                                                                                             G, N, done);
@@ -2443,10 +2538,10 @@ public:
       if (staged) {
       } else if (SA && NF == 1 && NB == 1 && tvp == 4) {
         if (SA->ntiles)
-          k_iisph_pressure_seg<NF, NB, kMinBlocks, 16, true><<<std::min(SA->ntiles, kActiveBlocks), kNT, 0, s>>>(
+          k_iisph_pressure_seg<NF, NB, kMinBlocks, 8 | kAlone, true><<<std::min(SA->ntiles, kActiveBlocks), kNT, 0, s>>>(
               PA, G, N, *SA, S->model_->status_d + kStJacFirst);
       } else
-      with_shape<PressureShapes, NF == 1 && NB == 1>(tvp, [&](auto sh) {
+      with_shape_for<PressureShapes, NF == 1 && NB == 1, NF == 1 && NB == 1>(SA ? ~0u : n, tvp, [&](auto sh) {
         using Sh = decltype(sh);
         if (SA) {
           if (SA->ntiles)
@@ -2798,15 +2893,18 @@ public:
       }
       if constexpr (kTuned)
         if (staged) k_pcg_init_staged<8><<<rg, kNT, kStageSmem, s>>>(P, G, N, R, st);
-      if (!staged)
-      with_shape<PcgShapes, kTuned>(tv_init, [&](auto sh) {
-        using Sh = decltype(sh);
-        if (seg) {
+      if (staged) {
+      } else if (seg) {
+        with_shape<PcgSegShapes, kTuned>(tv_init, [&](auto sh) {
+          using Sh = decltype(sh);
           if (tg) k_pcg_init_seg<NB, GC, Sh::minb, Sh::bt><<<tg, kNT, 0, s>>>(P, G, N, SA);
-        } else {
+        });
+      } else {
+        with_shape_for<PcgShapes, kTuned, NB == 1>(P.n, tv_init, [&](auto sh) {
+          using Sh = decltype(sh);
           k_pcg_init<NB, GC, Sh::minb, Sh::bt><<<rg, kNT, 0, s>>>(P, G, N, R);
-        }
-      });
+        });
+      }
       count_launch();
     }
     PG_LAUNCH_CHECK();
@@ -2835,15 +2933,18 @@ public:
         else if (staged)
           k_pcg_q_staged<8><<<rg, kNT, kStageSmem, cs>>>(P, G, N, R, st);
       }
-      if (!tiles && !staged)
-        with_shape<PcgShapes, kTuned>(tv_q, [&](auto sh) {
+      if (tiles || staged) {
+      } else if (seg) {
+        with_shape<PcgSegShapes, kTuned>(tv_q, [&](auto sh) {
           using Sh = decltype(sh);
-          if (seg) {
-            if (tg) k_pcg_q_seg<NB, GC, Sh::minb, Sh::bt><<<tg, kNT, 0, cs>>>(P, G, N, SA);
-          } else {
-            k_pcg_q<NB, GC, Sh::minb, Sh::bt><<<rg, kNT, 0, cs>>>(P, G, N, R);
-          }
+          if (tg) k_pcg_q_seg<NB, GC, Sh::minb, Sh::bt><<<tg, kNT, 0, cs>>>(P, G, N, SA);
         });
+      } else {
+        with_shape_for<PcgShapes, kTuned, NB == 1>(P.n, tv_q, [&](auto sh) {
+          using Sh = decltype(sh);
+          k_pcg_q<NB, GC, Sh::minb, Sh::bt><<<rg, kNT, 0, cs>>>(P, G, N, R);
+        });
+      }
       count_launch();
       if (prof) model_->prof.end(cs);
       if (prof) model_->prof.begin("pcg_update", cs);
