@@ -10,6 +10,46 @@ namespace prtcl_gpu {
 namespace {
 constexpr uint32_t kNoSrc = 0xFFFFFFFFu;
 char const *kSchemes[] = {"density", "gravity", "symplectic_euler", "iisph", "wkbb18", "aiast12"};
+
+// a slot's range of a group in the new layout: its first item, its first item
+// in the old layout (kNoSrc: a new scene), a new scene's positions
+struct SlotRange {
+  uint32_t first, old;
+  float const *x;
+};
+// the slot of item i (ranges by first item, empty ones included)
+__device__ __forceinline__ SlotRange slot_of(SlotRange const *slots, uint32_t n, uint32_t i) {
+  uint32_t lo = 0, hi = n - 1;
+  while (lo < hi) {
+    uint32_t mid = (lo + hi + 1) / 2;
+    if (slots[mid].first <= i) lo = mid;
+    else hi = mid - 1;
+  }
+  return slots[lo];
+}
+// map[i]: the old index of the new layout's item i
+__global__ void k_slot_map(SlotRange const *slots, uint32_t n, uint32_t items, uint32_t *map) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= items) return;
+  SlotRange r = slot_of(slots, n, i);
+  map[i] = r.old == kNoSrc ? kNoSrc : r.old + (i - r.first);
+}
+// the new scenes' items: position and, where given, mass and time of birth
+// (one launch for all scenes; a copy, an allocation and a wait for each field of
+// each scene, and the maps put together item by item on the host, took 11.1 ms
+// of the 45 of 48 scenes' arrival, 8 steps and departure, now 2.2 of 36)
+__global__ void k_slot_fill(SlotRange const *slots, uint32_t n, uint32_t items, float4 *x, float *m, float *tb,
+                            float mass, float birth) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= items) return;
+  SlotRange r = slot_of(slots, n, i);
+  if (r.old != kNoSrc) return;
+  float const *p = r.x + size_t(i - r.first) * 3;
+  x[i] = make_float4(p[0], p[1], p[2], 0.0f);
+  if (m) m[i] = mass;
+  if (tb) tb[i] = birth;
+}
+
 std::string full(char const *n) { return std::string("prtcl::schemes::") + n + "[T=f32, N=3, K=Cubic Spline]"; }
 } // namespace
 
@@ -57,9 +97,23 @@ Batch::Batch(prtcl_gpu_batch_params const &p) : p_(p) {
   nh_.load(m_);
   nh_.set_radius(2.0 * double(h));
   PG_CUDA(cudaStreamSynchronize(s));
+  PG_CUDA(cudaStreamCreateWithFlags(&up_, cudaStreamNonBlocking));
 }
 
-Batch::~Batch() { cudaStreamSynchronize(m_.stream()); }
+Batch::~Batch() {
+  cudaStreamSynchronize(m_.stream());
+  for (auto &sc : scenes_) drop_positions(sc);
+  if (up_) {
+    cudaStreamSynchronize(up_);
+    cudaStreamDestroy(up_);
+  }
+}
+
+// (on the model's stream, which may still read them)
+void Batch::drop_positions(Scene &sc) {
+  if (sc.x) cudaFreeAsync(sc.x, m_.stream());
+  sc.x = nullptr;
+}
 
 void Batch::set_global(char const *name, void const *value) {
   SmallField *f = m_.find_global(name);
@@ -76,8 +130,21 @@ int64_t Batch::add(float const *xf, size_t nf, float const *xb, size_t nb) {
   sc.id = next_id_++;
   sc.nf = nf;
   sc.nb = nb;
-  sc.xf.assign(xf, xf + 3 * nf);
-  sc.xb.assign(xb, xb + 3 * nb);
+  // straight to the device, where they wait for the next commit; on a stream
+  // of its own, so that the call does not wait for steps that are under way
+  size_t nx = 3 * nf, nbx = 3 * nb;
+  if (nx + nbx) {
+    PG_CUDA(cudaMallocAsync(&sc.x, (nx + nbx) * sizeof(float), up_));
+    try {
+      if (nx) PG_CUDA(cudaMemcpyAsync(sc.x, xf, nx * sizeof(float), cudaMemcpyHostToDevice, up_));
+      if (nbx) PG_CUDA(cudaMemcpyAsync(sc.x + nx, xb, nbx * sizeof(float), cudaMemcpyHostToDevice, up_));
+      PG_CUDA(cudaStreamSynchronize(up_));
+      scenes_.reserve(scenes_.size() + 1);
+    } catch (...) {
+      cudaFreeAsync(sc.x, up_);
+      throw;
+    }
+  }
   scenes_.push_back(std::move(sc));
   dirty_ = true;
   return scenes_.back().id;
@@ -92,6 +159,7 @@ Batch::Scene &Batch::find(int64_t id) {
 void Batch::remove(int64_t id) {
   Scene &sc = find(id);
   if (sc.fresh) {
+    drop_positions(sc);
     scenes_.erase(std::find_if(scenes_.begin(), scenes_.end(), [&](Scene const &x) { return x.id == id; }));
     return;
   }
@@ -124,31 +192,47 @@ void Batch::commit() {
   uint32_t slots = used.empty() ? 0u : *used.rbegin() + 1u;
   if (slots > 65536) throw Error("batch: at most 65536 scenes");
   std::sort(keep.begin(), keep.end(), [](Scene const &a, Scene const &b) { return a.slot < b.slot; });
-  // 2. per-slot counts and the remap of each group (new index -> old index)
-  std::vector<uint32_t> fcount(slots, 0), bcount(slots, 0);
-  std::vector<uint32_t> fmap, bmap;
+  // 2. per-slot ranges and the remap of each group (new index -> old index)
+  std::vector<uint32_t> fcount(slots, 0), bcount(slots, 0), fresh;
+  std::vector<SlotRange> frange(slots, SlotRange{0, kNoSrc, nullptr}), brange = frange;
   for (auto &sc : keep) {
     fcount[sc.slot] = uint32_t(sc.nf);
     bcount[sc.slot] = uint32_t(sc.nb);
-    for (size_t k = 0; k < sc.nf; ++k) fmap.push_back(sc.fresh ? kNoSrc : uint32_t(fstart_[sc.slot] + k));
-    for (size_t k = 0; k < sc.nb; ++k) bmap.push_back(sc.fresh ? kNoSrc : uint32_t(bstart_[sc.slot] + k));
-  }
-  auto remap = [&](Group *g, std::vector<uint32_t> const &map) {
-    uint32_t *d = nullptr;
-    if (!map.empty()) {
-      PG_CUDA(cudaMallocAsync(&d, map.size() * 4, s));
-      PG_CUDA(cudaMemcpyAsync(d, map.data(), map.size() * 4, cudaMemcpyHostToDevice, s));
+    if (sc.fresh) {
+      fresh.push_back(sc.slot);
+      frange[sc.slot].x = sc.x;
+      brange[sc.slot].x = sc.x + 3 * sc.nf;
+    } else {
+      frange[sc.slot].old = fstart_[sc.slot];
+      brange[sc.slot].old = bstart_[sc.slot];
     }
-    g->remap(d, map.size(), s);
-    if (d) PG_CUDA(cudaFreeAsync(d, s));
+  }
+  auto remap = [&](Group *g, std::vector<SlotRange> &range, std::vector<uint32_t> const &count, SlotRange *&d) {
+    size_t items = 0;
+    for (uint32_t k = 0; k < slots; ++k) {
+      range[k].first = uint32_t(items);
+      items += count[k];
+    }
+    if (items >= (size_t(1) << 28)) throw Error("group '" + g->name + "' too large: at most 2^28 - 1 items");
+    uint32_t *map = nullptr;
+    if (items) {
+      PG_CUDA(cudaMallocAsync(&d, slots * sizeof(SlotRange), s));
+      // (pageable source: the call returns once the bytes are staged)
+      PG_CUDA(cudaMemcpyAsync(d, range.data(), slots * sizeof(SlotRange), cudaMemcpyHostToDevice, s));
+      PG_CUDA(cudaMallocAsync(&map, items * sizeof(uint32_t), s));
+      k_slot_map<<<div_up(items, 256), 256, 0, s>>>(d, slots, uint32_t(items), map); count_launch();
+      PG_LAUNCH_CHECK();
+    }
+    g->remap(map, items, s);
+    if (map) PG_CUDA(cudaFreeAsync(map, s));
   };
-  remap(f_, fmap);
-  remap(b_, bmap);
+  SlotRange *fd = nullptr, *bd = nullptr;
+  remap(f_, frange, fcount, fd);
+  remap(b_, brange, bcount, bd);
   // 3. segments (slot state of survivors kept; new scenes start from zero)
   Segments &S = *m_.seg;
   S.set_slots(slots, s);
-  for (auto &sc : keep)
-    if (sc.fresh) S.reset_slot(sc.slot, s);
+  S.reset_slots(fresh, s);
   S.assign(b_, bcount, s);
   S.assign(f_, fcount, s);
   std::vector<int> np(std::max<uint32_t>(slots, 1), 0);
@@ -158,26 +242,31 @@ void Batch::commit() {
   nh_.set_segments({S.find(b_)->seg, S.find(f_)->seg}, slots);
   fstart_ = S.find(f_)->start;
   bstart_ = S.find(b_)->start;
-  // 4. upload the new scenes (velocity, acceleration, density, ... are zero)
+  // 4. the new scenes' items (velocity, acceleration, density, ... are zero)
   float h = float(p_.smoothing_scale), rho0 = float(p_.rest_density);
   float mass = float(double(h) * double(h) * double(h) * double(rho0));
   float tb = float(t_) - 1.0f;
   std::vector<uint8_t> due(std::max<uint32_t>(slots, 1), 0);
-  bool any_fresh = false;
-  VaryingField *fx = f_->find_varying("position"), *fm = f_->find_varying("mass");
-  VaryingField *ft = f_->find_varying("time_of_birth"), *bx = b_->find_varying("position");
-  for (auto &sc : keep) {
-    if (!sc.fresh) continue;
-    any_fresh = true;
-    due[sc.slot] = 1;
-    std::vector<float> m(sc.nf, mass), t(sc.nf, tb);
-    upload_varying_range(*fx, fstart_[sc.slot], sc.xf.data(), sc.nf, s);
-    upload_varying_range(*fm, fstart_[sc.slot], m.data(), sc.nf, s);
-    upload_varying_range(*ft, fstart_[sc.slot], t.data(), sc.nf, s);
-    upload_varying_range(*bx, bstart_[sc.slot], sc.xb.data(), sc.nb, s);
-    // the host vectors above must outlive their copies
-    PG_CUDA(cudaStreamSynchronize(s));
-  }
+  bool any_fresh = !fresh.empty();
+  for (uint32_t k : fresh) due[k] = 1;
+  auto fill = [&](Group *g, SlotRange *d, char const *m, char const *t) {
+    if (d && any_fresh) {
+      auto ptr = [&](char const *n) -> float * {
+        if (!n) return nullptr;
+        VaryingField *f = g->find_varying(n);
+        f->version++;
+        return static_cast<float *>(f->d);
+      };
+      k_slot_fill<<<div_up(g->count, 256), 256, 0, s>>>(d, slots, uint32_t(g->count),
+                                                        reinterpret_cast<float4 *>(ptr("position")), ptr(m), ptr(t),
+                                                        mass, tb);
+      count_launch();
+      PG_LAUNCH_CHECK();
+    }
+    if (d) PG_CUDA(cudaFreeAsync(d, s));
+  };
+  fill(f_, fd, "mass", "time_of_birth");
+  fill(b_, bd, nullptr, nullptr);
   scenes_ = std::move(keep);
   removed_.clear();
   slots_ = slots;
@@ -194,10 +283,7 @@ void Batch::commit() {
     if (!sc.fresh) continue;
     sc.fresh = false;
     sc.since_permute = 0;
-    sc.xf.clear();
-    sc.xf.shrink_to_fit();
-    sc.xb.clear();
-    sc.xb.shrink_to_fit();
+    drop_positions(sc);
   }
 }
 

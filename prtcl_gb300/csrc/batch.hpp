@@ -53,14 +53,16 @@ private:
     int64_t steps = 0;
     int since_permute = 0;
     bool fresh = true;            // not yet in the device layout
-    std::vector<float> xf, xb;    // positions until uploaded
+    float *x = nullptr;           // positions on the device until committed: fluid, then boundary
   };
   void commit();
+  void drop_positions(Scene &sc);
   Scene &find(int64_t id);
   void run(Scheme &s, char const *proc);
   void set_global(char const *name, void const *value);
 
   prtcl_gpu_batch_params p_;
+  cudaStream_t up_ = nullptr;     // uploads of new scenes
   Model m_;
   Nhood nh_;
   std::unique_ptr<Scheme> density_, gravity_, euler_, iisph_, wkbb18_, aiast12_;

@@ -167,29 +167,6 @@ void upload_varying(VaryingField &f, size_t count, void const *host, size_t n_it
   if (sync) PG_CUDA(cudaStreamSynchronize(s));
 }
 
-void upload_varying_range(VaryingField &f, size_t offset, void const *host, size_t n, cudaStream_t s) {
-  if (offset + n > f.cap) throw Error("upload: range beyond the field");
-  f.version++;
-  if (n == 0) return;
-  size_t hbytes = n * f.type.host_item_bytes();
-  if (!f.type.is_vec3() && !f.type.is_mat3()) {
-    PG_CUDA(cudaMemcpyAsync(static_cast<char *>(f.d) + offset * f.type.host_item_bytes(), host, hbytes,
-                            cudaMemcpyHostToDevice, s));
-    return;
-  }
-  void *stage = nullptr;
-  PG_CUDA(cudaMallocAsync(&stage, hbytes, s));
-  PG_CUDA(cudaMemcpyAsync(stage, host, hbytes, cudaMemcpyHostToDevice, s));
-  if (f.type.is_vec3())
-    k_expand_vec3<<<div_up(n, 256), 256, 0, s>>>(static_cast<float *>(stage), static_cast<float4 *>(f.d) + offset, n);
-  else
-    k_to_planar9<<<div_up(n, 256), 256, 0, s>>>(static_cast<float *>(stage), static_cast<float *>(f.d) + offset, n,
-                                                 f.cap);
-  count_launch();
-  PG_LAUNCH_CHECK();
-  PG_CUDA(cudaFreeAsync(stage, s));
-}
-
 void download_varying_range(VaryingField const &f, size_t offset, void *host, size_t n, cudaStream_t s) {
   if (offset + n > f.cap) throw Error("download: range beyond the field");
   if (n == 0) return;
@@ -398,15 +375,20 @@ void Segments::set_slots(uint32_t n, cudaStream_t s) {
   slots = n;
 }
 
-// zero the state of one slot (a scene that takes the slot over)
-void Segments::reset_slot(uint32_t k, cudaStream_t s) {
-  if (k >= slots) throw Error("segments: slot out of range");
-  PG_CUDA(cudaMemsetAsync(tickets + k, 0, sizeof(unsigned), s));
-  PG_CUDA(cudaMemsetAsync(scal + size_t(k) * 16, 0, 16 * sizeof(double), s));
-  PG_CUDA(cudaMemsetAsync(stat + size_t(k) * 8, 0, 8 * sizeof(int), s));
-  PG_CUDA(cudaMemsetAsync(stats + size_t(k) * 8, 0, 8 * sizeof(double), s));
-  PG_CUDA(cudaMemsetAsync(iters + k, 0, sizeof(int), s));
-  PG_CUDA(cudaMemsetAsync(due + k, 0, 1, s));
+// zero the state of slots (ascending) that new scenes take over, a run of
+// neighbouring slots at a time
+void Segments::reset_slots(std::vector<uint32_t> const &ks, cudaStream_t s) {
+  for (size_t b = 0, e; b < ks.size(); b = e) {
+    for (e = b + 1; e < ks.size() && ks[e] == ks[e - 1] + 1; ++e) {}
+    size_t k = ks[b], n = e - b;
+    if (k + n > slots) throw Error("segments: slot out of range");
+    PG_CUDA(cudaMemsetAsync(tickets + k, 0, n * sizeof(unsigned), s));
+    PG_CUDA(cudaMemsetAsync(scal + k * 16, 0, n * 16 * sizeof(double), s));
+    PG_CUDA(cudaMemsetAsync(stat + k * 8, 0, n * 8 * sizeof(int), s));
+    PG_CUDA(cudaMemsetAsync(stats + k * 8, 0, n * 8 * sizeof(double), s));
+    PG_CUDA(cudaMemsetAsync(iters + k, 0, n * sizeof(int), s));
+    PG_CUDA(cudaMemsetAsync(due + k, 0, n, s));
+  }
 }
 
 void Segments::assign(Group const *g, std::vector<uint32_t> const &count, cudaStream_t s) {

@@ -128,7 +128,7 @@ struct Segments {
   }
   // set the number of slots (state of remaining slots kept, new ones zeroed)
   void set_slots(uint32_t slots, cudaStream_t s);
-  void reset_slot(uint32_t slot, cudaStream_t s);
+  void reset_slots(std::vector<uint32_t> const &ks, cudaStream_t s);
   // ranges of group g: count[s] items in slot s, consecutively in slot order
   void assign(Group const *g, std::vector<uint32_t> const &count, cudaStream_t s);
 };
@@ -265,9 +265,7 @@ void save_model(Model &m, std::string const &path, cudaStream_t s);
 void load_model(Model &m, std::string const &path, cudaStream_t s);
 // a group as a legacy ASCII VTK file, the reference's SaveVTK format (vtk.cu)
 void save_vtk(Group &g, std::string const &path, cudaStream_t s);
-// items [offset, offset + n) of a field, in the host layout (stream-ordered;
-// the download synchronises)
-void upload_varying_range(VaryingField &f, size_t offset, void const *host, size_t n, cudaStream_t s);
+// items [offset, offset + n) of a field, in the host layout (synchronises)
 void download_varying_range(VaryingField const &f, size_t offset, void *host, size_t n, cudaStream_t s);
 
 } // namespace prtcl_gpu
