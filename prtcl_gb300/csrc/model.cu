@@ -517,6 +517,15 @@ float4 const *Model::packed_xs(Group *g, VaryingField *x, VaryingField *sc, char
   return out;
 }
 
+float4 *Model::current_xs(Group *g, VaryingField *x, VaryingField *sc, char const *kind) {
+  auto it = packs_.find({g, kind});
+  if (it == packs_.end() || !it->second.d || it->second.key != vkey({x, sc}, g->count)) return nullptr;
+  return static_cast<float4 *>(it->second.d);
+}
+void Model::xs_written(Group *g, VaryingField *x, VaryingField *sc, char const *kind) {
+  pack_commit(g, kind, vkey({x, sc}, g->count));
+}
+
 float4 const *Model::packed_xmr(Group *g, VaryingField *x, VaryingField *m, VaryingField *rho, cudaStream_t s) {
   auto key = vkey({x, m, rho}, g->count);
   bool stale = false;

@@ -227,6 +227,11 @@ public:
   //   packed_xmr (x, y, z, m / rho)
   //   packed_pr  p / (rho rho)
   float4 const *packed_xs(Group *g, VaryingField *x, VaryingField *s, char const *kind, cudaStream_t st);
+  // the buffer behind packed_xs where its records are current, for a kernel that
+  // changes x and writes the records with it; xs_written() marks them current
+  // for the field's new version
+  float4 *current_xs(Group *g, VaryingField *x, VaryingField *s, char const *kind);
+  void xs_written(Group *g, VaryingField *x, VaryingField *s, char const *kind);
   float4 const *packed_xmr(Group *g, VaryingField *x, VaryingField *m, VaryingField *rho, cudaStream_t st);
   float const *packed_pr(Group *g, VaryingField *p, VaryingField *rho, cudaStream_t st);
   // the buffer behind packed_pr, for kernels that write p and p / rho^2

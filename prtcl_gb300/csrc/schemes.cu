@@ -497,20 +497,19 @@ __global__ void k_integrate_velocity(uint32_t n, float4 *__restrict__ v, float4 
   v[i] = vi;
 }
 
-// order-preserving map of floats to unsigned integers (for atomicMax)
-__device__ __forceinline__ unsigned f2ord(float f) {
-  unsigned u = __float_as_uint(f);
-  return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord2f(unsigned u) {
-  return __uint_as_float((u & 0x80000000u) ? (u & 0x7FFFFFFFu) : ~u);
-}
-
 // symplectic_euler.integrate_position (schemes/symplectic_euler.hpp:236-270):
 // x += dt v; max_speed = max(max_speed, |v|) over all dynamic particles
+//
+// A speed is never negative, and the bits of non-negative floats, and of a
+// negative or NaN maximum beside them, compare as integers like the floats'
+// maximum: one atomic per warp that raises it, on the global itself.  xm, where
+// given: the packed records (x, m) of the next sweeps.  (The maximum's two
+// conversions and the records each had a launch of their own, 2 to 4 us of a
+// small scene's step of 220.)
 __global__ void k_integrate_position(uint32_t n, float4 *__restrict__ x, float4 const *__restrict__ v, Globals G,
-                                     unsigned *maxord) {
+                                     float4 *__restrict__ xm, float const *__restrict__ m) {
   uint32_t i = grid_tid();
+  int top = *reinterpret_cast<volatile int const *>(G.max_speed);
   float sp = -INFINITY;
   if (i < n) {
     float dt = *G.dt;
@@ -519,13 +518,13 @@ __global__ void k_integrate_position(uint32_t n, float4 *__restrict__ x, float4 
     xi.y = xi.y + dt * vi.y;
     xi.z = xi.z + dt * vi.z;
     x[i] = xi;
+    if (xm) xm[i] = make_float4(xi.x, xi.y, xi.z, m[i]);
     sp = sqrtf(nsq3(mk3(vi)));
   }
   for (int o = 16; o > 0; o >>= 1) sp = fmaxf(sp, __shfl_down_sync(0xffffffffu, sp, o));
-  if ((threadIdx.x & 31) == 0 && sp > -INFINITY) atomicMax(maxord, f2ord(sp));
+  if ((threadIdx.x & 31) == 0 && sp > -INFINITY && __float_as_int(sp) > top)
+    atomicMax(reinterpret_cast<int *>(G.max_speed), __float_as_int(sp));
 }
-__global__ void k_max_speed_begin(Globals G, unsigned *maxord) { *maxord = f2ord(*G.max_speed); }
-__global__ void k_max_speed_end(Globals G, unsigned const *maxord) { *G.max_speed = ord2f(*maxord); }
 
 // ---------------------------------------------------------------------------
 // iisph.setup (schemes/iisph.hpp:188-354)
@@ -615,13 +614,13 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
   AA[i] = aa * ((dt * dt) * (rho0 / ri));
 }
 
-// before and after the set-up sweeps
-__global__ void k_setup_begin(int *status) { status[kStSetupBad] = 0; }
 struct RestDensities {
   float const *p[kMaxNbrGroups];
   int n;
 };
-__global__ void k_setup_end(int *nprde, int total, Globals G, RestDensities D, double *scalars) {
+// before the set-up sweeps
+__global__ void k_setup_begin(int *status, int *nprde, int total, Globals G, RestDensities D, double *scalars) {
+  status[kStSetupBad] = 0;
   *nprde = total;
   scalars[kSSetup] = double(*G.h);
   for (int k = 0; k < D.n; ++k) scalars[kSSetup + 1 + k] = double(*D.p[k]);
@@ -2336,20 +2335,22 @@ public:
     });
     reg("integrate_position", [this](Nhood &, cudaStream_t s) {
       Globals G = globals(*model_);
-      unsigned *maxord = reinterpret_cast<unsigned *>(model_->status_d + 8);
-      k_max_speed_begin<<<1, 1, 0, s>>>(G, maxord); count_launch();
       for (Group *g : dyn_) {
         uint32_t n = uint32_t(g->count);
         if (!n) continue;
-        VaryingField *x = g->find_varying("position");
+        VaryingField *x = g->find_varying("position"), *m = g->find_varying("mass");
+        if (m && m->type != ft_real()) m = nullptr;
+        // the sweeps' records of the group, where they are current
+        float4 *xm = m ? model_->current_xs(g, x, m, "xm") : nullptr;
         ProfScope ps(model_->prof, "integrate_position", s);
         k_integrate_position<<<div_up(n, 256), 256, 0, s>>>(n, dptr<float4>(x),
-                                                            dptr<float4>(g->find_varying("velocity")), G, maxord);
+                                                            dptr<float4>(g->find_varying("velocity")), G, xm,
+                                                            xm ? dptr<float>(m) : nullptr);
         count_launch();
+        PG_LAUNCH_CHECK();
         x->version++;
+        if (xm) model_->xs_written(g, x, m, "xm");
       }
-      k_max_speed_end<<<1, 1, 0, s>>>(G, maxord); count_launch();
-      PG_LAUNCH_CHECK();
     });
   }
   std::string name() const override { return "symplectic_euler"; }
@@ -2578,9 +2579,11 @@ public:
     int nf = int(fluid_.size()), nb = int(bound_.size());
     // one fused sweep per group (pass 2 of a group reads only its own c)
     long long total = 0;
-    k_setup_begin<<<1, 1, 0, s>>>(model_->status_d); count_launch();
+    for (auto *F : active()) total += (long long)F->g->count;
+    // nprde = number of fluid particles (the generated reduction adds 1 per particle)
+    k_setup_begin<<<1, 1, 0, s>>>(model_->status_d, G.nprde, int(total), G, rest_densities(), model_->scalars_d);
+    count_launch();
     for (auto *F : active()) {
-      total += (long long)F->g->count;
       dispatch_fb<SETUP>(nf, nb, this, *F, lists(nh, F->g, G, s), G, s);
       PG_LAUNCH_CHECK();
       F->c->version++;
@@ -2588,8 +2591,6 @@ public:
       F->AA->version++;
       wrote_pressure(*F);
     }
-    // nprde = number of fluid particles (the generated reduction adds 1 per particle)
-    k_setup_end<<<1, 1, 0, s>>>(G.nprde, int(total), G, rest_densities(), model_->scalars_d); count_launch();
     PG_LAUNCH_CHECK();
     if (capturing(s)) zero_key_.clear(); // queued for later, possibly more than once
     else zero_key_ = zero_key(nh, s);
