@@ -333,6 +333,7 @@ private:
   int4 *cell_gi_ = nullptr;
   float4 *xsorted_ = nullptr;
   // the grid and the positions that a counted grid's update left in xsorted_
+  bool rows_zero_ = false; // the list build's words of stats_d_ are zero
   uint64_t xsorted_epoch_ = 0;
   std::vector<uint64_t> xsorted_of_;
   uint32_t *hist_ = nullptr;
