@@ -789,6 +789,9 @@ __global__ void __launch_bounds__(kNT, MINB) k_iisph_pressure(uint32_t n, Pressu
     double acc = start + out[0];
     R.scalars[kSJacobi] = acc;
     if (last_group) *G.aprde = float(acc);
+    // (also where a captured graph runs it unseen by the host: the pressure is
+    // not set-up's any more)
+    if (!done) R.status[kStSetupBad] = 1;
   }
 }
 
