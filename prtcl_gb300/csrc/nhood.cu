@@ -2368,6 +2368,13 @@ void Nhood::need_r2s(cudaStream_t s) {
   r2s_epoch_ = epoch_;
 }
 
+// an epoch names one update of one neighbourhood of the process, so that what is
+// keyed on it cannot match a later neighbourhood at the same address
+static uint64_t next_epoch() {
+  static std::atomic<uint64_t> n{0};
+  return ++n;
+}
+
 // grouped_uniform_grid::update (util/grouped_uniform_grid.hpp:126-337)
 void Nhood::update(cudaStream_t s) {
   if (!model_) throw Error("Neighborhood::Update before Load");
@@ -2389,7 +2396,7 @@ void Nhood::update(cudaStream_t s) {
   if (N >= (size_t(1) << 31)) throw Error("too many items for the grid");
   N_ = N;
   ensure_grid_capacity(N);
-  epoch_++;
+  epoch_ = next_epoch();
   has_grid_ = true;
   counted_ = false;
   if (N == 0) {
