@@ -62,6 +62,7 @@ constexpr int kStJacIter = 4, kStJacDone = 5;
 // 138 us at 1M items; 11 us are left of them): set-up and solve of the 1M dam
 // break 1.54 -> 1.31 ms, of the 27k one 222 -> 204 us.
 constexpr int kStJacFirst = 6, kStSetupBad = 7; // kStSetupBad: 0 after a clean setup, until a solve takes it
+constexpr int kMeetSlot = 32; // tickets[32, 33]: the barriers of k_jacobi_loop
 constexpr int kSSetup = 32; // scalars[32]: smoothing scale, then one rest density per fluid group
 
 // ---------------------------------------------------------------------------
@@ -1008,9 +1009,11 @@ __global__ void k_jacobi_begin(Globals G, Red R, RestDensities D, int same) {
   R.status[kStJacFirst] = jacobi_first(G, D, R.status, R.scalars, same);
   R.status[kStJacIter] = 0;
   R.status[kStJacDone] = (*G.nprde >= 1) ? 0 : 1;
+  R.ticket[kMeetSlot] = 0u;
   *G.jac_iters = 0;
 }
-__global__ void k_jacobi_control(Globals G, Red R, cudaGraphConditionalHandle h, int use_handle, int kernels) {
+// (one thread; returns whether the loop has ended)
+__device__ int jacobi_control(Globals const &G, Red const &R) {
   int done = R.status[kStJacDone];
   if (!done) {
     int it = R.status[kStJacIter] + 1;
@@ -1030,9 +1033,138 @@ __global__ void k_jacobi_control(Globals G, Red R, cudaGraphConditionalHandle h,
       if (rel > R.stats[3]) R.stats[3] = rel;
     }
   }
+  return done;
+}
+__global__ void k_jacobi_control(Globals G, Red R, cudaGraphConditionalHandle h, int use_handle, int kernels) {
+  int done = jacobi_control(G, R);
   // the body's kernels ran (those of a repeat after the end return at once)
   if (kernels) atomicAdd(&g_loop_kernels, (unsigned long long)kernels);
   if (use_handle) cudaGraphSetConditional(h, done ? 0u : 1u);
+}
+
+// The whole relaxed-Jacobi loop of a small scene in one cooperative launch: the
+// blocks are all resident (one item a thread), so they meet at barriers where
+// the graph's loop has two launches, a control's launch and a turn of the loop.  A thread keeps its item's values in
+// registers; the fields that its neighbours read (acceleration, p / rho^2) go
+// through memory, with loads that the barriers order (not the read-only ones).
+// Values, sums and their order are those of the separate sweeps.  Set-up and
+// solve of the 27k dam break 159 -> 144 us, an 8-step run of 2k particles 1.71
+// -> 1.54 ms, of 27k 2.00 -> 1.84.
+//
+// A barrier gives up after kMeetTries polls (about a second): the kernel then
+// returns with -1 iterations noted.
+constexpr unsigned kMeetTries = 1u << 21;
+struct Meet {
+  unsigned *arrived, *turn; // zero between launches (k_jacobi_begin); counts barriers
+};
+// last(): run by the block that arrives last, in all its threads, before the
+// others go on.  False where the barrier gave up.
+template <class F> __device__ bool meet(Meet const &M, F &&last) {
+  __shared__ unsigned s_turn;
+  __shared__ int s_last, s_ok;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    s_turn = *(volatile unsigned *)M.turn; // moves on only after this block has arrived
+    s_last = atomicAdd(M.arrived, 1u) == gridDim.x - 1 ? 1 : 0;
+    s_ok = 1;
+  }
+  __syncthreads();
+  if (s_last) {
+    __threadfence();
+    last();
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      *M.arrived = 0u;
+      __threadfence();
+      atomicAdd(M.turn, 1u);
+    }
+  } else if (threadIdx.x == 0) {
+    unsigned tries = 0;
+    while (*(volatile unsigned *)M.turn == s_turn && ++tries < kMeetTries) __nanosleep(64);
+    if (tries >= kMeetTries) s_ok = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return s_ok != 0;
+}
+
+__global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs A, float4 *a, Globals G, Nbrs<1, 1> N,
+                                                        Red R, Meet M) {
+  constexpr uint32_t kForm = 8 | kAhead;
+  uint32_t i = grid_tid();
+  bool mine = i < n;
+  KernelParams K = kparams(*G.h);
+  bool uc = use_cache(N, K);
+  float rho0 = *A.rho0, dt = *G.dt, omega = *G.omega;
+  FluidN const &F = N.f[0];
+  BoundN const &B = N.b[0];
+  f3 xi = {0.0f, 0.0f, 0.0f};
+  float ri = 1.0f, pi = 0.0f;
+  if (mine) {
+    xi = mk3(A.x[i]);
+    ri = A.rho[i];
+    pi = A.p[i];
+  }
+  bool zero = *(volatile int const *)&R.status[kStJacFirst] != 0;
+  int ended = *(volatile int const *)&R.status[kStJacDone];
+  __shared__ double sh[32];
+  __shared__ int s_ended;
+  while (!ended) {
+    f3 ai = {0.0f, 0.0f, 0.0f};
+    float ap = 0.0f;
+    if (mine && !zero) {
+      float pri = pi / (ri * ri), bterm = (2.0f * pi) / (ri * ri);
+      walk_nbrs_cached<kForm>(F.L, i, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), __ldca(F.pr + j)}; },
+                              [&](WithRec<float> const &r, float gf, bool in, auto cached) {
+        ai = sub_if(in, ai, scl3(r.x.w * (pri + r.v), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
+      });
+      walk_nbrs_cached<kForm>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+                              [&](float4 xv, float gf, bool in, auto cached) {
+        ai = sub_if(in, ai, scl3(((0.7f * rho0) * xv.w) * bterm, pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
+      });
+    }
+    if (mine) a[i] = make_float4(ai.x, ai.y, ai.z, 0.0f);
+    // (with zero sums nobody reads an acceleration)
+    if (!zero && !meet(M, [] {})) break;
+    double part = 0.0;
+    if (mine) {
+      if (!zero) {
+        walk_nbrs_cached<kForm>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldca(F.a + j))}; },
+                                [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
+          ap = add_if(in, ap, r.x.w * dot3(sub3(ai, r.v), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
+        });
+        walk_nbrs_cached<kForm>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+                                [&](float4 xv, float gf, bool in, auto cached) {
+          ap = add_if(in, ap, (rho0 * xv.w) * dot3(sub3(ai, f3{0.0f, 0.0f, 0.0f}),
+                                                   pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
+        });
+      }
+      part += pressure_finish(i, A, ap, rho0, dt, omega);
+      pi = A.p[i];
+    }
+    // the density error, as reduce_commit sums it, and the loop's control
+    double sum = block_sum(part, sh);
+    if (threadIdx.x == 0) R.partials[blockIdx.x] = sum;
+    bool ok = meet(M, [&] {
+      double acc = 0.0;
+      for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += __ldcg(&R.partials[b]);
+      acc = block_sum(acc, sh);
+      if (threadIdx.x == 0) {
+        acc = 0.0 + acc;
+        R.scalars[kSJacobi] = acc;
+        *G.aprde = float(acc);
+        jacobi_control(G, R);
+      }
+    });
+    if (!ok) break;
+    if (threadIdx.x == 0) s_ended = *(volatile int const *)&R.status[kStJacDone];
+    __syncthreads();
+    ended = s_ended;
+    zero = false;
+  }
+  if (!ended && threadIdx.x == 0) *G.jac_iters = -1; // a barrier gave up
 }
 
 // ---------------------------------------------------------------------------
@@ -2727,7 +2859,9 @@ public:
         count_launch();
       }
     };
-    if (model_->prof.enabled) {
+    if (!seg && !staged && act.size() == 1 && !model_->prof.enabled && loop_in_one_launch(*act[0], nf, nb, s)) {
+      jacobi_loop(*act[0], *views[0], G, R, s);
+    } else if (model_->prof.enabled) {
       // host-driven: one iteration per round trip
       for (int it = 0; it < 100000; ++it) {
         body(s, cudaGraphConditionalHandle{}, false, true, nullptr);
@@ -2754,8 +2888,38 @@ public:
   }
 
 private:
+  // one cooperative launch takes the loop of a small scene of the tuned layout:
+  // the sweeps' knobs at their defaults, every block resident
+  bool loop_in_one_launch(FluidG const &F, int nf, int nb, cudaStream_t s) {
+    auto const &t = model_->tune.v;
+    if (nf != 1 || nb != 1 || t[kTuneAccel] || t[kTunePressure] || t[kTuneJacobiUnroll] != 1) return false;
+    if (F.g->count == 0 || F.g->count > kSmallItems || capturing(s)) return false;
+    if (resident_ < 0) {
+      int dev = 0, sms = 0, coop = 0, per = 0;
+      PG_CUDA(cudaGetDevice(&dev));
+      PG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      PG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+      PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_jacobi_loop, kNT, 0));
+      resident_ = coop ? sms * per : 0;
+    }
+    return div_up(F.g->count, kNT) <= unsigned(resident_);
+  }
+  void jacobi_loop(FluidG &F, NbrView const &v, Globals G, Red R, cudaStream_t s) {
+    uint32_t n = uint32_t(F.g->count);
+    auto N = nbrs<1, 1>(v, s);
+    N.f[0].pr = model_->packed_pr(F.g, F.p, F.rho, s);
+    PressureArgs PA{dptr<float4>(F.x), dptr<float4>(F.a), dptr<float>(F.rho), dptr<float>(F.s), dptr<float>(F.AA),
+                    dptr<float>(F.p), model_->pr_buffer(F.g, s), dptr<float>(F.Ap), u(F.rho0)};
+    float4 *a = dptr<float4>(F.a);
+    Meet M{R.ticket + kMeetSlot, R.ticket + kMeetSlot + 1};
+    void *args[] = {&n, &PA, &a, &G, &N, &R, &M};
+    PG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const *>(k_jacobi_loop), dim3(div_up(n, kNT)), dim3(kNT),
+                                        args, 0, s));
+    count_launch();
+  }
   WhileLoop loop_;
   std::vector<uint64_t> zero_key_;
+  int resident_ = -1; // blocks of k_jacobi_loop that fit the device
 };
 
 // ---------------------------------------------------------------------------
