@@ -1380,7 +1380,8 @@ struct PcgArgs {
 
 // system product of wkbb18.accumulate_acceleration (schemes/wkbb18.hpp:
 // 339-396): (A w)_i = w_i - dt * a_f(w)_i
-template <int NB, bool GC, int BT = 8 | kAlone>
+// LOOP: w changes during the launch (its loads are ordered by the barriers)
+template <int NB, bool GC, int BT = 8 | kAlone, bool LOOP = false>
 __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const &K, bool uc, float dt, float rho0,
                                             float mu, Nbrs<0, NB> const &N, float4 const *__restrict__ w, uint32_t i) {
   float Li[9];
@@ -1398,7 +1399,7 @@ __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const
   do {
     af = {0.0f, 0.0f, 0.0f};
     off = false;
-    walk_nbrs_cached<BT>(P.self, i, flat, [&](uint32_t j) { return WithRec<f3>{__ldg(P.xmr + j), mk3(__ldg(w + j))}; },
+    walk_nbrs_cached<BT>(P.self, i, flat, [&](uint32_t j) { return WithRec<f3>{__ldg(P.xmr + j), mk3(LOOP ? __ldca(w + j) : __ldg(w + j))}; },
                          [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
       constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
       f3 xij = sub3(xi, mk3(r.x));
@@ -1431,8 +1432,9 @@ __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const
 
 // scalars: 0 b_nsq, 1 thr, 2 r_nsq, 3 next_rdy, 4 prev_rdy, 5 pdq,
 // 6 alpha, 7 beta (f32 values held in double slots)
-__global__ void k_pcg_guess(PcgArgs P) {
+__global__ void k_pcg_guess(PcgArgs P, unsigned *arrived) {
   uint32_t i = grid_tid();
+  if (i == 0) *arrived = 0u; // k_pcg_loop's barriers
   if (i < P.n) P.X[i] = P.v[i];
 }
 
@@ -1467,10 +1469,10 @@ __device__ __forceinline__ void pcg_init_finish(PcgArgs const &P, uint32_t i, f3
   rr += f2d(dot3(r, r));
   ry += f2d(dot3(r, y));
 }
-template <int NB, bool GC, int BT = 8 | kAlone>
+template <int NB, bool GC, int BT = 8 | kAlone, bool LOOP = false>
 __device__ __forceinline__ double pcg_q_item(PcgArgs const &P, KernelParams const &K, bool uc, float dt, float rho0,
                                              float mu, Nbrs<0, NB> const &N, uint32_t i) {
-  return pcg_q_finish(P, i, wkbb18_system<NB, GC, BT>(P, K, uc, dt, rho0, mu, N, P.P, i));
+  return pcg_q_finish(P, i, wkbb18_system<NB, GC, BT, LOOP>(P, K, uc, dt, rho0, mu, N, P.P, i));
 }
 __device__ __forceinline__ void pcg_update_item(PcgArgs const &P, float alpha, uint32_t i, double &rr, double &ry) {
   f3 x = mk3(P.X[i]), p = mk3(P.P[i]), r = mk3(P.Rr[i]), q = mk3(P.Q[i]);
@@ -1876,10 +1878,10 @@ __global__ void k_pcg_p(PcgArgs P, Red R) {
 
 // loop control of the device PCG loop: continue while active, and never run
 // more than max_k + 1 bodies
-__global__ void k_pcg_control(PcgArgs P, Red R, cudaGraphConditionalHandle h, int use_handle, int kernels) {
+// (one thread; returns whether the loop goes on)
+__device__ bool pcg_control(PcgArgs const &P, Red const &R) {
   int body = R.status[kStPcgBody] + 1;
   R.status[kStPcgBody] = body;
-  if (kernels) atomicAdd(&g_loop_kernels, (unsigned long long)kernels);
   int maxk = *P.max_k;
   bool cont = R.status[kStPcgActive] && body < (maxk < 0 ? 0 : maxk) + 1 && body < 1000000;
   if (!cont) {
@@ -1888,7 +1890,65 @@ __global__ void k_pcg_control(PcgArgs P, Red R, cudaGraphConditionalHandle h, in
     if (R.status[kStPcgActive]) R.stats[6] += 1.0;
     R.status[kStPcgActive] = 0;
   }
+  return cont;
+}
+__global__ void k_pcg_control(PcgArgs P, Red R, cudaGraphConditionalHandle h, int use_handle, int kernels) {
+  bool cont = pcg_control(P, R);
+  if (kernels) atomicAdd(&g_loop_kernels, (unsigned long long)kernels);
   if (use_handle) cudaGraphSetConditional(h, cont ? 1u : 0u);
+}
+
+// The PCG loop of a small scene in one cooperative launch, as k_jacobi_loop is
+// of the Jacobi loop: three barriers where the graph's loop has four launches
+// and a turn.  Diagonal and solve 89 -> 77 us at 2k items, 124 -> 110 at 27k, 146
+// -> 136 at 60k (with gradient correction 239 -> 230).
+template <bool GC>
+__global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<0, 1> N, Red R, Meet M) {
+  uint32_t i = grid_tid();
+  bool mine = i < P.n;
+  KernelParams K = kparams(*G.h);
+  bool uc = use_cache(N, K);
+  float dt = *G.dt, rho0 = *P.rho0, mu = *P.mu;
+  double volatile const *sc = R.scalars + kSPcg;
+  int volatile const *active = &R.status[kStPcgActive];
+  __shared__ double sh[32];
+  // the sums of the block that arrives last, as reduce_commit forms them
+  auto total = [&](int k) {
+    double acc = 0.0;
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += __ldcg(&R.partials[k * kMaxRedBlocks + b]);
+    return block_sum(acc, sh);
+  };
+  auto partial = [&](int k, double v) {
+    double t = block_sum(v, sh);
+    if (threadIdx.x == 0) R.partials[k * kMaxRedBlocks + blockIdx.x] = t;
+  };
+  bool ok = true;
+  while (ok && *active) {
+    partial(0, mine ? 0.0 + pcg_q_item<1, GC, 8 | kAhead, true>(P, K, uc, dt, rho0, mu, N, i) : 0.0);
+    ok = meet(M, [&] {
+      double pq = total(0);
+      if (threadIdx.x == 0) {
+        pcg_q_scalars(R.scalars + kSPcg, R.status, pq, *P.tol);
+        if (!R.status[kStPcgActive]) pcg_control(P, R);
+      }
+    });
+    if (!ok || !*active) break;
+    double rr = 0.0, ry = 0.0;
+    if (mine) pcg_update_item(P, float(sc[6]), i, rr, ry);
+    partial(0, rr);
+    partial(1, ry);
+    ok = meet(M, [&] {
+      double t0 = total(0), t1 = total(1);
+      if (threadIdx.x == 0) {
+        pcg_update_scalars(R.scalars + kSPcg, R.status, t0, t1, *P.tol, *P.max_k);
+        pcg_control(P, R);
+      }
+    });
+    if (!ok || !*active) break;
+    if (mine) pcg_p_item(P, float(sc[7]), i);
+    ok = meet(M, [] {});
+  }
+  if (!ok && threadIdx.x == 0) R.status[kStPcgIter] = -1; // a barrier gave up
 }
 
 // --- the PCG loop over the tiles of a batched model, per slot -------------
@@ -2300,6 +2360,24 @@ protected:
     PG_CUDA(cudaFuncSetAttribute(k_pcg_init_staged<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStageSmem)));
     PG_CUDA(cudaFuncSetAttribute(k_pcg_q_staged<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStageSmem)));
     return true;
+  }
+  static bool capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+    PG_CUDA(cudaStreamIsCapturing(s, &c));
+    return c != cudaStreamCaptureStatusNone;
+  }
+  // blocks of a cooperative kernel of kNT threads that the device holds at once
+  // (asked for once per scheme: `known` starts at -1)
+  template <class Kernel> static int resident_blocks(Kernel *kernel, int &known) {
+    if (known < 0) {
+      int dev = 0, sms = 0, coop = 0, per = 0;
+      PG_CUDA(cudaGetDevice(&dev));
+      PG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+      PG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+      PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kernel, kNT, 0));
+      known = coop ? sms * per : 0;
+    }
+    return known;
   }
   float const *u(SmallField *f) { return static_cast<float const *>(model_->small_ptr(*f)); }
   void need(std::initializer_list<std::pair<void const *, char const *>> l) {
@@ -2730,11 +2808,6 @@ public:
     if (capturing(s)) zero_key_.clear(); // queued for later, possibly more than once
     else zero_key_ = zero_key(nh, s);
   }
-  static bool capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-    PG_CUDA(cudaStreamIsCapturing(s, &c));
-    return c != cudaStreamCaptureStatusNone;
-  }
   RestDensities rest_densities() {
     RestDensities D{};
     for (auto &F : fluid_)
@@ -2894,15 +2967,7 @@ private:
     auto const &t = model_->tune.v;
     if (nf != 1 || nb != 1 || t[kTuneAccel] || t[kTunePressure] || t[kTuneJacobiUnroll] != 1) return false;
     if (F.g->count == 0 || F.g->count > kSmallItems || capturing(s)) return false;
-    if (resident_ < 0) {
-      int dev = 0, sms = 0, coop = 0, per = 0;
-      PG_CUDA(cudaGetDevice(&dev));
-      PG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-      PG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-      PG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_jacobi_loop, kNT, 0));
-      resident_ = coop ? sms * per : 0;
-    }
-    return div_up(F.g->count, kNT) <= unsigned(resident_);
+    return div_up(F.g->count, kNT) <= unsigned(resident_blocks(k_jacobi_loop, resident_));
   }
   void jacobi_loop(FluidG &F, NbrView const &v, Globals G, Red R, cudaStream_t s) {
     uint32_t n = uint32_t(F.g->count);
@@ -3045,7 +3110,8 @@ public:
     bool seg = segmented(F.g);
     SegArgs SA = seg ? seg_args(F.g) : SegArgs{};
     unsigned tg = SA.ntiles;
-    k_pcg_guess<<<eg, 256, 0, s>>>(P); count_launch();
+    Meet M{model_->red_count_d + kMeetSlot, model_->red_count_d + kMeetSlot + 1};
+    k_pcg_guess<<<eg, 256, 0, s>>>(P, M.arrived); count_launch();
     constexpr bool kTuned = NB == 1 && !GC;
     int tv_init = fluid_.size() == 1 ? model_->tune.v[kTunePcgInit] : 0;
     int tv_q = fluid_.size() == 1 ? model_->tune.v[kTunePcgQ] : 0;
@@ -3137,7 +3203,18 @@ public:
         k_pcg_control<<<1, 1, 0, cs>>>(P, R, h, use_handle ? 1 : 0, use_handle ? 4 : 0);
       count_launch();
     };
-    if (model_->prof.enabled) {
+    bool one_launch = false;
+    if constexpr (NB == 1)
+      one_launch = !seg && !staged && !tiles && fluid_.size() == 1 && !tv_q && !model_->prof.enabled &&
+                   n <= kSmallItems && !capturing(s) && rg <= unsigned(resident_blocks(k_pcg_loop<GC>, resident_));
+    if (one_launch) {
+      if constexpr (NB == 1) {
+        void *args[] = {&P, &G, &N, &R, &M};
+        PG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const *>(k_pcg_loop<GC>), dim3(rg), dim3(kNT), args, 0,
+                                            s));
+        count_launch();
+      }
+    } else if (model_->prof.enabled) {
       // host-driven (timed launches): one iteration per round trip
       for (int it = 0; it < 1000000; ++it) {
         body(s, cudaGraphConditionalHandle{}, false, true);
@@ -3193,6 +3270,7 @@ private:
   float4 *vec_[5] = {};
   size_t vec_cap_ = 0;
   std::map<Group *, WhileLoop> loops_;
+  int resident_ = -1; // blocks of k_pcg_loop that fit the device
   void free_vectors() {
     for (auto &p : vec_)
       if (p) {
