@@ -57,7 +57,7 @@ constexpr int kStJacIter = 4, kStJacDone = 5;
 // neighbour, so its own mass and density count too).  Setup notes what it
 // found (kStSetupBad, and in scalars[kSSetup..] the smoothing scale and rest
 // densities it used), the host checks that no field, list or pressure has
-// changed since, and k_jacobi_begin sets kStJacFirst where both agree.  Of
+// changed since, and k_jacobi_begin (k_jacobi_loop) takes them where both agree.  Of
 // the 4 to 5 iterations a step takes, this takes out one pair of sweeps (95 +
 // 138 us at 1M items; 11 us are left of them): set-up and solve of the 1M dam
 // break 1.54 -> 1.31 ms, of the 27k one 222 -> 204 us.
@@ -620,7 +620,9 @@ struct RestDensities {
   int n;
 };
 // before the set-up sweeps
-__global__ void k_setup_begin(int *status, int *nprde, int total, Globals G, RestDensities D, double *scalars) {
+__global__ void k_setup_begin(int *status, int *nprde, int total, Globals G, RestDensities D, double *scalars,
+                              unsigned *arrived) {
+  *arrived = 0u; // k_jacobi_loop's barriers
   status[kStSetupBad] = 0;
   *nprde = total;
   scalars[kSSetup] = double(*G.h);
@@ -628,10 +630,15 @@ __global__ void k_setup_begin(int *status, int *nprde, int total, Globals G, Res
 }
 // whether the loop's first iteration may take zero sums (see kStJacFirst):
 // `same` is the host's part
-__device__ __forceinline__ int jacobi_first(Globals const &G, RestDensities const &D, int *status,
-                                            double const *scalars, int same) {
+__device__ __forceinline__ bool zero_sums_hold(Globals const &G, RestDensities const &D, int const *status,
+                                               double const *scalars, int same) {
   bool ok = same && !status[kStSetupBad] && scalars[kSSetup] == double(*G.h);
   for (int k = 0; k < D.n; ++k) ok = ok && scalars[kSSetup + 1 + k] == double(*D.p[k]) && isfinite(*D.p[k]);
+  return ok;
+}
+__device__ __forceinline__ int jacobi_first(Globals const &G, RestDensities const &D, int *status,
+                                            double const *scalars, int same) {
+  bool ok = zero_sums_hold(G, D, status, scalars, same);
   status[kStSetupBad] = 1; // the solve changes the pressure
   return ok ? 1 : 0;
 }
@@ -1009,7 +1016,6 @@ __global__ void k_jacobi_begin(Globals G, Red R, RestDensities D, int same) {
   R.status[kStJacFirst] = jacobi_first(G, D, R.status, R.scalars, same);
   R.status[kStJacIter] = 0;
   R.status[kStJacDone] = (*G.nprde >= 1) ? 0 : 1;
-  R.ticket[kMeetSlot] = 0u;
   *G.jac_iters = 0;
 }
 // (one thread; returns whether the loop has ended)
@@ -1055,7 +1061,7 @@ __global__ void k_jacobi_control(Globals G, Red R, cudaGraphConditionalHandle h,
 // returns with -1 iterations noted.
 constexpr unsigned kMeetTries = 1u << 21;
 struct Meet {
-  unsigned *arrived, *turn; // zero between launches (k_jacobi_begin); counts barriers
+  unsigned *arrived, *turn; // zero between launches (k_setup_begin, k_pcg_guess); counts barriers
 };
 // last(): run by the block that arrives last, in all its threads, before the
 // others go on.  False where the barrier gave up.
@@ -1091,7 +1097,8 @@ template <class F> __device__ bool meet(Meet const &M, F &&last) {
 }
 
 __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs A, float4 *a, Globals G, Nbrs<1, 1> N,
-                                                        Red R, Meet M) {
+                                                        Red R, Meet M, const __grid_constant__ RestDensities D,
+                                                        int same) {
   constexpr uint32_t kForm = 8 | kAhead;
   uint32_t i = grid_tid();
   bool mine = i < n;
@@ -1107,8 +1114,17 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
     ri = A.rho[i];
     pi = A.p[i];
   }
-  bool zero = *(volatile int const *)&R.status[kStJacFirst] != 0;
-  int ended = *(volatile int const *)&R.status[kStJacDone];
+  // what k_jacobi_begin does, by every block for itself; the flags are written
+  // once every block has read them
+  bool zero = zero_sums_hold(G, D, R.status, R.scalars, same);
+  int ended = *G.nprde >= 1 ? 0 : 1;
+  if (ended && i == 0) {
+    R.status[kStSetupBad] = 1;
+    R.status[kStJacIter] = 0;
+    R.status[kStJacDone] = 1;
+    *G.jac_iters = 0;
+  }
+  bool begun = false;
   __shared__ double sh[32];
   __shared__ int s_ended;
   while (!ended) {
@@ -1155,9 +1171,15 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
         acc = 0.0 + acc;
         R.scalars[kSJacobi] = acc;
         *G.aprde = float(acc);
+        if (!begun) {
+          R.status[kStSetupBad] = 1;
+          R.status[kStJacIter] = 0;
+          R.status[kStJacDone] = 0;
+        }
         jacobi_control(G, R);
       }
     });
+    begun = true;
     if (!ok) break;
     if (threadIdx.x == 0) s_ended = *(volatile int const *)&R.status[kStJacDone];
     __syncthreads();
@@ -2379,6 +2401,20 @@ protected:
     }
     return known;
   }
+  // a cooperative launch; false, and no further ones, where the context at hand
+  // holds fewer blocks than the device
+  template <class Kernel>
+  static bool launch_resident(Kernel *kernel, unsigned blocks, void **args, cudaStream_t s, int &known) {
+    cudaError_t e = cudaLaunchCooperativeKernel(reinterpret_cast<void const *>(kernel), dim3(blocks), dim3(kNT), args, 0, s);
+    if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+      cudaGetLastError();
+      known = 0;
+      return false;
+    }
+    PG_CUDA(e);
+    count_launch();
+    return true;
+  }
   float const *u(SmallField *f) { return static_cast<float const *>(model_->small_ptr(*f)); }
   void need(std::initializer_list<std::pair<void const *, char const *>> l) {
     for (auto &p : l)
@@ -2794,7 +2830,8 @@ public:
     long long total = 0;
     for (auto *F : active()) total += (long long)F->g->count;
     // nprde = number of fluid particles (the generated reduction adds 1 per particle)
-    k_setup_begin<<<1, 1, 0, s>>>(model_->status_d, G.nprde, int(total), G, rest_densities(), model_->scalars_d);
+    k_setup_begin<<<1, 1, 0, s>>>(model_->status_d, G.nprde, int(total), G, rest_densities(), model_->scalars_d,
+                                  model_->red_count_d + kMeetSlot);
     count_launch();
     for (auto *F : active()) {
       dispatch_fb<SETUP>(nf, nb, this, *F, lists(nh, F->g, G, s), G, s);
@@ -2901,7 +2938,10 @@ public:
     // (the staged sweeps take every iteration in full)
     int same = !staged && !zero_key_.empty() && !capturing(s) && zero_key_ == zero_key(nh, s) ? 1 : 0;
     zero_key_.clear();
-    if (seg) {
+    bool one_launch = !seg && !staged && act.size() == 1 && !model_->prof.enabled &&
+                      loop_in_one_launch(*act[0], nf, nb, s) && jacobi_loop(*act[0], *views[0], G, R, same, s);
+    if (one_launch) {
+    } else if (seg) {
       k_seg_jacobi_begin<<<div_up(std::max<uint32_t>(SA.slots, 1), 256), 256, 0, s>>>(SA, G, R, rest_densities(), same);
       count_launch();
       k_seg_active<<<1, 1024, 0, s>>>(SA); count_launch();
@@ -2932,8 +2972,7 @@ public:
         count_launch();
       }
     };
-    if (!seg && !staged && act.size() == 1 && !model_->prof.enabled && loop_in_one_launch(*act[0], nf, nb, s)) {
-      jacobi_loop(*act[0], *views[0], G, R, s);
+    if (one_launch) {
     } else if (model_->prof.enabled) {
       // host-driven: one iteration per round trip
       for (int it = 0; it < 100000; ++it) {
@@ -2961,15 +3000,16 @@ public:
   }
 
 private:
-  // one cooperative launch takes the loop of a small scene of the tuned layout:
-  // the sweeps' knobs at their defaults, every block resident
+  // one cooperative launch takes the loop of a small scene of the tuned layout
+  // where every block is resident, whatever the sweeps' shapes (which the tuner
+  // times in launches of their own) unless iterations are repeated in a graph
   bool loop_in_one_launch(FluidG const &F, int nf, int nb, cudaStream_t s) {
     auto const &t = model_->tune.v;
-    if (nf != 1 || nb != 1 || t[kTuneAccel] || t[kTunePressure] || t[kTuneJacobiUnroll] != 1) return false;
+    if (nf != 1 || nb != 1 || t[kTuneJacobiUnroll] != 1) return false;
     if (F.g->count == 0 || F.g->count > kSmallItems || capturing(s)) return false;
     return div_up(F.g->count, kNT) <= unsigned(resident_blocks(k_jacobi_loop, resident_));
   }
-  void jacobi_loop(FluidG &F, NbrView const &v, Globals G, Red R, cudaStream_t s) {
+  bool jacobi_loop(FluidG &F, NbrView const &v, Globals G, Red R, int same, cudaStream_t s) {
     uint32_t n = uint32_t(F.g->count);
     auto N = nbrs<1, 1>(v, s);
     N.f[0].pr = model_->packed_pr(F.g, F.p, F.rho, s);
@@ -2977,10 +3017,9 @@ private:
                     dptr<float>(F.p), model_->pr_buffer(F.g, s), dptr<float>(F.Ap), u(F.rho0)};
     float4 *a = dptr<float4>(F.a);
     Meet M{R.ticket + kMeetSlot, R.ticket + kMeetSlot + 1};
-    void *args[] = {&n, &PA, &a, &G, &N, &R, &M};
-    PG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const *>(k_jacobi_loop), dim3(div_up(n, kNT)), dim3(kNT),
-                                        args, 0, s));
-    count_launch();
+    RestDensities D = rest_densities();
+    void *args[] = {&n, &PA, &a, &G, &N, &R, &M, &D, &same};
+    return launch_resident(k_jacobi_loop, div_up(n, kNT), args, s, resident_);
   }
   WhileLoop loop_;
   std::vector<uint64_t> zero_key_;
@@ -3204,16 +3243,13 @@ public:
       count_launch();
     };
     bool one_launch = false;
-    if constexpr (NB == 1)
-      one_launch = !seg && !staged && !tiles && fluid_.size() == 1 && !tv_q && !model_->prof.enabled &&
-                   n <= kSmallItems && !capturing(s) && rg <= unsigned(resident_blocks(k_pcg_loop<GC>, resident_));
+    if constexpr (NB == 1) {
+      void *args[] = {&P, &G, &N, &R, &M};
+      one_launch = !seg && !staged && !tiles && fluid_.size() == 1 && !model_->prof.enabled && n <= kSmallItems &&
+                   !capturing(s) && rg <= unsigned(resident_blocks(k_pcg_loop<GC>, resident_)) &&
+                   launch_resident(k_pcg_loop<GC>, rg, args, s, resident_);
+    }
     if (one_launch) {
-      if constexpr (NB == 1) {
-        void *args[] = {&P, &G, &N, &R, &M};
-        PG_CUDA(cudaLaunchCooperativeKernel(reinterpret_cast<void const *>(k_pcg_loop<GC>), dim3(rg), dim3(kNT), args, 0,
-                                            s));
-        count_launch();
-      }
     } else if (model_->prof.enabled) {
       // host-driven (timed launches): one iteration per round trip
       for (int it = 0; it < 1000000; ++it) {

@@ -1,6 +1,6 @@
 """The PCG loop of a small scene as one cooperative launch gives the velocity
 change, the acceleration and the iteration count of the launches one by one
-(another shape of the product), with and without gradient correction, at item
+(driven from the host, as with profiling on), with and without gradient correction, at item
 counts around a block and at the largest it takes, up to the iteration cap."""
 import numpy as np
 import pytest
@@ -26,10 +26,11 @@ def scene(n, **params):
     return d
 
 
-def solve(d, scheme, knob):
-    d.model.tune_set("pcg_q", knob)
+def solve(d, scheme, singly):
     d.run(scheme, "compute_diagonal")
+    d.model.profile(singly)
     d.run(scheme, "accumulate_acceleration")
+    d.model.profile(False)
     return ([d.get_varying("f", "wkbb18_velocity_delta", 3), d.get_varying("f", "acceleration", 3)],
             d.get_uniform("f", "wkbb18_iterations"))
 
@@ -40,7 +41,7 @@ def check(d, gc, iterations=None):
         d.scheme("wkbb18_gc")
         d.run("correction", "compute_gradient_correction")
     scheme = "wkbb18_gc" if gc else "wkbb18"
-    a, b = solve(d, scheme, 0), solve(d, scheme, 1)
+    a, b = solve(d, scheme, False), solve(d, scheme, True)
     for x, y in zip(a[0], b[0]):
         assert_bitwise(x, y)
     assert a[1] == b[1] >= 0
