@@ -130,22 +130,21 @@ int64_t Batch::add(float const *xf, size_t nf, float const *xb, size_t nb) {
   sc.id = next_id_++;
   sc.nf = nf;
   sc.nb = nb;
+  scenes_.push_back(std::move(sc));
   // straight to the device, where they wait for the next commit; on a stream
   // of its own, so that the call does not wait for steps that are under way
+  float *&x = scenes_.back().x;
   size_t nx = 3 * nf, nbx = 3 * nb;
-  if (nx + nbx) {
-    PG_CUDA(cudaMallocAsync(&sc.x, (nx + nbx) * sizeof(float), up_));
-    try {
-      if (nx) PG_CUDA(cudaMemcpyAsync(sc.x, xf, nx * sizeof(float), cudaMemcpyHostToDevice, up_));
-      if (nbx) PG_CUDA(cudaMemcpyAsync(sc.x + nx, xb, nbx * sizeof(float), cudaMemcpyHostToDevice, up_));
-      PG_CUDA(cudaStreamSynchronize(up_));
-      scenes_.reserve(scenes_.size() + 1);
-    } catch (...) {
-      cudaFreeAsync(sc.x, up_);
-      throw;
-    }
+  try {
+    if (nx + nbx) PG_CUDA(cudaMallocAsync(&x, (nx + nbx) * sizeof(float), up_));
+    if (nx) PG_CUDA(cudaMemcpyAsync(x, xf, nx * sizeof(float), cudaMemcpyHostToDevice, up_));
+    if (nbx) PG_CUDA(cudaMemcpyAsync(x + nx, xb, nbx * sizeof(float), cudaMemcpyHostToDevice, up_));
+    if (nx + nbx) PG_CUDA(cudaStreamSynchronize(up_));
+  } catch (...) {
+    if (x) cudaFreeAsync(x, up_);
+    scenes_.pop_back();
+    throw;
   }
-  scenes_.push_back(std::move(sc));
   dirty_ = true;
   return scenes_.back().id;
 }
