@@ -170,7 +170,8 @@ int prtcl_gpu_profile_reset(prtcl_gpu_model *model);
  * iisph_pressure, wkbb18_diag, pcg_init, pcg_q (values 0..3, a launch
  * shape each; pcg_q 4: a cell-tile sweep without neighbour lists, for
  * unbatched models), jacobi_unroll (1, 2 or 4 relaxed-Jacobi iterations per
- * iteration of the device loop's graph), staging (1: unbatched models with
+ * iteration of the device loop's graph; at 1 the loop of a scene of at most
+ * 77,824 items is one cooperative launch instead), staging (1: unbatched models with
  * one fluid and one boundary group build staged lists, and the
  * relaxed-Jacobi and PCG sweeps read their neighbours' records from shared
  * memory per tile of 128 items), grid_sort (1, the default: a grid whose cell

@@ -8,7 +8,8 @@ the tuner is free to pick the fastest per workload:
   wkbb18_diag, pcg_init, pcg_q) select a launch shape: threads per block,
   blocks resident per SM (the register cap) and neighbour-walk batch;
 * jacobi_unroll is the number of relaxed-Jacobi iterations per iteration of
-  the device loop's graph (1, 2 or 4);
+  the device loop's graph (1, 2 or 4; at 1 the loop of a small scene is one
+  cooperative launch instead);
 * staging (single-scene models) builds staged neighbour lists and runs the
   staged relaxed-Jacobi and PCG sweeps, which read their neighbours'
   records from shared memory (0 or 1);
