@@ -2273,10 +2273,13 @@ static bool same_dir(DirKey const &a, DirKey const &b) {
 }
 
 void Nhood::settle(cudaStream_t s) {
-  if (!key_check_) return;
-  PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, kStRows * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-  PG_CUDA(cudaStreamSynchronize(s));
-  if (!confirmed()) update(s);
+  // (an update that replaces one of another layout is counted, so its fullest
+  // cell is still to be confirmed; the sort that replaces that one is final)
+  while (key_check_) {
+    PG_CUDA(cudaMemcpyAsync(stats_h_, stats_d_, kStRows * sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    PG_CUDA(cudaStreamSynchronize(s));
+    if (!confirmed()) update(s);
+  }
 }
 
 // Whether a grid of N items is built by counting, with the tables allocated:
