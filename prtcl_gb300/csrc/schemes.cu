@@ -1071,15 +1071,19 @@ constexpr unsigned kMeetTries = 1u << 21;
 struct Meet {
   unsigned *arrived, *turn; // zero between launches (k_setup_begin, k_pcg_guess); counts barriers
 };
+// The turn to wait for, read where the launch begins: it moves on only after
+// this block's first arrival, which a fence follows the read before.  Later ones
+// are counted.  (Read beside each arrival, with nothing between the two, the
+// load could take effect after the arrival and find the next turn: the block
+// would wait for one that does not come.)
+__device__ __forceinline__ unsigned meet_turn(Meet const &M) { return *(volatile unsigned *)M.turn; }
 // last(): run by the block that arrives last, in all its threads, before the
 // others go on.  False where the barrier gave up.
-template <class F> __device__ bool meet(Meet const &M, F &&last) {
-  __shared__ unsigned s_turn;
+template <class F> __device__ bool meet(Meet const &M, unsigned &turn, F &&last) {
   __shared__ int s_last, s_ok;
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    s_turn = *(volatile unsigned *)M.turn; // moves on only after this block has arrived
     s_last = atomicAdd(M.arrived, 1u) == gridDim.x - 1 ? 1 : 0;
     s_ok = 1;
   }
@@ -1096,10 +1100,11 @@ template <class F> __device__ bool meet(Meet const &M, F &&last) {
     }
   } else if (threadIdx.x == 0) {
     unsigned tries = 0;
-    while (*(volatile unsigned *)M.turn == s_turn && ++tries < kMeetTries) __nanosleep(64);
+    while (*(volatile unsigned *)M.turn == turn && ++tries < kMeetTries) __nanosleep(64);
     if (tries >= kMeetTries) s_ok = 0;
     __threadfence();
   }
+  ++turn;
   __syncthreads();
   return s_ok != 0;
 }
@@ -1109,6 +1114,7 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
                                                         int same) {
   constexpr uint32_t kForm = 8 | kAhead;
   uint32_t i = grid_tid();
+  unsigned turn = meet_turn(M);
   bool mine = i < n;
   KernelParams K = kparams(*G.h);
   bool uc = use_cache(N, K);
@@ -1151,7 +1157,7 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
     }
     if (mine) a[i] = make_float4(ai.x, ai.y, ai.z, 0.0f);
     // (with zero sums nobody reads an acceleration)
-    if (!zero && !meet(M, [] {})) break;
+    if (!zero && !meet(M, turn, [] {})) break;
     double part = 0.0;
     if (mine) {
       if (!zero) {
@@ -1171,7 +1177,7 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
     // the density error, as reduce_commit sums it, and the loop's control
     double sum = block_sum(part, sh);
     if (threadIdx.x == 0) R.partials[blockIdx.x] = sum;
-    bool ok = meet(M, [&] {
+    bool ok = meet(M, turn, [&] {
       double acc = 0.0;
       for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += __ldcg(&R.partials[b]);
       acc = block_sum(acc, sh);
@@ -1938,6 +1944,7 @@ __global__ void k_pcg_control(PcgArgs P, Red R, cudaGraphConditionalHandle h, in
 template <bool GC>
 __global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<0, 1> N, Red R, Meet M) {
   uint32_t i = grid_tid();
+  unsigned turn = meet_turn(M);
   bool mine = i < P.n;
   KernelParams K = kparams(*G.h);
   bool uc = use_cache(N, K);
@@ -1958,7 +1965,7 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<
   bool ok = true;
   while (ok && *active) {
     partial(0, mine ? 0.0 + pcg_q_item<1, GC, 8 | kAhead, true>(P, K, uc, dt, rho0, mu, N, i) : 0.0);
-    ok = meet(M, [&] {
+    ok = meet(M, turn, [&] {
       double pq = total(0);
       if (threadIdx.x == 0) {
         pcg_q_scalars(R.scalars + kSPcg, R.status, pq, *P.tol);
@@ -1970,7 +1977,7 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<
     if (mine) pcg_update_item(P, float(sc[6]), i, rr, ry);
     partial(0, rr);
     partial(1, ry);
-    ok = meet(M, [&] {
+    ok = meet(M, turn, [&] {
       double t0 = total(0), t1 = total(1);
       if (threadIdx.x == 0) {
         pcg_update_scalars(R.scalars + kSPcg, R.status, t0, t1, *P.tol, *P.max_k);
@@ -1979,7 +1986,7 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<
     });
     if (!ok || !*active) break;
     if (mine) pcg_p_item(P, float(sc[7]), i);
-    ok = meet(M, [] {});
+    ok = meet(M, turn, [] {});
   }
   if (!ok && threadIdx.x == 0) R.status[kStPcgIter] = -1; // a barrier gave up
 }
