@@ -1060,7 +1060,8 @@ __global__ void k_jacobi_control(Globals G, Red R, cudaGraphConditionalHandle h,
 // blocks are all resident (one item a thread), so they meet at barriers where
 // the graph's loop has two launches, a control's launch and a turn of the loop.  A thread keeps its item's values in
 // registers; the fields that its neighbours read (acceleration, p / rho^2) go
-// through memory, with loads that the barriers order (not the read-only ones).
+// through memory, with ordinary loads, which the barriers order for compiler and
+// device alike (a read-only or cache-hinted load need not be).
 // Values, sums and their order are those of the separate sweeps.  Set-up and
 // solve of the 27k dam break 159 -> 144 us, an 8-step run of 2k particles 1.71
 // -> 1.54 ms, of 27k 2.00 -> 1.84.
@@ -1146,7 +1147,7 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
     float ap = 0.0f;
     if (mine && !zero) {
       float pri = pi / (ri * ri), bterm = (2.0f * pi) / (ri * ri);
-      walk_nbrs_cached<kForm>(F.L, i, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), __ldca(F.pr + j)}; },
+      walk_nbrs_cached<kForm>(F.L, i, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), F.pr[j]}; },
                               [&](WithRec<float> const &r, float gf, bool in, auto cached) {
         ai = sub_if(in, ai, scl3(r.x.w * (pri + r.v), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
       });
@@ -1161,7 +1162,7 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
     double part = 0.0;
     if (mine) {
       if (!zero) {
-        walk_nbrs_cached<kForm>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldca(F.a + j))}; },
+        walk_nbrs_cached<kForm>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(F.a[j])}; },
                                 [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
           ap = add_if(in, ap, r.x.w * dot3(sub3(ai, r.v), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
         });
@@ -1179,7 +1180,7 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
     if (threadIdx.x == 0) R.partials[blockIdx.x] = sum;
     bool ok = meet(M, turn, [&] {
       double acc = 0.0;
-      for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += __ldcg(&R.partials[b]);
+      for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += R.partials[b];
       acc = block_sum(acc, sh);
       if (threadIdx.x == 0) {
         acc = 0.0 + acc;
@@ -1419,7 +1420,7 @@ struct PcgArgs {
 // LOOP: w changes during the launch (its loads are ordered by the barriers)
 template <int NB, bool GC, int BT = 8 | kAlone, bool LOOP = false>
 __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const &K, bool uc, float dt, float rho0,
-                                            float mu, Nbrs<0, NB> const &N, float4 const *__restrict__ w, uint32_t i) {
+                                            float mu, Nbrs<0, NB> const &N, float4 const *w, uint32_t i) {
   float Li[9];
   if (GC)
 #pragma unroll
@@ -1435,7 +1436,7 @@ __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const
   do {
     af = {0.0f, 0.0f, 0.0f};
     off = false;
-    walk_nbrs_cached<BT>(P.self, i, flat, [&](uint32_t j) { return WithRec<f3>{__ldg(P.xmr + j), mk3(LOOP ? __ldca(w + j) : __ldg(w + j))}; },
+    walk_nbrs_cached<BT>(P.self, i, flat, [&](uint32_t j) { return WithRec<f3>{__ldg(P.xmr + j), mk3(LOOP ? w[j] : __ldg(w + j))}; },
                          [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
       constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
       f3 xij = sub3(xi, mk3(r.x));
@@ -1955,7 +1956,7 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<
   // the sums of the block that arrives last, as reduce_commit forms them
   auto total = [&](int k) {
     double acc = 0.0;
-    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += __ldcg(&R.partials[k * kMaxRedBlocks + b]);
+    for (unsigned b = threadIdx.x; b < gridDim.x; b += blockDim.x) acc += R.partials[k * kMaxRedBlocks + b];
     return block_sum(acc, sh);
   };
   auto partial = [&](int k, double v) {
