@@ -154,6 +154,14 @@ int prtcl_gpu_model_stream(prtcl_gpu_model *model, void **stream_out);
 /* Wait for all work queued on the model's stream (and `stream`, if given). */
 int prtcl_gpu_model_synchronize(prtcl_gpu_model *model, void *stream);
 
+/* The relaxed-Jacobi and PCG loops of a scene of at most 77,824 items are one
+ * launch each, whose blocks wait for one another.  Such a wait gives up after
+ * this many polls (default 2^21, about a second).  The call that sees it first
+ * (the next procedure, list build, synchronisation or copy to the host) fails
+ * with PRTCL_GPU_ERROR; velocities, positions and the viscosity solve's results
+ * are those from before the solve, and later solves run as usual. */
+int prtcl_gpu_model_solver_polls(prtcl_gpu_model *model, uint32_t polls);
+
 /* Per-kernel timing with CUDA events on the launching stream (no
  * counterpart in the reference, whose only tracing is a disabled scope
  * macro, schemes/iisph.hpp:35).  While enabled, every procedure and grid

@@ -70,6 +70,7 @@ SIGNATURES = {
     "prtcl_gpu_profile_reset": [vp],
     "prtcl_gpu_tune_knobs": [C.c_char_p, i64, i64p],
     "prtcl_gpu_model_tune_set": [vp, cp, i32],
+    "prtcl_gpu_model_solver_polls": [vp, C.c_uint32],
     "prtcl_gpu_model_tune_get": [vp, cp, i32p],
     "prtcl_gpu_nhood_create": [pp],
     "prtcl_gpu_nhood_destroy": [vp],

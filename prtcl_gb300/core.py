@@ -303,6 +303,11 @@ class Model:
         results, different speed."""
         check(load().prtcl_gpu_model_tune_set(self._h, b(knob), int(value)))
 
+    def solver_polls(self, polls):
+        """Polls before a barrier of a one-launch solver loop gives up
+        (prtcl_gpu_model_solver_polls; the default is about a second)."""
+        check(load().prtcl_gpu_model_solver_polls(self._h, int(polls)))
+
     def tune_get(self, knob):
         v = C.c_int32(0)
         check(load().prtcl_gpu_model_tune_get(self._h, b(knob), C.byref(v)))

@@ -223,6 +223,7 @@ int prtcl_gpu_field_download(prtcl_gpu_model *model, const char *group, const ch
   return guard([&] {
     Group &g = model->m.group(group);
     download_varying(varying(model->m, group, field), g.count, host, size_t(count), model->m.pick(stream));
+    model->m.check_solver(model->m.pick(stream));
   });
 }
 int prtcl_gpu_field_info(prtcl_gpu_model *model, const char *group, const char *field, char *ctype_out,
@@ -287,6 +288,7 @@ int prtcl_gpu_model_stats(prtcl_gpu_model *model, double *out, int32_t n, int32_
     double st[16];
     PG_CUDA(cudaMemcpyAsync(st, model->m.stats_d, sizeof st, cudaMemcpyDeviceToHost, model->m.stream()));
     PG_CUDA(cudaStreamSynchronize(model->m.stream()));
+    model->m.check_solver(model->m.stream());
     for (int i = 0; i < n && i < 16; ++i) out[i] = st[i];
     if (reset) model->m.stats_reset(model->m.stream());
   });
@@ -329,7 +331,13 @@ int prtcl_gpu_model_synchronize(prtcl_gpu_model *model, void *stream) {
   return guard([&] {
     if (stream) PG_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
     PG_CUDA(cudaStreamSynchronize(model->m.stream()));
+    model->m.check_solver(model->m.pick(stream));
   });
+}
+int prtcl_gpu_model_solver_polls(prtcl_gpu_model *model, uint32_t polls) {
+  NEED(model);
+  model->m.solver_polls = polls;
+  return PRTCL_GPU_OK;
 }
 
 int prtcl_gpu_model_group_names(prtcl_gpu_model *model, char *buf, int64_t size, int64_t *needed_out) {
@@ -342,12 +350,20 @@ int prtcl_gpu_group_save_vtk(prtcl_gpu_model *model, const char *group, const ch
   NEED(model);
   NEED(group);
   NEED(path);
-  return guard([&] { save_vtk(model->m.group(group), path, model->m.stream()); });
+  return guard([&] {
+    PG_CUDA(cudaStreamSynchronize(model->m.stream()));
+    model->m.check_solver(model->m.stream());
+    save_vtk(model->m.group(group), path, model->m.stream());
+  });
 }
 int prtcl_gpu_model_save(prtcl_gpu_model *model, const char *path) {
   NEED(model);
   NEED(path);
-  return guard([&] { save_model(model->m, path, model->m.stream()); });
+  return guard([&] {
+    PG_CUDA(cudaStreamSynchronize(model->m.stream()));
+    model->m.check_solver(model->m.stream());
+    save_model(model->m, path, model->m.stream());
+  });
 }
 int prtcl_gpu_model_load(prtcl_gpu_model *model, const char *path) {
   NEED(model);

@@ -582,6 +582,9 @@ Model::Model() {
   PG_CUDA(cudaMemset(scalars_d, 0, 64 * sizeof(double)));
   PG_CUDA(cudaMalloc(&status_d, 16 * sizeof(int)));
   PG_CUDA(cudaMemset(status_d, 0, 16 * sizeof(int)));
+  PG_CUDA(cudaHostAlloc(reinterpret_cast<void **>(&solver_gave_up), sizeof(int), cudaHostAllocMapped));
+  *solver_gave_up = 0;
+  PG_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&solver_gave_up_d), solver_gave_up, 0));
   PG_CUDA(cudaMalloc(&stats_d, 16 * sizeof(double)));
   stats_reset(stream_);
   PG_CUDA(cudaStreamSynchronize(stream_));
@@ -600,6 +603,7 @@ Model::~Model() {
   cudaFree(scalars_d);
   cudaFree(status_d);
   cudaFree(stats_d);
+  cudaFreeHost(solver_gave_up);
   cudaStreamDestroy(stream_);
 }
 
@@ -701,6 +705,19 @@ void Model::stats_reset(cudaStream_t s) {
 void Model::small_get(SmallField const &f, void *host, cudaStream_t s) {
   PG_CUDA(cudaMemcpyAsync(host, small_ptr(f), f.type.host_item_bytes(), cudaMemcpyDeviceToHost, s));
   PG_CUDA(cudaStreamSynchronize(s));
+  check_solver(s);
+}
+
+void Model::check_solver(cudaStream_t s) {
+  int at = *static_cast<int volatile *>(solver_gave_up);
+  if (at == solver_raised_) return;
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &c) != cudaSuccess || c != cudaStreamCaptureStatusNone) return; // the next call raises it
+  solver_raised_ = at;
+  // behind the launch that gave up, and the loops queued since, which did nothing
+  PG_CUDA(cudaMemsetAsync(red_count_d + kMeetSlot, 0, 2 * sizeof(unsigned), s));
+  throw Error("solver loop: the blocks of its launch did not meet within the limit of " + std::to_string(solver_polls) +
+              " polls; the solve and the steps queued behind it are unfinished");
 }
 
 } // namespace prtcl_gpu

@@ -207,6 +207,15 @@ public:
   unsigned *red_count_d = nullptr; // last-block tickets
   double *scalars_d = nullptr;   // 64 FP64 solver scalars
   int *status_d = nullptr;       // 16 status words (error flags, iteration counts)
+  // The barriers of the one-launch solver loops (schemes.cu): polls before one
+  // gives up, and the launches by number with the last one that gave up, in
+  // host memory that the device writes.  check_solver() raises that once, where
+  // the host sees it first, and lets later loops on stream s run again.
+  static constexpr int kMeetSlot = 32; // red_count_d[32, 33]: arrived, turn
+  unsigned solver_polls = 1u << 21;    // about a second
+  int solver_launches = 0;
+  int *solver_gave_up = nullptr, *solver_gave_up_d = nullptr;
+  void check_solver(cudaStream_t s);
   // device-loop statistics (accumulated by the loop control kernels):
   // 0 Jacobi solves, 1 Jacobi iterations, 2 solves stopped at the cap,
   // 3 largest final aprde / nprde, 4 PCG solves, 5 PCG iterations,
@@ -252,6 +261,7 @@ private:
   std::map<std::string, SmallField> global_;
   char *arena_d_ = nullptr;
   size_t arena_cap_ = 0, arena_used_ = 0;
+  int solver_raised_ = 0;
   cudaStream_t stream_ = nullptr;
   void reindex();
 };

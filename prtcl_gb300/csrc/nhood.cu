@@ -2706,6 +2706,7 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
       PG_CUDA(cudaMemcpyAsync(stats_h_ + kStRows, stats_d_ + kStRows, kMaxListGroups * sizeof(uint32_t),
                               cudaMemcpyDeviceToHost, s));
     PG_CUDA(cudaStreamSynchronize(s));
+    model_->check_solver(s);
     if (key_check_ && !confirmed()) {
       // a new grid (read-back layout, or sorted), then these lists
       update(s);

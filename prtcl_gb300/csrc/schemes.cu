@@ -62,7 +62,6 @@ constexpr int kStJacIter = 4, kStJacDone = 5;
 // 138 us at 1M items; 11 us are left of them): set-up and solve of the 1M dam
 // break 1.54 -> 1.31 ms, of the 27k one 222 -> 204 us.
 constexpr int kStJacFirst = 6, kStSetupBad = 7; // kStSetupBad: 0 after a clean setup, until a solve takes it
-constexpr int kMeetSlot = 32; // tickets[32, 33]: the barriers of k_jacobi_loop
 constexpr int kSSetup = 32; // scalars[32]: smoothing scale, then one rest density per fluid group
 
 // ---------------------------------------------------------------------------
@@ -142,7 +141,12 @@ struct Globals {
   int const *jac_max;   // iisph_maximum_iterations
   float const *jac_eta; // iisph_maximum_density_error
   int *jac_iters;       // iisph_iterations
+  unsigned const *turn; // of the solver loops' barriers (Meet)
 };
+// whether a solver loop gave up and the host has not seen it yet: what it was
+// for is left alone then
+constexpr unsigned kGaveUp = 0x80000000u;
+__device__ __forceinline__ bool gave_up(Globals const &G) { return (*(unsigned volatile const *)G.turn & kGaveUp) != 0u; }
 
 struct Red {
   double *partials; // [3][kMaxRedBlocks]
@@ -497,13 +501,14 @@ __global__ void k_integrate_velocity(uint32_t n, float4 *__restrict__ v, float4 
                                      float const *__restrict__ tb, Globals G) {
   uint32_t i = grid_tid();
   if (i >= n) return;
+  bool keep = gave_up(G);
   float dt = *G.dt, t = *G.t, fade = *G.fade;
   float u = ustep(0.0f, (t - tb[i]) - fade);
   float4 vi = v[i], ai = a[i];
   vi.x = vi.x + (dt * ai.x) * u;
   vi.y = vi.y + (dt * ai.y) * u;
   vi.z = vi.z + (dt * ai.z) * u;
-  v[i] = vi;
+  if (!keep) v[i] = vi;
 }
 
 // symplectic_euler.integrate_position (schemes/symplectic_euler.hpp:236-270):
@@ -519,6 +524,7 @@ __global__ void k_integrate_position(uint32_t n, float4 *__restrict__ x, float4 
                                      float4 *__restrict__ xm, float const *__restrict__ m) {
   uint32_t i = grid_tid();
   int top = *reinterpret_cast<volatile int const *>(G.max_speed);
+  bool keep = gave_up(G);
   float sp = -INFINITY;
   if (i < n) {
     float dt = *G.dt;
@@ -526,9 +532,12 @@ __global__ void k_integrate_position(uint32_t n, float4 *__restrict__ x, float4 
     xi.x = xi.x + dt * vi.x;
     xi.y = xi.y + dt * vi.y;
     xi.z = xi.z + dt * vi.z;
-    x[i] = xi;
-    if (xm) xm[i] = make_float4(xi.x, xi.y, xi.z, m[i]);
-    sp = sqrtf(nsq3(mk3(vi)));
+    float mi = xm ? m[i] : 0.0f;
+    if (!keep) {
+      x[i] = xi;
+      if (xm) xm[i] = make_float4(xi.x, xi.y, xi.z, mi);
+      sp = sqrtf(nsq3(mk3(vi)));
+    }
   }
   for (int o = 16; o > 0; o >>= 1) sp = fmaxf(sp, __shfl_down_sync(0xffffffffu, sp, o));
   if ((threadIdx.x & 31) == 0 && sp > -INFINITY && __float_as_int(sp) > top)
@@ -628,9 +637,7 @@ struct RestDensities {
   int n;
 };
 // before the set-up sweeps
-__global__ void k_setup_begin(int *status, int *nprde, int total, Globals G, RestDensities D, double *scalars,
-                              unsigned *arrived) {
-  *arrived = 0u; // k_jacobi_loop's barriers
+__global__ void k_setup_begin(int *status, int *nprde, int total, Globals G, RestDensities D, double *scalars) {
   status[kStSetupBad] = 0;
   *nprde = total;
   scalars[kSSetup] = double(*G.h);
@@ -1066,27 +1073,43 @@ __global__ void k_jacobi_control(Globals G, Red R, cudaGraphConditionalHandle h,
 // solve of the 27k dam break 159 -> 144 us, an 8-step run of 2k particles 1.71
 // -> 1.54 ms, of 27k 2.00 -> 1.84.
 //
-// A barrier gives up after kMeetTries polls (about a second): the kernel then
-// returns with -1 iterations noted.
-constexpr unsigned kMeetTries = 1u << 21;
+// A barrier gives up after `polls` polls.  That marks the turn (kGaveUp) and
+// notes the launch where the host sees it (Model::check_solver, which raises an
+// error and zeroes the words again).  Until then every barrier gives up at once,
+// loops that begin return, and the fields that the solve was for stay as they
+// are: velocities, positions and PCG's results are not written (gave_up).
 struct Meet {
-  unsigned *arrived, *turn; // zero between launches (k_setup_begin, k_pcg_guess); counts barriers
+  unsigned *arrived, *turn; // arrivals at the running barrier (zero between launches); barriers passed, modulo 2^31
+  int *host, launch;
+  unsigned polls;
 };
 // The turn to wait for, read where the launch begins: it moves on only after
 // this block's first arrival, which a fence follows the read before.  Later ones
 // are counted.  (Read beside each arrival, with nothing between the two, the
 // load could take effect after the arrival and find the next turn: the block
 // would wait for one that does not come.)
-__device__ __forceinline__ unsigned meet_turn(Meet const &M) { return *(volatile unsigned *)M.turn; }
+// (thread 0 reads it before the launch's other first loads, the block shares
+// it after them)
+__device__ __forceinline__ unsigned meet_read(Meet const &M) {
+  return threadIdx.x == 0 ? *(volatile unsigned *)M.turn : 0u;
+}
+__device__ __forceinline__ unsigned meet_share(unsigned turn) {
+  __shared__ unsigned s_turn;
+  if (threadIdx.x == 0) s_turn = turn;
+  __syncthreads();
+  return s_turn;
+}
 // last(): run by the block that arrives last, in all its threads, before the
 // others go on.  False where the barrier gave up.
 template <class F> __device__ bool meet(Meet const &M, unsigned &turn, F &&last) {
   __shared__ int s_last, s_ok;
+  unsigned next = (turn + 1u) & (kGaveUp - 1u);
   __threadfence();
   __syncthreads();
   if (threadIdx.x == 0) {
-    s_last = atomicAdd(M.arrived, 1u) == gridDim.x - 1 ? 1 : 0;
-    s_ok = 1;
+    bool all = atomicAdd(M.arrived, 1u) == gridDim.x - 1;
+    s_ok = !all || *(volatile unsigned *)M.turn == turn ? 1 : 0;
+    s_last = all && s_ok ? 1 : 0;
   }
   __syncthreads();
   if (s_last) {
@@ -1097,15 +1120,20 @@ template <class F> __device__ bool meet(Meet const &M, unsigned &turn, F &&last)
     if (threadIdx.x == 0) {
       *M.arrived = 0u;
       __threadfence();
-      atomicAdd(M.turn, 1u);
+      atomicAdd(M.turn, next - turn);
     }
-  } else if (threadIdx.x == 0) {
-    unsigned tries = 0;
-    while (*(volatile unsigned *)M.turn == turn && ++tries < kMeetTries) __nanosleep(64);
-    if (tries >= kMeetTries) s_ok = 0;
+  } else if (threadIdx.x == 0 && s_ok) {
+    unsigned now, polls = 0;
+    while ((now = *(volatile unsigned *)M.turn) == turn && polls++ < M.polls) __nanosleep(64);
+    if (now == turn) {
+      atomicOr(M.turn, kGaveUp);
+      *(volatile int *)M.host = M.launch;
+      __threadfence_system();
+    }
+    if (now != next) s_ok = 0;
     __threadfence();
   }
-  ++turn;
+  turn = next;
   __syncthreads();
   return s_ok != 0;
 }
@@ -1115,7 +1143,7 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
                                                         int same) {
   constexpr uint32_t kForm = 8 | kAhead;
   uint32_t i = grid_tid();
-  unsigned turn = meet_turn(M);
+  unsigned turn = meet_read(M);
   bool mine = i < n;
   KernelParams K = kparams(*G.h);
   bool uc = use_cache(N, K);
@@ -1133,6 +1161,8 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
   // once every block has read them
   bool zero = zero_sums_hold(G, D, R.status, R.scalars, same);
   int ended = *G.nprde >= 1 ? 0 : 1;
+  turn = meet_share(turn);
+  if (turn & kGaveUp) return;
   if (ended && i == 0) {
     R.status[kStSetupBad] = 1;
     R.status[kStJacIter] = 0;
@@ -1201,7 +1231,6 @@ __global__ void __launch_bounds__(kNT, 4) k_jacobi_loop(uint32_t n, PressureArgs
     ended = s_ended;
     zero = false;
   }
-  if (!ended && threadIdx.x == 0) *G.jac_iters = -1; // a barrier gave up
 }
 
 // ---------------------------------------------------------------------------
@@ -1469,9 +1498,8 @@ __device__ __forceinline__ f3 wkbb18_system(PcgArgs const &P, KernelParams const
 
 // scalars: 0 b_nsq, 1 thr, 2 r_nsq, 3 next_rdy, 4 prev_rdy, 5 pdq,
 // 6 alpha, 7 beta (f32 values held in double slots)
-__global__ void k_pcg_guess(PcgArgs P, unsigned *arrived) {
+__global__ void k_pcg_guess(PcgArgs P) {
   uint32_t i = grid_tid();
-  if (i == 0) *arrived = 0u; // k_pcg_loop's barriers
   if (i < P.n) P.X[i] = P.v[i];
 }
 
@@ -1945,13 +1973,15 @@ __global__ void k_pcg_control(PcgArgs P, Red R, cudaGraphConditionalHandle h, in
 template <bool GC>
 __global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<0, 1> N, Red R, Meet M) {
   uint32_t i = grid_tid();
-  unsigned turn = meet_turn(M);
+  unsigned turn = meet_read(M);
   bool mine = i < P.n;
   KernelParams K = kparams(*G.h);
   bool uc = use_cache(N, K);
   float dt = *G.dt, rho0 = *P.rho0, mu = *P.mu;
   double volatile const *sc = R.scalars + kSPcg;
   int volatile const *active = &R.status[kStPcgActive];
+  turn = meet_share(turn);
+  if (turn & kGaveUp) return;
   __shared__ double sh[32];
   // the sums of the block that arrives last, as reduce_commit forms them
   auto total = [&](int k) {
@@ -1989,7 +2019,6 @@ __global__ void __launch_bounds__(kNT, 4) k_pcg_loop(PcgArgs P, Globals G, Nbrs<
     if (mine) pcg_p_item(P, float(sc[7]), i);
     ok = meet(M, turn, [] {});
   }
-  if (!ok && threadIdx.x == 0) R.status[kStPcgIter] = -1; // a barrier gave up
 }
 
 // --- the PCG loop over the tiles of a batched model, per slot -------------
@@ -2097,11 +2126,13 @@ __global__ void k_seg_pcg_begin(SegArgs S) {
 // a = vd / dt
 __global__ void k_pcg_apply(PcgArgs P, Globals G, Red R) {
   uint32_t i = grid_tid();
-  if (i == 0 && R.status) *P.iterations = R.status[kStPcgIter];
+  bool keep = gave_up(G);
+  if (i == 0 && R.status && !keep) *P.iterations = R.status[kStPcgIter];
   if (i >= P.n) return;
   float dt = *G.dt, t = *G.t, fade = *G.fade;
   float u = ustep(0.0f, (t - P.tb[i]) - fade);
   f3 d = scl3(u, sub3(mk3(P.X[i]), mk3(P.v[i])));
+  if (keep) return;
   P.vd[i] = make_float4(d.x, d.y, d.z, 0.0f);
   P.a[i] = make_float4(d.x / dt, d.y / dt, d.z / dt, 0.0f);
 }
@@ -2256,6 +2287,7 @@ void Scheme::run(std::string const &procedure, Nhood &nh, cudaStream_t s) {
   auto it = procs_.find(procedure);
   if (it == procs_.end()) throw Error("procedure does not exist");
   if (!model_) throw Error("scheme has not been loaded");
+  model_->check_solver(s);
   it->second(nh, s);
 }
 
@@ -2308,7 +2340,12 @@ protected:
     G.jac_max = static_cast<int const *>(gp("iisph_maximum_iterations"));
     G.jac_eta = static_cast<float const *>(gp("iisph_maximum_density_error"));
     G.jac_iters = static_cast<int *>(gp("iisph_iterations"));
+    G.turn = m.red_count_d + Model::kMeetSlot + 1;
     return G;
+  }
+  Meet meeting(Model &m) {
+    return Meet{m.red_count_d + Model::kMeetSlot, m.red_count_d + Model::kMeetSlot + 1, m.solver_gave_up_d,
+                ++m.solver_launches, m.solver_polls};
   }
   Red red(Model &m, int slot) {
     Red R;
@@ -2849,8 +2886,7 @@ public:
     long long total = 0;
     for (auto *F : active()) total += (long long)F->g->count;
     // nprde = number of fluid particles (the generated reduction adds 1 per particle)
-    k_setup_begin<<<1, 1, 0, s>>>(model_->status_d, G.nprde, int(total), G, rest_densities(), model_->scalars_d,
-                                  model_->red_count_d + kMeetSlot);
+    k_setup_begin<<<1, 1, 0, s>>>(model_->status_d, G.nprde, int(total), G, rest_densities(), model_->scalars_d);
     count_launch();
     for (auto *F : active()) {
       dispatch_fb<SETUP>(nf, nb, this, *F, lists(nh, F->g, G, s), G, s);
@@ -3035,7 +3071,7 @@ private:
     PressureArgs PA{dptr<float4>(F.x), dptr<float4>(F.a), dptr<float>(F.rho), dptr<float>(F.s), dptr<float>(F.AA),
                     dptr<float>(F.p), model_->pr_buffer(F.g, s), dptr<float>(F.Ap), u(F.rho0)};
     float4 *a = dptr<float4>(F.a);
-    Meet M{R.ticket + kMeetSlot, R.ticket + kMeetSlot + 1};
+    Meet M = meeting(*model_);
     RestDensities D = rest_densities();
     void *args[] = {&n, &PA, &a, &G, &N, &R, &M, &D, &same};
     return launch_resident(k_jacobi_loop, div_up(n, kNT), args, s, resident_);
@@ -3168,8 +3204,7 @@ public:
     bool seg = segmented(F.g);
     SegArgs SA = seg ? seg_args(F.g) : SegArgs{};
     unsigned tg = SA.ntiles;
-    Meet M{model_->red_count_d + kMeetSlot, model_->red_count_d + kMeetSlot + 1};
-    k_pcg_guess<<<eg, 256, 0, s>>>(P, M.arrived); count_launch();
+    k_pcg_guess<<<eg, 256, 0, s>>>(P); count_launch();
     constexpr bool kTuned = NB == 1 && !GC;
     int tv_init = fluid_.size() == 1 ? model_->tune.v[kTunePcgInit] : 0;
     int tv_q = fluid_.size() == 1 ? model_->tune.v[kTunePcgQ] : 0;
@@ -3263,6 +3298,7 @@ public:
     };
     bool one_launch = false;
     if constexpr (NB == 1) {
+      Meet M = meeting(*model_);
       void *args[] = {&P, &G, &N, &R, &M};
       one_launch = !seg && !staged && !tiles && fluid_.size() == 1 && !model_->prof.enabled && n <= kSmallItems &&
                    !capturing(s) && rg <= unsigned(resident_blocks(k_pcg_loop<GC>, resident_)) &&
