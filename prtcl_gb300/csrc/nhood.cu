@@ -2354,9 +2354,10 @@ bool Nhood::confirmed() {
   bool ok = true;
   KeyInfo k = key_from_stats(stats_h_);
   if (!same_key(k, key_) ||
-      (counted_ && !same_dir(dir_from_stats(stats_h_, k, seg_count_ ? seg_bits_ : 0), dir_key_)))
+      (counted_ && !same_dir(dir_from_stats(stats_h_, k, seg_count_ ? seg_bits_ : 0), dir_key_))) {
+    // (another layout folds cells into one entry: its fullest says nothing)
     ok = key_known_ = false;
-  if (counted_ && stats_h_[kStMaxCell] > kDirMaxCell) {
+  } else if (counted_ && stats_h_[kStMaxCell] > kDirMaxCell) {
     dense_ = true;
     ok = false;
   }
