@@ -598,7 +598,10 @@ __global__ void k_cells_key(uint32_t const *ukeys, uint32_t const *vals, size_t 
 // on its own before: 27k dam break 96 -> 49 us, 1M 242 -> 110, 4M uniform
 // points in random order 535 -> 238, 1.5M clustered 337 -> 175.
 constexpr int kDirectBits = 27;
-constexpr uint32_t kDirNT = 256, kDirMaxCell = 256;
+// A grid that had such a cell is sorted until no cell has more than kDirRoomy
+// items (k_cf_fill looks, of a sorted grid that might be counted), so that a
+// cell that stays about as full is not counted in vain every other update.
+constexpr uint32_t kDirNT = 256, kDirMaxCell = 256, kDirRoomy = 192;
 static_assert(kDirNT / 32 * kDirRun == kDirTile, "a warp per run");
 
 __device__ __forceinline__ uint64_t block_excl_scan64(uint64_t v, uint64_t *sh /* kDirNT / 32 */, uint64_t &total) {
@@ -950,12 +953,13 @@ __global__ void __launch_bounds__(kScanNT) k_cf_count(uint64_t const *__restrict
 }
 
 // excl_tiles: the exclusive scan of k_cf_count's sums; cell(s) is the
-// number of cell starts at or before s, minus one
+// number of cell starts at or before s, minus one.  crowd, where given: set
+// where a cell has more than kDirRoomy items
 __global__ void __launch_bounds__(kScanNT) k_cf_fill(const __grid_constant__ PosTable pt, GridView gv, uint64_t const *__restrict__ keys,
                                                      uint32_t const *__restrict__ vals, uint32_t const *excl_tiles,
                                                      size_t N, int32_t *s2c, int32_t *cell_start,
                                                      uint64_t *cell_key, int4 *cell_gi, int *ncells,
-                                                     int32_t *cell_adj) {
+                                                     int32_t *cell_adj, uint32_t *crowd) {
   __shared__ uint32_t sh[32];
   size_t base = size_t(blockIdx.x) * kScanTile + size_t(threadIdx.x) * kScanIPT;
   uint64_t key[kScanIPT];
@@ -996,6 +1000,7 @@ __global__ void __launch_bounds__(kScanNT) k_cf_fill(const __grid_constant__ Pos
       // (a cell's 26 slots start at a multiple of 104 bytes: 8-byte stores)
       int2 *a = reinterpret_cast<int2 *>(cell_adj + size_t(c) * 26);
       for (int q = 0; q < 13; ++q) a[q] = make_int2(-1, -1);
+      if (crowd && si + kDirRoomy < N && keys[si + kDirRoomy] == key[k]) *crowd = 1u;
     }
     if (si == N - 1) {
       cell_start[c + 1] = int32_t(N);
@@ -2285,7 +2290,7 @@ void Nhood::settle(cudaStream_t s) {
 // Whether a grid of N items is built by counting, with the tables allocated:
 // the knob is on, the entries are at most 2^27 and 128 an item (8 bytes each,
 // about what the lists take; an entry that no item maps to is never read) or
-// 2^18, and the last counted grid at this radius had no overfull cell.
+// 2^18, and no cell was overfull lately.
 bool Nhood::direct_ready(size_t N, cudaStream_t s) {
   if (!model_->tune.v[kTuneGridSort] || dense_ || !dir_key_.nruns || dir_key_.bits > kDirectBits) return false;
   size_t entries = std::max<size_t>(size_t(1) << dir_key_.bits, kDirTile);
@@ -2360,6 +2365,8 @@ bool Nhood::confirmed() {
   } else if (counted_ && stats_h_[kStMaxCell] > kDirMaxCell) {
     dense_ = true;
     ok = false;
+  } else if (!counted_ && !stats_h_[kStMaxCell]) {
+    dense_ = false; // (k_cf_fill's word)
   }
   return ok;
 }
@@ -2521,7 +2528,8 @@ void Nhood::update(cudaStream_t s) {
     k_cf_count<<<unsigned(tiles_c), kScanNT, 0, s>>>(kin, N, block_sums_); count_launch();
     k_scan_single<<<1, 1024, 0, s>>>(block_sums_, tiles_c); count_launch();
     k_cf_fill<<<unsigned(tiles_c), kScanNT, 0, s>>>(pt, gv, kin, vin, block_sums_, N, s2c_, cell_start_,
-                                                   cell_key_, cell_gi_, ncells_d_, cell_adj_);
+                                                   cell_key_, cell_gi_, ncells_d_, cell_adj_,
+                                                   dense_ ? stats_d_ + kStMaxCell : nullptr);
     count_launch();
     PG_LAUNCH_CHECK();
   }

@@ -305,7 +305,7 @@ private:
   uint32_t *order_ = nullptr; // group items in grid order (list build)
   // grid by counting: per cell key the item count (zero between updates), the
   // cell, and the tile sums; counted_: the present grid was built that way;
-  // dense_: a cell was too full for it, at this radius
+  // dense_: a cell was too full for it, at this radius, and the cells have not emptied since
   uint32_t *dir_count_ = nullptr, *dir_cell_ = nullptr;
   uint64_t *dir_sums_ = nullptr;
   uint32_t *dir_touched_ = nullptr;

@@ -55,3 +55,29 @@ def test_mispredicted_layout_is_no_crowd():
         for k in want:
             assert_bitwise(g[k], want[k], k)
     assert launches == counted
+
+
+@pytest.mark.parametrize("m", [257, 400])
+def test_counts_again_once_a_crowd_is_gone(m):
+    """A cell too full to count, one that is nearly so, then none: sorted while
+    it lasts and once more, counted after that."""
+    rng = np.random.default_rng(m)
+    even = points(rng, np.arange(0, 120, 2))
+
+    def crowd(k):
+        x = even.copy()
+        x[:k] = (rng.random((k, 3)) * 0.8 * R + 0.1 * R).astype(np.float32)
+        return x
+
+    counted, sorted_ = launches_of(1, even), launches_of(0, even)
+    d, o = scene(even), scene(even, 0)
+    took = []
+    for x in (even, even, crowd(m), crowd(m), crowd(230), crowd(230), even, even, even):
+        launches, g = move(d, x)
+        want = move(o, x)[1]
+        for k in want:
+            assert_bitwise(g[k], want[k], k)
+        took.append(launches)
+    cluster = took[3]  # (the cluster sort, where the radix sort's passes are the knob's other side)
+    assert cluster != counted
+    assert took[1] == counted and took[3:7] == [cluster] * 4 and took[7:] == [counted] * 2
