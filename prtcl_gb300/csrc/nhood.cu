@@ -2107,6 +2107,23 @@ static void free_all(std::initializer_list<void *> ps) {
     if (p) cudaFree(p);
 }
 
+// all of them, or (false: no memory) none
+static bool alloc_all(std::initializer_list<std::pair<void **, size_t>> ps) {
+  for (auto const &p : ps) {
+    cudaError_t e = cudaMalloc(p.first, p.second);
+    if (e == cudaSuccess) continue;
+    *p.first = nullptr;
+    for (auto const &q : ps) {
+      if (*q.first) cudaFree(*q.first);
+      *q.first = nullptr;
+    }
+    if (e != cudaErrorMemoryAllocation) PG_CUDA(e);
+    cudaGetLastError();
+    return false;
+  }
+  return true;
+}
+
 Nhood::~Nhood() {
   for (auto &kv : lists_) free_lists(kv.second);
   free_all({keys_a_, keys_b_, vals_a_, vals_b_, ukeys_, flags_, scan_, r2s_, s2c_, cell_start_, cell_adj_, cell_key_,
@@ -2290,22 +2307,30 @@ void Nhood::settle(cudaStream_t s) {
 // Whether a grid of N items is built by counting, with the tables allocated:
 // the knob is on, the entries are at most 2^27 and 128 an item (8 bytes each,
 // about what the lists take; an entry that no item maps to is never read) or
-// 2^18, and no cell was overfull lately.
+// 2^18, and no cell was overfull lately.  Where there is no memory for the
+// tables, or they would have to be allocated while s captures, the grid is
+// sorted, which needs none of them.
 bool Nhood::direct_ready(size_t N, cudaStream_t s) {
   if (!model_->tune.v[kTuneGridSort] || dense_ || !dir_key_.nruns || dir_key_.bits > kDirectBits) return false;
-  size_t entries = std::max<size_t>(size_t(1) << dir_key_.bits, kDirTile);
-  if (entries > std::max<size_t>(128 * N, size_t(1) << 18)) return false;
-  if (entries > dir_cap_) {
+  size_t entries = std::max<size_t>(size_t(1) << dir_key_.bits, kDirTile), most = std::max<size_t>(128 * N, size_t(1) << 18);
+  if (entries > most) return false;
+  // (tables made for many more items are given back)
+  if (entries > dir_cap_ || dir_cap_ > 4 * most) {
+    if (capturing(s)) return entries <= dir_cap_;
+    if (dir_wait_ > 0) return --dir_wait_, false;
     free_all({dir_count_, dir_cell_, dir_sums_, dir_touched_});
     dir_count_ = dir_cell_ = nullptr;
     dir_sums_ = nullptr;
     dir_touched_ = nullptr;
     dir_cap_ = 0;
     size_t tiles = entries / kDirTile, runs = entries / kDirRun;
-    PG_CUDA(cudaMalloc(&dir_count_, entries * sizeof(uint32_t)));
-    PG_CUDA(cudaMalloc(&dir_cell_, entries * sizeof(uint32_t)));
-    PG_CUDA(cudaMalloc(&dir_sums_, (tiles + kDirBlocks) * sizeof(uint64_t)));
-    PG_CUDA(cudaMalloc(&dir_touched_, runs * kMark * sizeof(uint32_t)));
+    if (!alloc_all({{reinterpret_cast<void **>(&dir_count_), entries * sizeof(uint32_t)},
+                    {reinterpret_cast<void **>(&dir_cell_), entries * sizeof(uint32_t)},
+                    {reinterpret_cast<void **>(&dir_sums_), (tiles + kDirBlocks) * sizeof(uint64_t)},
+                    {reinterpret_cast<void **>(&dir_touched_), runs * kMark * sizeof(uint32_t)}})) {
+      dir_wait_ = 256; // updates until it is tried again
+      return false;
+    }
     PG_CUDA(cudaMemsetAsync(dir_count_, 0, entries * sizeof(uint32_t), s));
     PG_CUDA(cudaMemsetAsync(dir_touched_, 0, runs * kMark * sizeof(uint32_t), s));
     dir_cap_ = entries;

@@ -311,6 +311,7 @@ private:
   uint32_t *dir_touched_ = nullptr;
   DirKey dir_key_{};
   size_t dir_cap_ = 0;
+  int dir_wait_ = 0;
   bool counted_ = false, dense_ = false;
   uint64_t r2s_epoch_ = 0;
   uint64_t *hkeys_ = nullptr;  // cell-key hash table (adjacency lookups)

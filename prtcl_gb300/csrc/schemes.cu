@@ -2439,11 +2439,6 @@ protected:
     PG_CUDA(cudaFuncSetAttribute(k_pcg_q_staged<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kStageSmem)));
     return true;
   }
-  static bool capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
-    PG_CUDA(cudaStreamIsCapturing(s, &c));
-    return c != cudaStreamCaptureStatusNone;
-  }
   // blocks of a cooperative kernel of kNT threads that the device holds at once
   // (asked for once per scheme: `known` starts at -1)
   template <class Kernel> static int resident_blocks(Kernel *kernel, int &known) {
