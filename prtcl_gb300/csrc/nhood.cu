@@ -766,13 +766,13 @@ __global__ void k_dir_scatter(GridView gv, int G, uint2 const *__restrict__ plac
 // (and the positions in that order, which the list build reads)
 __global__ void k_dir_order(const __grid_constant__ PosTable pt, uint32_t const *__restrict__ vals,
                             int32_t const *__restrict__ s2c, int32_t const *__restrict__ cell_start, size_t N,
-                            uint32_t *__restrict__ out, float4 *__restrict__ xs) {
+                            uint32_t *__restrict__ out, float4 *__restrict__ xs, int fullest) {
   size_t s = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
   if (s >= N) return;
   uint32_t h = vals[s];
   int c = s2c[s], b = cell_start[c], e = cell_start[c + 1], r = int(s);
   float4 x = pt.pos[h >> 28][h & 0x0FFFFFFFu];
-  if (e - b <= int(kDirMaxCell)) { // (a fuller cell: repeated with the radix sort)
+  if (e - b <= fullest) { // (a fuller cell: repeated with the radix sort)
     r = b;
     for (int t = b; t < e; ++t) r += vals[t] < h ? 1 : 0;
   }
@@ -2366,7 +2366,10 @@ void Nhood::build_direct(GridView const &gv, int G, size_t N, cudaStream_t s) {
       k_dir_adj<<<std::min(div_up(N, kDirAdjNT), kDirBlocks), kDirAdjNT, 0, s>>>(gv, T, scan_, cell_key_, cell_gi_,
                                                                                cell_adj_, s2c_);
     count_launch();
-    k_dir_order<<<nb, 256, 0, s>>>(pt, vals_b_, s2c_, cell_start_, N, vals_a_, xsorted_); count_launch();
+    // (a captured update is replayed without a look at its fullest cell)
+    k_dir_order<<<nb, 256, 0, s>>>(pt, vals_b_, s2c_, cell_start_, N, vals_a_, xsorted_,
+                                   capturing(s) ? INT32_MAX : int(kDirMaxCell));
+    count_launch();
     xsorted_of_ = pos_versions();
     xsorted_epoch_ = epoch_;
     PG_LAUNCH_CHECK();

@@ -50,3 +50,23 @@ def test_without_a_table():
     replay = captured(d)
     replay()
     equal(d, x)
+
+
+@pytest.mark.parametrize("m", [0, 300, 1500])
+def test_cells_that_fill_between_replays(m):
+    """Cells of any size come out in (group, raw index) order, at the first
+    replay and at later ones, whose cells the host does not look at."""
+    rng = np.random.default_rng(m)
+    x = (rng.random((3000, 3)) * 0.9).astype(np.float32)
+    x[:2] = (0.05, 0.05, 0.05), (0.85, 0.85, 0.85)  # (the key bits stay the same)
+    d = scene(x, 1)
+    for _ in range(2):
+        d.update()
+    replay = captured(d)
+    replay()
+    equal(d, x)
+    full = x.copy()
+    full[rng.permutation(np.arange(2, 3000))[:m]] = (rng.random((m, 3)) * 0.08 + 0.41).astype(np.float32)
+    d.set_varying("p", "position", full)
+    replay()
+    equal(d, full)
