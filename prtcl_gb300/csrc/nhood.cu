@@ -2404,7 +2404,7 @@ void Nhood::need_r2s(cudaStream_t s) {
   if (r2s_epoch_ == epoch_ || !N_) return;
   k_r2s<<<div_up(N_, 256), 256, 0, s>>>(sorted_vals_, view(), N_, r2s_); count_launch();
   PG_LAUNCH_CHECK();
-  r2s_epoch_ = epoch_;
+  if (!capturing(s)) r2s_epoch_ = epoch_; // (captured: it has not run yet)
 }
 
 // an epoch names one update of one neighbourhood of the process, so that what is
