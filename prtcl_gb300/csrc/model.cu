@@ -148,6 +148,7 @@ void upload_varying(VaryingField &f, size_t count, void const *host, size_t n_it
   if (n_items != count)
     throw Error("upload: item count " + std::to_string(n_items) + " != group count " + std::to_string(count));
   f.version++;
+  if (!sync && capturing(s)) f.unseen = true;
   if (count == 0) return;
   size_t hbytes = count * f.type.host_item_bytes();
   if (!f.type.is_vec3() && !f.type.is_mat3()) {
@@ -274,8 +275,10 @@ void Group::resize(size_t n, cudaStream_t s) {
 void Group::permute(uint32_t const *perm, cudaStream_t s) {
   size_t n = count;
   if (n == 0) return;
+  bool captured = capturing(s);
   for (auto &kv : varying) {
     VaryingField &f = kv.second;
+    if (captured) f.unseen = true;
     void *nd = alloc_field(f.type, f.cap, s);
     unsigned b = 256;
     if (f.type.is_vec3()) {
@@ -706,6 +709,22 @@ void Model::small_get(SmallField const &f, void *host, cudaStream_t s) {
   PG_CUDA(cudaMemcpyAsync(host, small_ptr(f), f.type.host_item_bytes(), cudaMemcpyDeviceToHost, s));
   PG_CUDA(cudaStreamSynchronize(s));
   check_solver(s);
+}
+
+std::vector<uint64_t> Model::field_versions() const {
+  std::vector<uint64_t> v;
+  for (auto const &g : groups_)
+    for (auto const &f : g.second->varying) v.push_back(f.second.version);
+  return v;
+}
+
+void Model::note_captured(std::vector<uint64_t> const &before) {
+  size_t k = 0;
+  for (auto &g : groups_)
+    for (auto &f : g.second->varying) {
+      if (k >= before.size() || f.second.version != before[k]) f.second.unseen = true;
+      ++k;
+    }
 }
 
 void Model::check_solver(cudaStream_t s) {

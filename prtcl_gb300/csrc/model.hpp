@@ -53,6 +53,9 @@ struct VaryingField {
   void *d = nullptr;   // device storage
   size_t cap = 0;      // items allocated
   uint64_t version = 0; // bumped whenever the values may have changed
+  // a captured procedure writes it: replays of its graph change the values
+  // without the version
+  bool unseen = false;
   size_t device_item_bytes() const; // bytes per item of the device array (non-planar)
 };
 
@@ -216,6 +219,9 @@ public:
   int solver_launches = 0;
   int *solver_gave_up = nullptr, *solver_gave_up_d = nullptr;
   void check_solver(cudaStream_t s);
+  // around a procedure on a capturing stream: the fields that it writes
+  std::vector<uint64_t> field_versions() const;
+  void note_captured(std::vector<uint64_t> const &before);
   // device-loop statistics (accumulated by the loop control kernels):
   // 0 Jacobi solves, 1 Jacobi iterations, 2 solves stopped at the cap,
   // 3 largest final aprde / nprde, 4 PCG solves, 5 PCG iterations,

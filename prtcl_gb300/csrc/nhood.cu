@@ -2605,7 +2605,9 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
   PosTable pt{};
   for (int g = 0; g < G; ++g)
     if (gg_[g].pos) pt.pos[g] = static_cast<float4 const *>(gg_[g].pos->d);
-  if (N_ > 0 && !(xsorted_epoch_ == epoch_ && xsorted_of_ == pos_versions())) {
+  bool seen = true; // (else a replay may have moved them since the update)
+  for (auto const &g : gg_) seen = seen && !(g.pos && g.pos->unseen);
+  if (N_ > 0 && !(seen && xsorted_epoch_ == epoch_ && xsorted_of_ == pos_versions())) {
     k_xsorted<<<div_up(N_, 256), 256, 0, s>>>(pt, sorted_vals_, N_, xsorted_); count_launch();
     PG_LAUNCH_CHECK();
   }

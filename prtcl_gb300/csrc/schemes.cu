@@ -2288,7 +2288,18 @@ void Scheme::run(std::string const &procedure, Nhood &nh, cudaStream_t s) {
   if (it == procs_.end()) throw Error("procedure does not exist");
   if (!model_) throw Error("scheme has not been loaded");
   model_->check_solver(s);
-  it->second(nh, s);
+  if (!capturing(s)) {
+    it->second(nh, s);
+    return;
+  }
+  std::vector<uint64_t> before = model_->field_versions();
+  try {
+    it->second(nh, s);
+  } catch (...) {
+    model_->note_captured(before);
+    throw;
+  }
+  model_->note_captured(before);
 }
 
 std::vector<std::string> Scheme::procedure_names() const {
