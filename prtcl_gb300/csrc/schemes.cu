@@ -2914,19 +2914,23 @@ public:
   }
   // What the first iteration's zero sums rest on (kStJacFirst): the fields
   // that setup read, the pressure it wrote, the grid of its lists and the
-  // stream it ran on.  A solve takes them only where the key is still the
-  // same; it is cleared by the solve, which changes the pressure.
+  // stream it ran on; empty where captured work writes one of the fields.  A
+  // solve takes them only where the key is still the same; it is cleared by the
+  // solve, which changes the pressure.
   std::vector<uint64_t> zero_key(Nhood &nh, cudaStream_t s) {
     std::vector<uint64_t> k{reinterpret_cast<uint64_t>(&nh), nh.epoch(), reinterpret_cast<uint64_t>(s)};
+    bool seen = true; // (else a replayed graph may have changed them)
     auto add = [&](Group *g, std::initializer_list<VaryingField const *> fs) {
       k.push_back(uint64_t(g->count));
       for (auto *f : fs) {
         k.push_back(reinterpret_cast<uint64_t>(f->d));
         k.push_back(f->version);
+        seen = seen && !f->unseen;
       }
     };
     for (auto &F : fluid_) add(F.g, {F.x, F.m, F.rho, F.p});
     for (auto &B : bound_) add(B.g, {B.x, B.V});
+    if (!seen) k.clear();
     return k;
   }
   void no_segments(char const *what) {
