@@ -51,10 +51,11 @@ constexpr int kStJacIter = 4, kStJacDone = 5;
 // the pressure acceleration is a zero, hence a = +0, hence every term of
 // iteration_pressure's sum is a zero, hence the sum is +0 (sums that start at
 // +0 and add or subtract zeros of either sign stay +0).  That holds while all
-// masses, volumes, densities and kernel gradients of the pairs are finite;
-// setup's helper sum c walks the same pairs with the same factors, and is not
-// finite where one of them is not (every item in the grid is its own
-// neighbour, so its own mass and density count too).  Setup notes what it
+// masses, volumes, densities and kernel gradients of the pairs, and the products
+// of rest density and volume, are finite; setup's helper sum c walks the same
+// pairs with the same factors, and is not finite where one of them is not (every
+// item in the grid is its own neighbour, so its own mass and density count too),
+// nor is its diagonal sum where one of the products is not.  Setup notes what it
 // found (kStSetupBad, and in scalars[kSSetup..] the smoothing scale and rest
 // densities it used), the host checks that no field, list or pressure has
 // changed since, and k_jacobi_begin (k_jacobi_loop) takes them where both agree.  Of
@@ -599,7 +600,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
     flat = false;
   } while (true);
   cout[i] = make_float4(c.x, c.y, c.z, 0.0f);
-  if (!(isfinite(c.x) && isfinite(c.y) && isfinite(c.z))) *bad = 1;
+  bool finite = isfinite(c.x) && isfinite(c.y) && isfinite(c.z);
   f3 vi = mk3(v[i]), ci = c;
   float mi = m[i];
   float sa = 0.0f, aa = 0.0f;
@@ -626,6 +627,7 @@ __global__ void __launch_bounds__(NT, MINB) k_iisph_setup(uint32_t n, float4 con
       aa = add_if(in, aa, w * dot3(ci, g));
     });
   }
+  if (!(finite && isfinite(aa))) *bad = 1;
   p[i] = 0.0f;
   pr[i] = 0.0f / (ri * ri);
   s[i] = (rho0 - ri) - ((dt * (rho0 / ri)) * sa);
