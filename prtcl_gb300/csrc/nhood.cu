@@ -1145,11 +1145,18 @@ __global__ void __launch_bounds__(128) k_cells_adj_hash(GridView gv, int4 const 
   }
 }
 
-__global__ void k_xsorted(const __grid_constant__ PosTable pt, uint32_t const *vals, size_t N, float4 *xs) {
+// the groups' present counts: an item that its group no longer has (resized
+// since the grid's update) is at infinity, where it is nobody's neighbour
+struct CountTable {
+  uint32_t n[kMaxGroups];
+};
+__global__ void k_xsorted(const __grid_constant__ PosTable pt, const __grid_constant__ CountTable ct, uint32_t const *vals,
+                          size_t N, float4 *xs) {
   size_t s = blockIdx.x * size_t(blockDim.x) + threadIdx.x;
   if (s < N) {
-    uint32_t h = vals[s];
-    float4 x = pt.pos[h >> 28][h & 0x0FFFFFFFu];
+    uint32_t h = vals[s], g = h >> 28, i = h & 0x0FFFFFFFu;
+    float4 x = make_float4(INFINITY, INFINITY, INFINITY, 0.0f);
+    if (i < ct.n[g]) x = pt.pos[g][i];
     x.w = __uint_as_float(h);
     xs[s] = x;
   }
@@ -1487,12 +1494,16 @@ __global__ void __launch_bounds__(kBuildNT, STAGE ? 5 : (NG <= 2 ? 9 : 1))
   if (t == 0) *hcache = with_gf ? K.h : __int_as_float(0x7fc00000);
   bool staged = false;
   if constexpr (STAGE) {
-    bool has = t < lo.n;
+    bool has = t < lo.n && t < gv.goff[q + 1] - gv.goff[q];
     int home = has ? gv.s2c[gv.r2s[gv.goff[q] + t]] : -1;
     staged = stage_tile(gv, home, has, blockIdx.x, lo, s_hkey, s_hbase);
   }
   if (t >= lo.n) return;
   uint32_t i = order ? order[t] : t;
+  if (gv.in_grid[q] && i >= gv.goff[q + 1] - gv.goff[q]) { // newer than the grid: no neighbours
+    for (int g = 0; g < lo.G; ++g) lo.cb[size_t(g) * lo.n + i] = make_uint2(0u, 0u);
+    return;
+  }
   RowState R[NG];
 #pragma unroll
   for (int g = 0; g < NG; ++g) R[g] = RowState{0u, 0u, false};
@@ -1983,7 +1994,7 @@ template <int NG>
 void launch_build_lists_warp(size_t N, cudaStream_t s, GridView const &gv, float4 const *xs, int q, ListOut const &lo,
                              float const *h, float *hcache) {
   uint32_t window = N <= kWinSmall ? kWinItems / 4 : N <= kWinMedium ? kWinItems / 2 : kWinItems;
-  unsigned nb = div_up(div_up(N, window), kWarps);
+  unsigned nb = std::max(div_up(div_up(N, window), kWarps), 1u); // (an empty grid: *hcache is written all the same)
   if (h) k_build_lists_warp<NG, true><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache, window);
   else k_build_lists_warp<NG, false><<<nb, kWarpNT, 0, s>>>(gv, xs, N, q, lo, h, hcache, window);
 }
@@ -2608,7 +2619,9 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
   bool seen = true; // (else a replay may have moved them since the update)
   for (auto const &g : gg_) seen = seen && !(g.pos && g.pos->unseen);
   if (N_ > 0 && !(seen && xsorted_epoch_ == epoch_ && xsorted_of_ == pos_versions())) {
-    k_xsorted<<<div_up(N_, 256), 256, 0, s>>>(pt, sorted_vals_, N_, xsorted_); count_launch();
+    CountTable ct{};
+    for (int g = 0; g < G; ++g) ct.n[g] = uint32_t(gg_[g].g->count);
+    k_xsorted<<<div_up(N_, 256), 256, 0, s>>>(pt, ct, sorted_vals_, N_, xsorted_); count_launch();
     PG_LAUNCH_CHECK();
   }
   // staged lists: with factors, for a group in cell order, at most two
@@ -2621,8 +2634,10 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
   bool warp = !st && in_grid_[q] && G <= 2 && model_->tune.v[kTuneListSplit] != 0;
   // with a thread per query, a group that is not in cell order (never
   // permuted, or resized since) is walked in grid order
+  // (not one resized since the grid's update, whose items that order is not of)
   uint32_t const *order = nullptr;
-  if (!ordered && !warp) {
+  size_t held = goff_[q + 1] - goff_[q];
+  if (!ordered && !warp && held == n) {
     if (n > order_cap_) {
       if (order_) PG_CUDA(cudaFree(order_));
       order_cap_ = n + n / 8;
@@ -2718,7 +2733,7 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
       ProfScope ps(model_->prof, "nhood_lists", s);
       if (warp) {
         // a group that grew since the grid's update: no neighbours of items the grid does not hold
-        if (size_t(goff_[q + 1] - goff_[q]) != n) PG_CUDA(cudaMemsetAsync(L.cb, 0, size_t(G) * n * sizeof(uint2), s));
+        if (held != n) PG_CUDA(cudaMemsetAsync(L.cb, 0, size_t(G) * n * sizeof(uint2), s));
         if (G == 1) launch_build_lists_warp<1>(N_, s, gv, xsorted_, q, lo, h, L.hcache);
         else launch_build_lists_warp<2>(N_, s, gv, xsorted_, q, lo, h, L.hcache);
       } else if (st) {
