@@ -442,7 +442,7 @@ __global__ void k_seg_active(SegArgs S) { seg_list_active(S); }
 template <uint32_t FORM, class Load, class Use>
 __device__ __forceinline__ void walk_kernel(NbrList const &L, uint32_t i, QuickKernel const &K, Load &&load, Use &&use) {
   if (K.quick) walk_nbrs<FORM, false>(L, i, load, [&](float4 x, float, bool in) { use(x, in, K); });
-  else walk_nbrs_singly(L, i, load, [&](float4 x, float, bool in) { use(x, in, K.k); });
+  else for_each_nbr<16>(L, i, false, [&](uint32_t j, float) { use(load(j), true, K.k); });
 }
 
 template <int NF, int NB, int NT = kNT, int MINB = kMinBlocks, int BT = 4 | kFill>
@@ -673,7 +673,7 @@ __device__ __forceinline__ void iisph_accel_item(uint32_t i, float4 const *__res
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    walk_nbrs_cached<BT>(F.L, i, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), __ldg(F.pr + j)}; },
+    walk_nbrs_cached<BT, false, true>(F.L, i, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), __ldg(F.pr + j)}; },
                          [&](WithRec<float> const &r, float gf, bool in, auto cached) {
       float coef = r.x.w * (pri + r.v);
       acc = sub_if(in, acc, scl3(coef, pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
@@ -683,7 +683,7 @@ __device__ __forceinline__ void iisph_accel_item(uint32_t i, float4 const *__res
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    walk_nbrs_cached<BT>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+    walk_nbrs_cached<BT, false, true>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
                          [&](float4 xv, float gf, bool in, auto cached) {
       float coef = ((0.7f * rho0) * xv.w) * bterm;
       acc = sub_if(in, acc, scl3(coef, pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
@@ -776,7 +776,7 @@ __device__ __forceinline__ double iisph_pressure_item(uint32_t i, PressureArgs c
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    walk_nbrs_cached<BT>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.a + j))}; },
+    walk_nbrs_cached<BT, false, true>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.a + j))}; },
                          [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
       ap = add_if(in, ap, r.x.w * dot3(sub3(ai, r.v), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
     });
@@ -784,7 +784,7 @@ __device__ __forceinline__ double iisph_pressure_item(uint32_t i, PressureArgs c
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    walk_nbrs_cached<BT>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+    walk_nbrs_cached<BT, false, true>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
                          [&](float4 xv, float gf, bool in, auto cached) {
       ap = add_if(in, ap, (rho0 * xv.w) * dot3(sub3(ai, f3{0.0f, 0.0f, 0.0f}), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
     });
@@ -1274,7 +1274,7 @@ __global__ void __launch_bounds__(kNT, kMinBlocks) k_viscosity(uint32_t n, float
         f3 xij = sub3(xi, mk3(r.x));
         float coef = divide_noting<kFlat>(((10.0f * (mu / ri)) * r.x.w) * dot3(sub3(vi, r.v), xij), nsq3(xij) + hh, off);
         ai = add_if(in, ai, scl3(coef, pgrad(is_cached(cached), gf, K, xij)));
-      });
+      }, [&] { return off; });
     }
 #pragma unroll
     for (int q = 0; q < NB; ++q) {
@@ -1288,7 +1288,7 @@ __global__ void __launch_bounds__(kNT, kMinBlocks) k_viscosity(uint32_t n, float
         float coef = divide_noting<kFlat>(((10.0f * (bmu / ri)) * vr) * dot3(sub3(vi, f3{0.0f, 0.0f, 0.0f}), xij),
                                           nsq3(xij) + hh, off);
         ai = add_if(in, ai, scl3(coef, pgrad(is_cached(cached), gf, K, xij)));
-      });
+      }, [&] { return off; });
     }
     if (!off) break;
     flat = false;
