@@ -148,6 +148,7 @@ void upload_varying(VaryingField &f, size_t count, void const *host, size_t n_it
   if (n_items != count)
     throw Error("upload: item count " + std::to_string(n_items) + " != group count " + std::to_string(count));
   f.version++;
+  f.uploads++;
   if (!sync && capturing(s)) f.unseen = true;
   if (count == 0) return;
   size_t hbytes = count * f.type.host_item_bytes();

@@ -53,6 +53,7 @@ struct VaryingField {
   void *d = nullptr;   // device storage
   size_t cap = 0;      // items allocated
   uint64_t version = 0; // bumped whenever the values may have changed
+  uint64_t uploads = 0; // how often the host wrote it
   // a captured procedure writes it: replays of its graph change the values
   // without the version
   bool unseen = false;

@@ -2805,6 +2805,7 @@ void Nhood::build_lists(int q, Lists &L, cudaStream_t s, float const *h, bool st
   L.view.tile_info = L.staged ? L.tile_info : nullptr;
   L.view.tile_cells = L.staged ? L.tile_cells : nullptr;
   L.view.n = uint32_t(n);
+  L.view.ordered = permuted_count_[q] == n && permuted_uploads_[q] == gg_[q].pos->uploads;
 }
 
 NbrView const &Nhood::lists(int q, cudaStream_t s, float const *h, bool stage) {
@@ -2859,6 +2860,7 @@ void Nhood::permute(Model &m, cudaStream_t s) {
     gg_[g].g->permute(perm, s);
     PG_CUDA(cudaFreeAsync(perm, s));
     permuted_count_[g] = n;
+    permuted_uploads_[g] = gg_[g].pos->uploads;
   }
   update(s);
 }
@@ -2884,6 +2886,7 @@ void Nhood::permute_segments(Model &m, uint8_t const *due_d, cudaStream_t s) {
     gg_[g].g->permute(perm, s);
     PG_CUDA(cudaFreeAsync(perm, s));
     permuted_count_[g] = n;
+    permuted_uploads_[g] = gg_[g].pos->uploads;
   }
   update(s);
 }

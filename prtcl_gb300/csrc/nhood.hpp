@@ -95,6 +95,7 @@ struct NbrView {
   uint2 const *cb[kMaxGroups];
   uint32_t cap[kMaxGroups]; // a multiple of kChunk
   uint32_t n;               // query items
+  bool ordered;             // the group was permuted into cell order at this size, its positions not uploaded since
   float const *hcache;      // NaN when no factors were computed
   // staged lists (nullptr when not built staged)
   uint16_t const *slots[kMaxGroups];
@@ -302,6 +303,7 @@ private:
   // item count of each group when it was last permuted into cell order (the
   // list build walks a group that was not in grid order instead)
   size_t permuted_count_[kMaxGroups] = {};
+  uint64_t permuted_uploads_[kMaxGroups] = {}; // uploads of its positions before that
   uint32_t *order_ = nullptr; // group items in grid order (list build)
   // grid by counting: per cell key the item count (zero between updates), the
   // cell, and the tile sums; counted_: the present grid was built that way;

@@ -93,6 +93,7 @@ void upload_varying_noalloc(VaryingField &f, size_t count, void const *host, siz
     throw Error("no-alloc upload: the stream is being captured; the call is synchronous and cannot be captured");
   void *stage = staged ? stage_address() : nullptr;
   f.version++;
+  f.uploads++;
   if (count == 0) return;
   if (!staged) {
     PG_CUDA(cudaMemcpyAsync(f.d, host, hbytes, cudaMemcpyHostToDevice, s));

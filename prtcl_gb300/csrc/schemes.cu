@@ -238,6 +238,22 @@ template <class Shapes, bool Tuned, class F> void with_shape(int v, F &&f) {
   }
   f(std::tuple_element_t<0, Shapes>{});
 }
+// Many items that were not permuted into cell order: the records of a warp's
+// gathers lie far apart, and L1 holds few of them until they are read again, so
+// the more loads in flight the better.  The walk with a branch per entry takes 16
+// entries together (8 in the diagonal) where the branch-free one gathers 4:
+// where the knob has its default, density and diagonal take it.  Branch-free /
+// branching, us: density of a lattice in its own order, 422k items 37 / 41, 636k
+// 91 / 65, 1M 144 / 95; in random order 85 / 72, 122 / 98, 189 / 143; diagonal 51 /
+// 61, 113 / 100, 177 / 154 and 99 / 83, 160 / 128, 237 / 193.  In cell order 1M is a
+// draw (78 / 78, 112 / 115) and fewer items are faster branch-free (636k 50 / 53,
+// 72 / 74).  Explicit viscosity gains nothing by it (181 / 181, 279 / 287).
+constexpr uint32_t kSpreadItems = 500'000;
+bool spread(uint32_t n, NbrView const &v) { return !v.ordered && n >= kSpreadItems; }
+template <class Shapes, class Spread, bool Tuned, class F> void with_shape_spread(bool spread, int v, F &&f) {
+  if (spread && v == 0) f(Spread{});
+  else with_shape<Shapes, Tuned>(v, f);
+}
 // the same for a plain launch over n items of a sweep that takes SmallShape
 template <class Shapes, bool Tuned, bool Small, class F> void with_shape_for(uint32_t n, int v, F &&f) {
   if constexpr (Small) {
@@ -256,11 +272,13 @@ template <class Shapes> std::string shapes_text() {
          " 2=" + shape_text<std::tuple_element_t<2, Shapes>>() + " 3=" + shape_text<std::tuple_element_t<3, Shapes>>();
 }
 using DensityShapes = FreeShapes<4 | kFill, 8 | kFill>;
+using DensitySpread = Shape<kNT, kMinBlocks, 16 | kAlone>;
 using SetupShapes = FreeShapes<8, 4>;
 using AccelShapes = FreeShapes<8 | kAlone, 8 | kFill>;
 using AccelSegShapes = RedShapes<8 | kFill, 8 | kAlone>;
 using PressureShapes = RedShapes<8 | kAlone, 8 | kFill>;
 using DiagShapes = FreeShapes<4 | kFill, 8 | kFill>;
+using DiagSpread = Shape<kNT, kMinBlocks, 8 | kAlone>;
 using PcgShapes = RedShapes<8 | kAlone, 8>;
 using PcgSegShapes = RedShapes<8, 8 | kAlone>;
 
@@ -441,8 +459,16 @@ __global__ void k_seg_active(SegArgs S) { seg_list_active(S); }
 // kernel per pair
 template <uint32_t FORM, class Load, class Use>
 __device__ __forceinline__ void walk_kernel(NbrList const &L, uint32_t i, QuickKernel const &K, Load &&load, Use &&use) {
-  if (K.quick) walk_nbrs<FORM, false>(L, i, load, [&](float4 x, float, bool in) { use(x, in, K); });
-  else for_each_nbr<16>(L, i, false, [&](uint32_t j, float) { use(load(j), true, K.k); });
+  if constexpr ((FORM & kAlone) != 0u) {
+    if (K.quick) {
+      for_each_nbr<FORM & 0xFFu>(L, i, false, [&](uint32_t j, float) { use(load(j), true, K); });
+      return;
+    }
+  } else if (K.quick) {
+    walk_nbrs<FORM, false>(L, i, load, [&](float4 x, float, bool in) { use(x, in, K); });
+    return;
+  }
+  for_each_nbr<16>(L, i, false, [&](uint32_t j, float) { use(load(j), true, K.k); });
 }
 
 template <int NF, int NB, int NT = kNT, int MINB = kMinBlocks, int BT = 4 | kFill>
@@ -2525,7 +2551,8 @@ public:
       uint32_t n = uint32_t(F.g->count);
       auto N = S->nbrs<NF, NB>(v, s);
       ProfScope ps(S->model_->prof, "density", s);
-      with_shape<DensityShapes, NF == 1 && NB == 1>(S->model_->tune.v[kTuneDensity], [&](auto sh) {
+      with_shape_spread<DensityShapes, DensitySpread, NF == 1 && NB == 1>(spread(n, v), S->model_->tune.v[kTuneDensity],
+                                                                         [&](auto sh) {
         using Sh = decltype(sh);
         k_density<NF, NB, Sh::nt, Sh::minb, Sh::bt><<<div_up(n, Sh::nt), Sh::nt, 0, s>>>(
             n, dptr<float4>(F.x), dptr<float>(F.rho), S->u(F.rho0), G, N);
@@ -3148,13 +3175,16 @@ public:
     auto N = bnbrs<NB>(v, s);
     float4 const *xmr = model_->packed_xmr(F.g, F.x, F.m, F.rho, s);
     ProfScope ps(model_->prof, "wkbb18_diag", s);
+    bool sp = spread(n, v);
     if (gc_)
-      k_wkbb18_diag<NB, true><<<div_up(n, kNT), kNT, 0, s>>>(n, uint32_t(F.sp->cap), xmr, dptr<float>(F.rho),
-                                                              dptr<float>(F.sp), u(F.rho0), u(F.mu), G,
-                                                              nl(v, F.g->index), N, dptr<float>(F.L),
-                                                              uint32_t(F.L->cap));
+      with_shape_spread<DiagShapes, DiagSpread, false>(sp, 0, [&](auto sh) {
+        using Sh = decltype(sh);
+        k_wkbb18_diag<NB, true, Sh::nt, Sh::minb, Sh::bt><<<div_up(n, kNT), kNT, 0, s>>>(
+            n, uint32_t(F.sp->cap), xmr, dptr<float>(F.rho), dptr<float>(F.sp), u(F.rho0), u(F.mu), G,
+            nl(v, F.g->index), N, dptr<float>(F.L), uint32_t(F.L->cap));
+      });
     else
-      with_shape<DiagShapes, NB == 1>(fluid_.size() == 1 ? model_->tune.v[kTuneDiag] : 0, [&](auto sh) {
+      with_shape_spread<DiagShapes, DiagSpread, NB == 1>(sp, fluid_.size() == 1 ? model_->tune.v[kTuneDiag] : 0, [&](auto sh) {
         using Sh = decltype(sh);
         k_wkbb18_diag<NB, false, Sh::nt, Sh::minb, Sh::bt><<<div_up(n, Sh::nt), Sh::nt, 0, s>>>(
             n, uint32_t(F.sp->cap), xmr, dptr<float>(F.rho), dptr<float>(F.sp), u(F.rho0), u(F.mu), G,
