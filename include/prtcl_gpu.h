@@ -191,7 +191,9 @@ int prtcl_gpu_profile_reset(prtcl_gpu_model *model);
  * most two neighbour groups; 0: by one thread per query).  prtcl_gb300/tune.py searches them
  * per workload and caches the choice.  prtcl_gpu_tune_knobs returns one line
  * per knob: "name default value=shape ...", a shape written as threads per
- * block x blocks per SM / neighbour-walk batch.  An unknown knob gives
+ * block x blocks per SM / neighbour-walk batch and a letter for the walk's form
+ * (b: a branch per entry; f, p, a: without), and the shapes that stand for the
+ * default at some sizes.  An unknown knob gives
  * PRTCL_GPU_NOT_FOUND, a value outside its set PRTCL_GPU_INVALID. */
 int prtcl_gpu_tune_knobs(char *buf, int64_t size, int64_t *needed_out);
 int prtcl_gpu_model_tune_set(prtcl_gpu_model *model, const char *knob, int32_t value);

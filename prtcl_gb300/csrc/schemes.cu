@@ -265,7 +265,9 @@ template <class Shapes, bool Tuned, bool Small, class F> void with_shape_for(uin
   with_shape<Shapes, Tuned>(v, f);
 }
 template <class Sh> std::string shape_text() {
-  return std::to_string(Sh::nt) + "x" + std::to_string(Sh::minb) + "/" + std::to_string(Sh::bt & 0xFF);
+  uint32_t f = uint32_t(Sh::bt);
+  return std::to_string(Sh::nt) + "x" + std::to_string(Sh::minb) + "/" + std::to_string(f & 0xFFu) +
+         ((f & kAlone) ? "b" : (f & kFill) ? "f" : (f & kAhead) ? "a" : "p");
 }
 template <class Shapes> std::string shapes_text() {
   return "0=" + shape_text<std::tuple_element_t<0, Shapes>>() + " 1=" + shape_text<std::tuple_element_t<1, Shapes>>() +
@@ -2290,17 +2292,22 @@ bool tune_value_ok(int k, int v) {
   return k >= 0 && k < kTuneKnobs && v >= 0 && v <= 3;
 }
 std::string tune_knob_table() {
-  // shapes as threads-per-block x blocks-per-SM / walk batch
-  std::string t;
-  t += "density 0 " + shapes_text<DensityShapes>() + "\n";
-  t += "iisph_setup 0 " + shapes_text<SetupShapes>() + "\n";
-  t += "iisph_accel 0 " + shapes_text<AccelShapes>() + " batched: " + shapes_text<AccelSegShapes>() +
+  // shapes as threads-per-block x blocks-per-SM / walk batch, form of the walk
+  // (b: a branch per entry; without: f records filled in past a row's end, p
+  // predicated off, a entries loaded ahead), and what stands for value 0 at
+  // some sizes
+  std::string t, small = " small: " + shape_text<SmallShape>() + " to " + std::to_string(kSmallItems);
+  std::string from = " from " + std::to_string(kSpreadItems);
+  t += "density 0 " + shapes_text<DensityShapes>() + " unordered: " + shape_text<DensitySpread>() + from + "\n";
+  t += "iisph_setup 0 " + shapes_text<SetupShapes>() + small + "\n";
+  t += "iisph_accel 0 " + shapes_text<AccelShapes>() + small + " batched: " + shapes_text<AccelSegShapes>() +
        " 4=persistent tiles (batched; 0 otherwise)\n";
-  t += "iisph_pressure 0 " + shapes_text<PressureShapes>() + " 4=persistent tiles (batched; 0 otherwise)\n";
-  t += "wkbb18_diag 0 " + shapes_text<DiagShapes>() + "\n";
-  t += "pcg_init 0 " + shapes_text<PcgShapes>() + "\n";
-  t += "pcg_q 0 " + shapes_text<PcgShapes>() + " 4=cell-tiles (no lists; plain models)\n";
-  t += "jacobi_unroll 1 1=1 2=2 4=4\n";
+  t += "iisph_pressure 0 " + shapes_text<PressureShapes>() + small + " 4=persistent tiles (batched; 0 otherwise)\n";
+  t += "wkbb18_diag 0 " + shapes_text<DiagShapes>() + " unordered: " + shape_text<DiagSpread>() + from + "\n";
+  t += "pcg_init 0 " + shapes_text<PcgShapes>() + small + " batched: " + shapes_text<PcgSegShapes>() + "\n";
+  t += "pcg_q 0 " + shapes_text<PcgShapes>() + small + " batched: " + shapes_text<PcgSegShapes>() +
+       " 4=cell-tiles (no lists; plain models)\n";
+  t += "jacobi_unroll 1 1=1 (one launch to " + std::to_string(kSmallItems) + " items) 2=2 4=4\n";
   t += "staging 0 0=off 1=staged lists and sweeps (unbatched models)\n";
   t += "grid_sort 1 0=tiled radix sort 1=counting where the keys are short, else one cluster launch up to 128k items\n";
   t += "list_split 1 0=one thread per query 1=one warp per run of queries of a cell\n";

@@ -36,10 +36,13 @@ state as an untuned one.
 Cache.  Choices persist in a JSON file keyed by the device name and a
 workload class (plain or batched, with the fluid count and scene count in
 powers of two): ``$PRTCL_GB300_TUNE_CACHE``, else
-``~/.cache/prtcl_gb300/tuning.json``.
+``~/.cache/prtcl_gb300/tuning.json``.  A choice is taken by a library with the
+same knob table (knob_fingerprint); by another, whose values stand for other
+shapes, the workload is tuned afresh.
 """
 from __future__ import annotations
 
+import hashlib
 import json
 import math
 import os
@@ -62,6 +65,16 @@ def knob_table():
         name, _, rest = line.partition(" ")
         out[name] = rest
     return out
+
+
+def knob_fingerprint():
+    """Names what the knobs' values stand for: a digest of the knob table
+    ("" where there is no library to ask, and nothing to apply a choice to)."""
+    try:
+        table = knob_table()
+    except ImportError:
+        return ""
+    return hashlib.sha1(json.dumps(table, sort_keys=True).encode()).hexdigest()[:16]
 
 
 def default_cache_path():
@@ -113,7 +126,7 @@ class Autotuner:
 
     def lookup(self, workload):
         rec = self._load().get(self.key(workload))
-        if not rec:
+        if not rec or rec.get("knobs") != knob_fingerprint():
             return None
         choice = rec.get("choice", {})
         if any(k not in VALUES or v not in VALUES[k] for k, v in choice.items()):
@@ -122,7 +135,8 @@ class Autotuner:
 
     def store(self, workload, choice, timings):
         data = self._load()
-        data[self.key(workload)] = {"choice": choice, "timings_us": timings, "when": time.strftime("%Y-%m-%dT%H:%M:%S")}
+        data[self.key(workload)] = {"choice": choice, "knobs": knob_fingerprint(), "timings_us": timings,
+                                    "when": time.strftime("%Y-%m-%dT%H:%M:%S")}
         os.makedirs(os.path.dirname(os.path.abspath(self.path)), exist_ok=True)
         tmp = self.path + f".{os.getpid()}.tmp"
         with open(tmp, "w") as f:
