@@ -158,15 +158,8 @@ __device__ __forceinline__ void load_held(NbrHeld &H, unsigned char const *ch, u
   }
 }
 
-// stop(): asked after each batch, whether the rest of the row is not wanted (the
-// row is to be walked again, by walk_nbrs_singly).  The sweep that asks, the
-// explicit viscosity, takes 122 -> 127 us for it at 1M items, and 253 -> 177 at
-// smoothing scales below 1e-5, where it is every row.
-struct NeverStop {
-  __device__ __forceinline__ constexpr bool operator()() const { return false; }
-};
-template <uint32_t FORM, bool GF, bool KEEP = false, class Load, class Use, class Stop = NeverStop>
-__device__ __forceinline__ void walk_nbrs(NbrList const &L, uint32_t i, Load &&load, Use &&use, Stop &&stop = Stop{}) {
+template <uint32_t FORM, bool GF, bool KEEP = false, class Load, class Use>
+__device__ __forceinline__ void walk_nbrs(NbrList const &L, uint32_t i, Load &&load, Use &&use) {
   constexpr uint32_t GATHER = FORM & 0xFFu;
   constexpr bool AHEAD = (FORM & kAhead) != 0u, FILL = (FORM & kFill) != 0u;
   static_assert(kNbrHeld % GATHER == 0 && GATHER % 2 == 0, "whole batches");
@@ -217,7 +210,6 @@ __device__ __forceinline__ void walk_nbrs(NbrList const &L, uint32_t i, Load &&l
 #pragma unroll
       for (uint32_t t = 0; t < GATHER; ++t) use(r[t], H.g[u + t], k + u + t < c);
     }
-    if (stop()) return;
   }
 }
 
@@ -239,27 +231,38 @@ __device__ __forceinline__ void walk_nbrs_singly(NbrList const &L, uint32_t i, L
   }
 }
 
-// use(record, factor, in, cached): with the lists' factors where `cached`, else
-// (the smoothing scale has changed since the lists were built, or the row
-// divides outside of the range of the branch-free divisions) without: one entry
-// at a time or, EACH, by for_each_nbr.  `cached` comes as a std::bool_constant,
-// or as a bool where the form is kAlone.  EACH is for sweeps without divisions
-// (27k items after a change of the scale, acceleration 24.9 -> 22.8 us, as long
-// as before there was a branch-free walk); beside divisions it spills in the
-// branch-free walk's registers (60k viscosity with gradient correction 240 ->
-// 252 us, 48 scenes 37.0 -> 39.9 ms), and so do the lists' factors in a row
-// walked one entry at a time (explicit viscosity 122 -> 207 us).
-template <uint32_t FORM, bool KEEP = false, bool EACH = false, class Load, class Use, class Stop = NeverStop>
-__device__ __forceinline__ void walk_nbrs_cached(NbrList const &L, uint32_t i, bool cached, Load &&load, Use &&use,
-                                                 Stop &&stop = Stop{}) {
-  if constexpr ((FORM & kAlone) != 0u)
-    for_each_nbr<FORM & 0xFFu, KEEP>(L, i, cached, [&](uint32_t j, float g) { use(load(j), g, true, cached); });
-  else if (cached)
-    walk_nbrs<FORM, true, KEEP>(L, i, load, [&](auto const &r, float g, bool in) { use(r, g, in, std::true_type{}); }, stop);
-  else if constexpr (EACH)
-    for_each_nbr<kNbrHeld, KEEP>(L, i, false, [&](uint32_t j, float g) { use(load(j), g, true, std::false_type{}); });
+// use(record, factor, in, cached).  Where `flat` (which implies cached) by
+// walk_nbrs, with the lists' factors; `cached` then comes as std::true_type.
+// Else, and where the form is kAlone, by for_each_nbr, and it comes as a bool:
+// whether the lists' factors hold (they do not once the smoothing scale has
+// changed since the lists were built).
+template <uint32_t FORM, class Load, class Use>
+__device__ __forceinline__ void walk_nbrs_flat(NbrList const &L, uint32_t i, bool flat, bool cached, Load &&load,
+                                               Use &&use) {
+  constexpr bool kAlways = (FORM & kAlone) != 0u;
+  if (!kAlways && flat)
+    walk_nbrs<kAlways ? kNbrHeld : FORM, true>(
+        L, i, load, [&](auto const &r, float g, bool in) { use(r, g, in, std::true_type{}); });
   else
-    walk_nbrs_singly(L, i, load, [&](auto const &r, float g, bool in) { use(r, g, in, std::false_type{}); });
+    for_each_nbr<kAlways ? (FORM & 0xFFu) : kNbrHeld>(
+        L, i, cached, [&](uint32_t j, float g) { use(load(j), g, true, cached); });
+}
+// The same where flat and cached are one, for the sweeps whose registers do not
+// stand for_each_nbr beside the branch-free walk: the other walk takes one entry
+// at a time, without the lists' factors (`cached` comes as std::false_type).
+// After a change of the scale, this / for_each_nbr: 1M items set-up 352 / 415 us,
+// diagonal 191 / 200, correction 272 / 324, 27k items 49 / 43, 27 / 25, 28 / 27; PCG
+// with its divisions 338 / 325, but 48 scenes 36.2 / 36.4 ms throughout.
+template <uint32_t FORM, bool KEEP = false, class Load, class Use>
+__device__ __forceinline__ void walk_nbrs_cached(NbrList const &L, uint32_t i, bool cached, Load &&load, Use &&use) {
+  if constexpr ((FORM & kAlone) != 0u) {
+    walk_nbrs_flat<FORM>(L, i, cached, cached, load, use);
+  } else {
+    if (cached)
+      walk_nbrs<FORM, true, KEEP>(L, i, load, [&](auto const &r, float g, bool in) { use(r, g, in, std::true_type{}); });
+    else
+      walk_nbrs_singly(L, i, load, [&](auto const &r, float g, bool in) { use(r, g, in, std::false_type{}); });
+  }
 }
 __device__ __forceinline__ bool is_cached(bool c) { return c; }
 template <bool C> __device__ __forceinline__ constexpr bool is_cached(std::bool_constant<C>) { return C; }

@@ -701,7 +701,7 @@ __device__ __forceinline__ void iisph_accel_item(uint32_t i, float4 const *__res
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    walk_nbrs_cached<BT, false, true>(F.L, i, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), __ldg(F.pr + j)}; },
+    walk_nbrs_flat<BT>(F.L, i, uc, uc, [&](uint32_t j) { return WithRec<float>{__ldg(F.xm + j), __ldg(F.pr + j)}; },
                          [&](WithRec<float> const &r, float gf, bool in, auto cached) {
       float coef = r.x.w * (pri + r.v);
       acc = sub_if(in, acc, scl3(coef, pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
@@ -711,7 +711,7 @@ __device__ __forceinline__ void iisph_accel_item(uint32_t i, float4 const *__res
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    walk_nbrs_cached<BT, false, true>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+    walk_nbrs_flat<BT>(B.L, i, uc, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
                          [&](float4 xv, float gf, bool in, auto cached) {
       float coef = ((0.7f * rho0) * xv.w) * bterm;
       acc = sub_if(in, acc, scl3(coef, pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
@@ -804,7 +804,7 @@ __device__ __forceinline__ double iisph_pressure_item(uint32_t i, PressureArgs c
 #pragma unroll
   for (int q = 0; q < NF; ++q) {
     FluidN const &F = N.f[q];
-    walk_nbrs_cached<BT, false, true>(F.L, i, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.a + j))}; },
+    walk_nbrs_flat<BT>(F.L, i, uc, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.a + j))}; },
                          [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
       ap = add_if(in, ap, r.x.w * dot3(sub3(ai, r.v), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(r.x)))));
     });
@@ -812,7 +812,7 @@ __device__ __forceinline__ double iisph_pressure_item(uint32_t i, PressureArgs c
 #pragma unroll
   for (int q = 0; q < NB; ++q) {
     BoundN const &B = N.b[q];
-    walk_nbrs_cached<BT, false, true>(B.L, i, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
+    walk_nbrs_flat<BT>(B.L, i, uc, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
                          [&](float4 xv, float gf, bool in, auto cached) {
       ap = add_if(in, ap, (rho0 * xv.w) * dot3(sub3(ai, f3{0.0f, 0.0f, 0.0f}), pgrad(is_cached(cached), gf, K, sub3(xi, mk3(xv)))));
     });
@@ -1289,26 +1289,26 @@ __global__ void __launch_bounds__(kNT, kMinBlocks) k_viscosity(uint32_t n, float
   float ri = rho[i];
   f3 ai, a0 = mk3(a[i]);
   Divisor rdiv = divisor(ri);
-  bool flat = uc, off;
+  bool flat = uc && hh >= 0x1p-40f && hh <= 0x1p40f, off; // (an item is its own neighbour, and divides by hh)
   do {
     ai = a0;
     off = false;
 #pragma unroll
     for (int q = 0; q < NF; ++q) {
       FluidN const &F = N.f[q];
-      walk_nbrs_cached<8>(F.L, i, flat, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.v + j))}; },
+      walk_nbrs_flat<8>(F.L, i, flat, uc, [&](uint32_t j) { return WithRec<f3>{__ldg(F.xm + j), mk3(__ldg(F.v + j))}; },
                           [&](WithRec<f3> const &r, float gf, bool in, auto cached) {
         constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
         f3 xij = sub3(xi, mk3(r.x));
         float coef = divide_noting<kFlat>(((10.0f * (mu / ri)) * r.x.w) * dot3(sub3(vi, r.v), xij), nsq3(xij) + hh, off);
         ai = add_if(in, ai, scl3(coef, pgrad(is_cached(cached), gf, K, xij)));
-      }, [&] { return off; });
+      });
     }
 #pragma unroll
     for (int q = 0; q < NB; ++q) {
       BoundN const &B = N.b[q];
       float bmu = *B.mu;
-      walk_nbrs_cached<8>(B.L, i, flat, [&](uint32_t j) { return __ldg(B.xV + j); },
+      walk_nbrs_flat<8>(B.L, i, flat, uc, [&](uint32_t j) { return __ldg(B.xV + j); },
                           [&](float4 xv, float gf, bool in, auto cached) {
         constexpr bool kFlat = std::is_same_v<decltype(cached), std::true_type>;
         f3 xij = sub3(xi, mk3(xv));
@@ -1316,7 +1316,7 @@ __global__ void __launch_bounds__(kNT, kMinBlocks) k_viscosity(uint32_t n, float
         float coef = divide_noting<kFlat>(((10.0f * (bmu / ri)) * vr) * dot3(sub3(vi, f3{0.0f, 0.0f, 0.0f}), xij),
                                           nsq3(xij) + hh, off);
         ai = add_if(in, ai, scl3(coef, pgrad(is_cached(cached), gf, K, xij)));
-      }, [&] { return off; });
+      });
     }
     if (!off) break;
     flat = false;
