@@ -1695,7 +1695,7 @@ __device__ __forceinline__ uint32_t *factor_word(unsigned char *ch, uint32_t slo
 // portions that turns wide is converted where it does; a row longer than the
 // capacity is counted on, not written.
 //
-// What bounds it: instruction issue (70 % of the slots at 28 warps per SM on
+// What bounds it: instruction issue (79 % of the slots at 30 warps per SM on
 // the dam break) and the latency between a unit's phases, which the resident
 // warps hide: candidates kept in registers or staged with their positions in
 // shared memory left 16 to 24 warps and took 516 to 645 us on the 1M dam
@@ -2385,7 +2385,6 @@ void Nhood::build_direct(GridView const &gv, int G, size_t N, cudaStream_t s) {
     xsorted_epoch_ = epoch_;
     PG_LAUNCH_CHECK();
   }
-  sorted_keys_ = nullptr;
   sorted_vals_ = vals_a_;
   counted_ = true;
   key_check_ = true; // the fullest cell is confirmed with the key statistics
@@ -2452,7 +2451,6 @@ void Nhood::update(cudaStream_t s) {
   if (N == 0) {
     key_check_ = false; // no statistics to confirm
     PG_CUDA(cudaMemsetAsync(ncells_d_, 0, sizeof(int), s));
-    sorted_keys_ = keys_a_;
     sorted_vals_ = vals_a_;
     return;
   }
@@ -2555,7 +2553,6 @@ void Nhood::update(cudaStream_t s) {
     std::swap(kin, kout);
     std::swap(vin, vout);
   }
-  sorted_keys_ = kin;
   sorted_vals_ = vin;
   gv = view();
   model_->prof.end(s); // grid_sort
@@ -2940,7 +2937,9 @@ size_t Nhood::device_bytes() const {
   // keys 2x8, values 2x4, ukeys 16, flags 4, scan 4, r2s 4, s2c 4, cell
   // start 4, adjacency 104, cell key 8, cell index 16, sorted positions 16
   size_t b = cap_ * (16 + 8 + 16 + 4 + 4 + 4 + 4 + 4 + 104 + 8 + 16 + 16);
-  b += hist_cap_ * 4 + block_sums_cap_ * 4 + dir_cap_ * 8 + hash_cap_ * 12;
+  b += hist_cap_ * 4 + block_sums_cap_ * 4 + hash_cap_ * 12;
+  // counting: per entry the count and the cell 8, the marks 4 kMark / kDirRun; the tiles' sums
+  b += dir_cap_ * 8 + dir_cap_ / kDirRun * kMark * 4 + (dir_cap_ ? (dir_cap_ / kDirTile + kDirBlocks) * 8 : 0);
   for (auto const &kv : lists_) {
     Lists const &L = kv.second;
     b += L.n * gg_.size() * sizeof(uint2);

@@ -346,7 +346,6 @@ private:
   uint32_t *stats_d_ = nullptr; // bit statistics / counters
   int *ncells_d_ = nullptr;
   uint32_t *stats_h_ = nullptr; // pinned
-  uint64_t const *sorted_keys_ = nullptr;
   uint32_t const *sorted_vals_ = nullptr;
   std::map<int, Lists> lists_;
 };
