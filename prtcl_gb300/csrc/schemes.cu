@@ -145,9 +145,11 @@ struct Globals {
   unsigned const *turn; // of the solver loops' barriers (Meet)
 };
 // whether a solver loop gave up and the host has not seen it yet: what it was
-// for is left alone then
+// for is left alone then.  (Only an earlier launch writes it: an ordinary load,
+// which L1 serves.  One past L1 by every warp to the one word took the velocity
+// integration of 1M items from 10.8 to 16.6 us.)
 constexpr unsigned kGaveUp = 0x80000000u;
-__device__ __forceinline__ bool gave_up(Globals const &G) { return (*(unsigned volatile const *)G.turn & kGaveUp) != 0u; }
+__device__ __forceinline__ bool gave_up(Globals const &G) { return (*G.turn & kGaveUp) != 0u; }
 
 struct Red {
   double *partials; // [3][kMaxRedBlocks]
